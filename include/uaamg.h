@@ -105,7 +105,12 @@ UAAMG_API uaamg_status uaamg_set_stream(uaamg_handle* h, void* stream);
  * coefficients on the device for every precision, once per mask.  Replaces the
  * per-apply set-up of UAAMGPreconditioner[3D]::apply (uaamg_preconditioner.cpp:
  * 183-189, uaamg_preconditioner_3d.cpp:205-214) and the GPU adapter's mask
- * upload (cuda_pcg_solver.cu:27-49).  `solid` is a HOST byte mask (padded). */
+ * upload (cuda_pcg_solver.cu:27-49).  `solid` is a HOST byte mask (padded).
+ * FP64 solves, and every V-cycle applied by itself (uaamg_precond_apply) or level
+ * inspected, use the reference's hierarchy.  FP32 and mixed solves precondition with
+ * the same Galerkin sums over aggregates that cover every fluid cell (a coarse cell is
+ * fluid when any child is, odd sizes round up), which needs far fewer iterations next
+ * to solids and on odd sizes; with Dirichlet walls they use the reference's. */
 UAAMG_API uaamg_status uaamg_set_problem_2d(uaamg_handle* h, int nx, int ny, double dx, double dy,
                                   const uint8_t* solid);
 UAAMG_API uaamg_status uaamg_set_problem_3d(uaamg_handle* h, int nx, int ny, int nz, double dx,

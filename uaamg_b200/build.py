@@ -72,14 +72,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     nvcc = _nvcc()
     os.makedirs(BUILD, exist_ok=True)
-    objs = []
-    for src, extra in UNITS:
+    objs, running = [], []
+    for src, extra in UNITS:  # the units are independent: compiled side by side
         obj = os.path.join(BUILD, os.path.splitext(src)[0] + ".o")
         cmd = [nvcc] + NVCC_COMMON + extra + ["-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
-        subprocess.run(cmd, check=True)
+        running.append((cmd, subprocess.Popen(cmd)))
         objs.append(obj)
+    for cmd, p in running:
+        if p.wait() != 0:
+            raise subprocess.CalledProcessError(p.returncode, cmd)
     tmp = LIB + ".tmp"
     cmd = [nvcc] + ARCH + ["-shared", "-o", tmp] + objs + ["-cudart", "static"]
     if verbose:

@@ -86,33 +86,38 @@ void free_problem(uaamg_handle* h) {
     h->hist_cap = 0;
     h->n = 0;
     h->dim = 0;
-    for (int q = 0; q < 3; ++q) h->ready[q] = false;
+    for (bool& r : h->ready) r = false;
 }
 
-// Engine of precision p with the current problem's hierarchy built.
-uaamg_status engine_for(uaamg_handle* h, int p, uaamg::Engine** out) {
+// Engine of precision p with the current problem's hierarchy built.  reference: the
+// engine that holds the reference's hierarchy (V-cycles applied by themselves, level
+// inspection): in the FP32 and mixed forms its own one, since their solves run on
+// covering aggregates (not with Dirichlet walls).
+uaamg_status engine_for(uaamg_handle* h, int p, uaamg::Engine** out, bool reference = false) {
     if (p < 0 || p > 2) return fail(h, UAAMG_INVALID_ARG, "unknown precision");
     if (!h->dim) return fail(h, UAAMG_NO_PROBLEM, "no problem set (call uaamg_set_problem_*)");
-    if (!h->eng[p]) {
-        h->eng[p] = p == uaamg::PREC_FP64 ? uaamg::create_engine_f64()
-                                          : uaamg::create_engine_f32(p == uaamg::PREC_MIXED);
-        if (!h->eng[p]) return fail(h, UAAMG_OOM, "engine allocation failed");
+    const int q = reference && p != uaamg::PREC_FP64 && !h->dirichlet ? p + 2 : p;
+    uaamg::Engine*& eng = h->eng[q];
+    if (!eng) {
+        eng = p == uaamg::PREC_FP64 ? uaamg::create_engine_f64()
+                                    : uaamg::create_engine_f32(p == uaamg::PREC_MIXED, q != p);
+        if (!eng) return fail(h, UAAMG_OOM, "engine allocation failed");
     }
-    h->eng[p]->set_stream(h->stream);
-    uaamg::api::apply_vcycle_mode(h->eng[p], h->sweeps);
-    h->eng[p]->set_smoothing(h->nu_fine, h->nu_coarse);
-    h->eng[p]->set_autotune(h->autotune != 0);
+    eng->set_stream(h->stream);
+    uaamg::api::apply_vcycle_mode(eng, h->sweeps);
+    eng->set_smoothing(h->nu_fine, h->nu_coarse);
+    eng->set_autotune(h->autotune != 0);
     if (h->lap_on)
-        h->eng[p]->set_operator(h->d_lap[0], h->d_lap[1], h->d_lap[2], h->nx + 2, h->lap_version);
+        eng->set_operator(h->d_lap[0], h->d_lap[1], h->d_lap[2], h->nx + 2, h->lap_version);
     else
-        h->eng[p]->set_operator(nullptr, nullptr, nullptr, 0, h->lap_version);
-    if (!h->ready[p]) {
-        int e = h->eng[p]->set_problem(h->dim, h->nx, h->ny, h->nz, h->dx, h->dy, h->dz,
-                                       h->d_solid, h->dirichlet);
-        if (e != uaamg::E_OK) return map_engine(h, e, "hierarchy set-up", h->eng[p]);
-        h->ready[p] = true;
+        eng->set_operator(nullptr, nullptr, nullptr, 0, h->lap_version);
+    if (!h->ready[q]) {
+        int e = eng->set_problem(h->dim, h->nx, h->ny, h->nz, h->dx, h->dy, h->dz,
+                                 h->d_solid, h->dirichlet);
+        if (e != uaamg::E_OK) return map_engine(h, e, "hierarchy set-up", eng);
+        h->ready[q] = true;
     }
-    *out = h->eng[p];
+    *out = eng;
     return UAAMG_OK;
 }
 
@@ -304,7 +309,7 @@ uaamg_status uaamg_set_variable_laplacian(uaamg_handle* h, const double* lap_dia
 uaamg_status uaamg_set_dirichlet_walls(uaamg_handle* h, int on) {
     if (!h) return UAAMG_INVALID_ARG;
     h->dirichlet = on ? 1 : 0;
-    for (int q = 0; q < 3; ++q) h->ready[q] = false;
+    for (bool& r : h->ready) r = false;
     return UAAMG_OK;
 }
 
@@ -377,7 +382,7 @@ uaamg_status uaamg_precond_apply(uaamg_handle* h, int precision, const double* r
     if (!r || !z) return fail(h, UAAMG_INVALID_ARG, "NULL array");
     cudaSetDevice(h->device);
     uaamg::Engine* eng = nullptr;
-    uaamg_status s = engine_for(h, precision, &eng);
+    uaamg_status s = engine_for(h, precision, &eng, true);
     if (s != UAAMG_OK) return s;
     const size_t bytes = h->n * sizeof(double);
     cudaError_t e = cudaMemcpyAsync(h->d_rhs, r, bytes, cudaMemcpyHostToDevice, h->stream);
@@ -431,7 +436,7 @@ uaamg_status uaamg_level_trim(uaamg_handle* h, int precision, int l, int* boxes,
     if (!h || !boxes || !trimmed) return UAAMG_INVALID_ARG;
     cudaSetDevice(h->device);
     uaamg::Engine* eng = nullptr;
-    uaamg_status s = engine_for(h, precision, &eng);
+    uaamg_status s = engine_for(h, precision, &eng, true);
     if (s != UAAMG_OK) return s;
     if (l < 0 || l >= eng->nlevels()) return fail(h, UAAMG_INVALID_ARG, "level out of range");
     return map_engine(h, eng->level_trim(l, boxes, trimmed), "level_trim");
@@ -442,7 +447,7 @@ uaamg_status uaamg_copy_level(uaamg_handle* h, int precision, int l, uint8_t* so
     if (!h) return UAAMG_INVALID_ARG;
     cudaSetDevice(h->device);
     uaamg::Engine* eng = nullptr;
-    uaamg_status s = engine_for(h, precision, &eng);
+    uaamg_status s = engine_for(h, precision, &eng, true);
     if (s != UAAMG_OK) return s;
     int e = eng->copy_level(l, solid, cx, cy, cz);
     return map_engine(h, e, "copy_level");

@@ -136,6 +136,9 @@ bool tune_lookup(const std::string& key, std::vector<int>* val);
 void tune_store(const std::string& key, const std::vector<int>& val);
 
 Engine* create_engine_f64();
-Engine* create_engine_f32(int mixed);
+// FP32 (mixed = 0) and mixed engines.  apply_only = 0: for solves, on covering
+// aggregates (engine.cuh, build); 1: the reference's hierarchy, for V-cycles applied by
+// themselves and for level inspection (no solve).
+Engine* create_engine_f32(int mixed, int apply_only);
 
 }  // namespace uaamg

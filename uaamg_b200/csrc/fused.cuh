@@ -342,7 +342,8 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
         cR2 = fcell<T, CS>(g, i0, j0, d2i, d2j);
     }
     int kb, ke;
-    zrange<DIM>(g, L.zc, kb, ke);
+    if constexpr (UP) zrange<DIM>(g, L.zc, kb, ke);
+    else zrange_restrict<DIM>(g, L.cg, L.zc, kb, ke);
     T* xpl = reinterpret_cast<T*>(sm + C::OFF_X);
     double acc[3] = {0.0, 0.0, 0.0};
     const int ic = kMX / 2 * (int)blockIdx.x + 1 + (lane >> 1);

@@ -26,8 +26,10 @@ struct uaamg_handle {
     size_t face_n[3] = {0, 0, 0};
     int hist_cap = 0;
     int last_iters = 0;
-    uaamg::Engine* eng[3] = {nullptr, nullptr, nullptr};
-    bool ready[3] = {false, false, false};
+    // by precision; 3 and 4: FP32 and mixed on the reference's hierarchy (V-cycles applied
+    // by themselves and level inspection; made on first use)
+    uaamg::Engine* eng[5] = {};
+    bool ready[5] = {};
     int sweeps = 0;  // V-cycle kernels (uaamg_set_vcycle_kernels): 0 fused marches +
                      // small-level kernel, 1 sweeps, 2 fused marches on every level,
                      // 3 four marches a level + small-level kernel, 4 four marches on

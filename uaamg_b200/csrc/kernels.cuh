@@ -114,10 +114,13 @@ __device__ __forceinline__ bool reduce_last(double (&v)[NV], double* partials,
 // Hierarchy set-up
 
 // Coarse cell solid iff at least half of its 2^DIM children are solid
-// (uaamg_preconditioner_3d.cpp:34-45; uaamg_preconditioner.cpp:43-53).
+// (uaamg_preconditioner_3d.cpp:34-45; uaamg_preconditioner.cpp:43-53).  cover (the
+// covering aggregates of the solves, engine.cuh): solid iff none of its children is
+// a fluid cell of the level; a child past the last row of an odd-sized level (a ghost
+// cell) is none.
 template <int DIM>
 __global__ void k_restrict_solid(Geom f, const uint8_t* __restrict__ fs, Geom c,
-                                 uint8_t* __restrict__ cs) {
+                                 uint8_t* __restrict__ cs, int cover) {
     pdl_entry();
     int ic, jc, kc;
     if (!thread_cell<DIM>(c, ic, jc, kc)) return;
@@ -129,8 +132,10 @@ __global__ void k_restrict_solid(Geom f, const uint8_t* __restrict__ fs, Geom c,
         for (int dj = 0; dj < 2; ++dj)
 #pragma unroll
             for (int dk = 0; dk < (DIM == 3 ? 2 : 1); ++dk)
-                sc += fs[cidx(f, i_f + di, j_f + dj, k_f + dk)] != 0;
-    cs[cidx(c, ic, jc, kc)] = (uint8_t)(2 * sc >= (DIM == 3 ? 8 : 4));
+                sc += fs[cidx(f, i_f + di, j_f + dj, k_f + dk)] != 0 || i_f + di > f.nx ||
+                      j_f + dj > f.ny || (DIM == 3 && k_f + dk > f.nz);
+    const int all = DIM == 3 ? 8 : 4;
+    cs[cidx(c, ic, jc, kc)] = (uint8_t)(cover ? sc == all : 2 * sc >= all);
 }
 
 // Finest-level couplings from the mask (uaamg_preconditioner_3d.cpp:50-66):
@@ -259,6 +264,8 @@ __global__ void k_restrict(LevelView<T> F, Geom cg, const uint8_t* __restrict__ 
     for (int di = 0; di < 2; ++di)
         for (int dj = 0; dj < 2; ++dj)
             for (int dk = 0; dk < (DIM == 3 ? 2 : 1); ++dk) {
+                // (covering aggregates of an odd-sized level: no such child)
+                if (i_f + di > F.g.nx || j_f + dj > F.g.ny || (DIM == 3 && k_f + dk > F.g.nz)) continue;
                 const int fid = cidx(F.g, i_f + di, j_f + dj, k_f + dk);
                 if (F.solid[fid]) continue;
                 const T d = diag_at<DIM>(F, fid);
@@ -287,6 +294,7 @@ __global__ void k_prolong(Geom cg, const uint8_t* __restrict__ cs, const T* __re
     for (int di = 0; di < 2; ++di)
         for (int dj = 0; dj < 2; ++dj)
             for (int dk = 0; dk < (DIM == 3 ? 2 : 1); ++dk) {
+                if (i_f + di > fg.nx || j_f + dj > fg.ny || (DIM == 3 && k_f + dk > fg.nz)) continue;
                 const int fid = cidx(fg, i_f + di, j_f + dj, k_f + dk);
                 if (!fs[fid]) fx[fid] += val;
             }

@@ -4,8 +4,8 @@
 #include "engine.cuh"
 
 namespace uaamg {
-Engine* create_engine_f32(int mixed) {
-    if (mixed) return new EngineT<float, __half>(true);
-    return new EngineT<float, float>(false);
+Engine* create_engine_f32(int mixed, int apply_only) {
+    if (mixed) return new EngineT<float, __half>(true, !apply_only, apply_only != 0);
+    return new EngineT<float, float>(false, !apply_only, apply_only != 0);
 }
 }  // namespace uaamg

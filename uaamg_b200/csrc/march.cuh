@@ -395,6 +395,15 @@ __device__ __forceinline__ void zrange(const Geom& g, int zc, int& kb, int& ke) 
     }
 }
 
+// The same for a march that restricts to the level cg: when cg has more than half of
+// this level's planes (covering aggregates, an odd number of planes), the last chunk
+// also walks the ghost plane nz + 1 (all zeros), which completes the last children set.
+template <int DIM>
+__device__ __forceinline__ void zrange_restrict(const Geom& g, const Geom& cg, int zc, int& kb, int& ke) {
+    zrange<DIM>(g, zc, kb, ke);
+    if (DIM == 3 && 2 * cg.nz > g.nz) ke = min(kb + zc, g.nz + 2);
+}
+
 // The thread's pair: cells A = (i, j) and B = (i, j + 1), lane = column, warp w =
 // tile rows 2w and 2w + 1.  A and B have opposite colours on every plane; the
 // lanes of a warp read consecutive words of a box row.
@@ -569,7 +578,7 @@ __global__ void __launch_bounds__(kThreads) k_restrict_res(const __grid_constant
     const int tid = threadIdx.x;
     const Pair o = own_pair<T>(g);
     int kb, ke;
-    zrange<DIM>(g, L.zc, kb, ke);
+    zrange_restrict<DIM>(g, L.cg, L.zc, kb, ke);
     MRing<DIM, S, P> R{reinterpret_cast<uint64_t*>(sm), sm + Lay::OFF_RING,
                        DIM == 3 ? kb - 1 : 0, DIM == 3 ? ke : 0};
     if (FINE) build_lut<DIM, T>(lut, L.idx2, L.idy2, L.idz2);

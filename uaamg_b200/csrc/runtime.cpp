@@ -94,7 +94,7 @@ struct DevProblem {
             cudaGetLastError();
             return E_OOM;
         }
-        eng = p == PREC_FP64 ? create_engine_f64() : create_engine_f32(p == PREC_MIXED);
+        eng = p == PREC_FP64 ? create_engine_f64() : create_engine_f32(p == PREC_MIXED, 0);
         if (!eng) return E_OOM;
         eng->set_stream(stream);
         return E_OK;
@@ -148,7 +148,8 @@ std::vector<int> tune_schedule(DevProblem& d, const uaamg_problem& p, const uaam
                 ++inner;
             }
     const int bucket = (int)(20.0 * (double)solid / (double)(inner ? inner : 1) + 0.5);
-    const std::string key = "nu|" + tune_gpu_id() + "|" +
+    // (v2: schedules timed on the covering aggregates)
+    const std::string key = "nu|v2|" + tune_gpu_id() + "|" +
                             (o.precision == PREC_MIXED ? "mixed" : "f32") + "|" + std::to_string(p.dim) +
                             "|" + std::to_string(p.nx) + "x" + std::to_string(p.ny) + "x" +
                             std::to_string(p.dim == 3 ? p.nz : 0) + "|s" + std::to_string(bucket);
@@ -440,7 +441,7 @@ uaamg_status uaamg_set_autotune(uaamg_handle* h, int on) {
     h->autotune = on ? 1 : 0;
     for (auto* e : h->eng)
         if (e) e->set_autotune(on != 0);
-    for (int q = 0; q < 3; ++q) h->ready[q] = false;  // re-tune at the next set-up
+    for (bool& r : h->ready) r = false;  // re-tune at the next set-up
     return UAAMG_OK;
 }
 
