@@ -440,6 +440,9 @@ private:
     int nu_fine_ = 1, nu_coarse_ = 1;  // pre- and post-smoothing sweeps: finest / coarse levels
     int tail_lt_ = 0;        // first level of the small-level kernel
     int tail_nc_ = 0;        // 1: the hierarchy has a tail (0: it does not fit the kernel)
+    T* dense_ = nullptr;      // the tail's cycle as a matrix (n rows, stride ld)
+    int* dense_cell_ = nullptr;
+    int dense_n_ = 0, dense_ld_ = 0;
     size_t tail_smem_ = 0;   // its dynamic shared memory (x and b of every tail level)
     cudaStream_t cap_ = nullptr;      // capture stream
     cudaGraphExec_t gexec_ = nullptr; // two PCG iterations
@@ -543,6 +546,9 @@ private:
         r_ = z_ = p_ = p2_ = ap_ = xlo_ = nullptr;
         b64_ = xd_ = partials_ = nullptr;
         vf_[0] = vf_[1] = vf_[2] = nullptr;
+        dense_ = nullptr;
+        dense_cell_ = nullptr;
+        dense_n_ = 0;
         vconv_ = -1;
         err_ = nullptr;
         cg_ = nullptr;
@@ -915,6 +921,7 @@ private:
         }
         if ((e = sync_check()) != E_OK) return e;
         if ((e = tail_setup<DIM>()) != E_OK) return e;
+        if ((e = dense_setup<DIM>()) != E_OK) return e;
         if (DIM == 3 && autotune_) return tune<DIM>();
         return E_OK;
     }
@@ -953,14 +960,12 @@ private:
         return E_OK;
     }
 
-    // Levels tail_lt_ .. nl-1 of the V-cycle (b of tail_lt_ in, its x out).
     template <int DIM>
-    void tail_launch(const int* done) {
+    TailArgs<T> tail_args() const {
         const int nl = (int)lv_.size();
         TailArgs<T> a{};
         a.nlev = nl - tail_lt_;
         int off = 0;
-        double bytes = 0.0;
         for (int q = 0; q < a.nlev; ++q) {
             const LevelBuf<T, CS>& L = lv_[tail_lt_ + q];
             TailLevel<T>& t = a.lv[q];
@@ -979,13 +984,57 @@ private:
             t.b = L.b;
             t.rnx = 1.0f / (float)L.g.nx;
             t.rny = 1.0f / (float)L.g.ny;
-            // codes, couplings and diagonal read once per pass, four passes
-            bytes += 4.0 * cells(L.g) * ((1.0 + DIM) * sizeof(T) + 1.0);
         }
         a.smem_elems = off;
-        bytes += 2.0 * cells(lv_[tail_lt_].g) * sizeof(T);  // the first level's b in, x out
+        return a;
+    }
+
+    // The tail's cycle as a dense matrix (solves in FP32 and mixed; tail.cuh).  Its
+    // buffers have one size whatever the mask, so a mask change allocates nothing.
+    template <int DIM>
+    int dense_setup() {
+        dense_n_ = 0;
+        if constexpr (sizeof(T) == 4) {
+            if (!cover_ || tail_nc_ == 0 || cells(lv_[tail_lt_].g) > (double)kDenseCells) return E_OK;
+            const Geom& g = lv_[tail_lt_].g;
+            const int n = (int)cells(g);
+            dense_ld_ = (n + 3) / 4 * 4;
+            int e;
+            if ((e = alloc(dense_, (size_t)n * dense_ld_)) || (e = alloc(dense_cell_, (size_t)n))) return e;
+            UAAMG_LAUNCH((KTag{K_SETUP, tail_lt_, 0.0}), k_tail_cells<DIM>, 1, 256, g, dense_cell_);
+            UAAMG_LAUNCH_SMEM((KTag{K_SETUP, tail_lt_, 0.0}), (k_tail<DIM, T>), n, tail_threads<T>(),
+                              tail_smem_, tail_args<DIM>(), (const int*)nullptr, dense_, dense_ld_);
+            if ((e = sync_check()) != E_OK) return e;
+            dense_n_ = n;
+        }
+        return E_OK;
+    }
+
+    // Levels tail_lt_ .. nl-1 of the V-cycle (b of tail_lt_ in, its x out).
+    template <int DIM>
+    void tail_launch(const int* done) {
+        const LevelBuf<T, CS>& L0 = lv_[tail_lt_];
+        if constexpr (sizeof(T) == 4) {
+            if (dense_n_ > 0) {
+                const int n = dense_n_, nb = (n + 7) / 8, n4 = (dense_ld_ + 127) / 128;
+                // matrix, cell numbers and b in, x out
+                const KTag tag{K_TAIL, tail_lt_, (double)n * dense_ld_ * sizeof(T) + 12.0 * n};
+#define UAAMG_DENSE(N4)                                                                     \
+    UAAMG_LAUNCH(tag, k_tail_dense<N4>, nb, 256, n, dense_ld_, dense_, dense_cell_, L0.b, L0.x, done)
+                if (n4 <= 1) UAAMG_DENSE(1);
+                else if (n4 <= 2) UAAMG_DENSE(2);
+                else if (n4 <= 4) UAAMG_DENSE(4);
+                else UAAMG_DENSE(8);
+#undef UAAMG_DENSE
+                return;
+            }
+        }
+        double bytes = 2.0 * cells(L0.g) * sizeof(T);  // the first level's b in, x out
+        for (size_t l = tail_lt_; l < lv_.size(); ++l)
+            // codes, couplings and diagonal read once per pass, four passes
+            bytes += 4.0 * cells(lv_[l].g) * ((1.0 + DIM) * sizeof(T) + 1.0);
         UAAMG_LAUNCH_SMEM((KTag{K_TAIL, tail_lt_, bytes}), (k_tail<DIM, T>), 1, tail_threads<T>(),
-                          tail_smem_, a, done);
+                          tail_smem_, tail_args<DIM>(), done, (T*)nullptr, 0);
     }
 
     // Autotuner: for every level with marches, time its V-cycle marches (down and up,

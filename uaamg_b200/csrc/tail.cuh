@@ -33,6 +33,11 @@ constexpr size_t kTailSmemBytes = 200 * 1024;    // x and b of every tail level
 template <class T>
 constexpr int tail_threads() { return sizeof(T) == 8 ? 512 : 1024; }
 
+// Largest tail level whose whole cycle is kept as a dense matrix (k_tail_dense): 4 MB,
+// every level the tail takes by its cell count; a larger first level (a long thin
+// coarsest level) keeps the one-block kernel.
+constexpr int kDenseCells = 1024;
+
 template <class T>
 struct TailLevel {
     Geom g;          // the level's global (pitched) layout
@@ -338,9 +343,12 @@ __device__ void tail_coarsest(const TailView<DIM, T>& V) {
 
 // One block.  Levels lv[0 .. nlev-2] go down (forward sweep, restriction),
 // lv[nlev-1] is solved, then back up (prolongation + even colour, odd colour).
+// With dense given (set-up of k_tail_dense): block q runs the cycle on the unit vector
+// of the first level's interior cell q instead and writes its x as row q (stride ld).
 template <int DIM, class T>
 __global__ void __launch_bounds__(tail_threads<T>()) k_tail(const __grid_constant__ TailArgs<T> A,
-                                                            const int* __restrict__ done) {
+                                                            const int* __restrict__ done,
+                                                            T* __restrict__ dense, int ld) {
     pdl_entry();
     if (done && *done) return;
     extern __shared__ __align__(16) unsigned char tail_smem[];
@@ -354,7 +362,8 @@ __global__ void __launch_bounds__(tail_threads<T>()) k_tail(const __grid_constan
         for (int c = threadIdx.x; c < n; c += blockDim.x) {
             int i, j, k;
             tail_ijk<DIM>(L, c, i, j, k);
-            sm[L.bs + i + j * L.csx + k * L.csxy] = __ldg(L.b + cidx(L.g, i, j, k));
+            sm[L.bs + i + j * L.csx + k * L.csxy] =
+                dense ? T(c == (int)blockIdx.x) : __ldg(L.b + cidx(L.g, i, j, k));
         }
     }
     __syncthreads();
@@ -379,8 +388,72 @@ __global__ void __launch_bounds__(tail_threads<T>()) k_tail(const __grid_constan
         for (int c = threadIdx.x; c < n; c += blockDim.x) {
             int i, j, k;
             tail_ijk<DIM>(L, c, i, j, k);
-            L.x[cidx(L.g, i, j, k)] = sm[L.xs + i + j * L.csx + k * L.csxy];
+            const T x = sm[L.xs + i + j * L.csx + k * L.csxy];
+            if (dense) dense[(size_t)blockIdx.x * ld + c] = x;
+            else L.x[cidx(L.g, i, j, k)] = x;
         }
+    }
+}
+
+// The same cycle as one product x = M b.  From the tail's first level down the cycle is
+// a fixed linear map of its n <= kDenseCells cells, so the FP32 and mixed solves apply
+// its matrix, formed at set-up by running k_tail on every unit vector (n blocks, 40-90
+// us once per mask), instead of some 60 dependent phases in one block.  M is symmetric
+// (forward and reverse sweeps are adjoint), so its rows as written serve as its rows as
+// read.  A warp owns a row; the row's entries and the cell numbers do not depend on the
+// kernel before, so they are loaded ahead of the dependency wait and only b's latency
+// remains on the chain.  Bound by launch and L2 latency: 256^3 (n = 512) 21.1 -> 6.6 us
+// a launch (timed with an event pair around it, about 5 us of it theirs); a solve of
+// 384^2 0.89 -> 0.72 ms, of 129 x 97 x 65 5.0 -> 4.3 ms.  Columns of inactive cells are
+// 0 and their b is finite.
+template <int N4>
+__global__ void __launch_bounds__(256) k_tail_dense(int n, int ld, const float* __restrict__ M,
+                                                    const int* __restrict__ cell,
+                                                    const float* __restrict__ b, float* __restrict__ x,
+                                                    const int* __restrict__ done) {
+    __shared__ __align__(16) float bs[128 * N4];
+    const int lane = threadIdx.x & 31, row = 8 * (int)blockIdx.x + (int)(threadIdx.x >> 5);
+    const int r = row < n ? row : n - 1;
+    const float4* mr = reinterpret_cast<const float4*>(M + (size_t)r * ld);
+    float4 m[N4];
+#pragma unroll
+    for (int q = 0; q < N4; ++q)
+        m[q] = 4 * (lane + 32 * q) < ld ? __ldg(mr + lane + 32 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    constexpr int NB = (128 * N4 + 255) / 256;
+    int cb[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int c = (int)threadIdx.x + 256 * q;
+        cb[q] = c < n ? __ldg(cell + c) : -1;
+    }
+    const int cx = __ldg(cell + r);
+    pdl_entry();
+    if (done && *done) return;
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int c = (int)threadIdx.x + 256 * q;
+        if (c < 128 * N4) bs[c] = cb[q] >= 0 ? b[cb[q]] : 0.f;
+    }
+    __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < N4; ++q) {
+        const float4 v = reinterpret_cast<const float4*>(bs)[lane + 32 * q];
+        s += (m[q].x * v.x + m[q].y * v.y) + (m[q].z * v.z + m[q].w * v.w);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0 && row < n) x[cx] = s;
+}
+
+// Cell numbers (level layout) of the first tail level's interior cells, x fastest.
+template <int DIM>
+__global__ void k_tail_cells(Geom g, int* cell) {
+    pdl_entry();
+    const int n = tail_ncell<DIM>(g);
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+        const int r = c / g.nx;
+        cell[c] = cidx(g, 1 + c % g.nx, 1 + (DIM == 3 ? r % g.ny : r), DIM == 3 ? 1 + r / g.ny : 0);
     }
 }
 
