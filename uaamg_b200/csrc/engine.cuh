@@ -33,6 +33,11 @@
 namespace uaamg {
 namespace {
 
+// Tensor maps of one box geometry over a level: b, codes, diagonal, couplings.
+struct BoxMaps {
+    CUtensorMap b, code, dg, cx, cy, cz;
+};
+
 template <class T, class CS>
 struct LevelBuf {
     Geom g;
@@ -50,13 +55,16 @@ struct LevelBuf {
     // plane-box tensor maps of the marches: b, x, codes, couplings, diagonal, and x
     // as the parent box read by the next-finer level's prolongation
     CUtensorMap mb, mx, mcode, mcx, mcy, mcz, mdg, mxq;
-    // boxes with a 2-cell ring for the fused marches (fused.cuh): b, codes, diagonal,
-    // couplings
-    CUtensorMap fb, fcode, fdg, fcx, fcy, fcz;
-    // small 3D levels: whole-tile boxes (fused.cuh k_level_box) and this level's x as
-    // their parent box
+    // boxes for the fused marches (fused.cuh) with a 2-cell ring (f) and, for the way down
+    // with STAR transfers, a 3-cell ring (fd); this level's x and codes as their parent
+    // boxes with STAR
+    BoxMaps f, fd;
+    CUtensorMap mxs, mps;
+    // small 3D levels: whole-tile boxes (fused.cuh k_level_box), likewise; this level's x
+    // as their parent box (bxq; STAR: x and codes bxs, bps)
     bool box = false;
-    CUtensorMap bb, bcode, bdg, bcx, bcy, bcz, bxq;
+    BoxMaps bx, bd;
+    CUtensorMap bxq, bxs, bps;
     T* trim = nullptr;  // coarse box levels: per box {d, c_x, c_y, c_z} or d = 0 (k_box_trim)
 };
 
@@ -391,6 +399,7 @@ public:
 private:
     bool mixed_;
     bool cover_ = false, apply_only_ = false;
+    bool star_ = false;  // the current hierarchy covers and its transfers reach face neighbours
     int dim_ = 0, dirichlet_ = 0;
     double dx_ = 1, dy_ = 1, dz_ = 1;
     Geom gref_;                      // the caller's (reference) layout of level 0
@@ -587,6 +596,26 @@ private:
                     DIM == 3 ? (unsigned)((g.nz + zc - 1) / zc) : 1u);
     }
 
+    // The tensor maps of level l's b (given), codes, diagonal and couplings with the boxes
+    // BT (T), BC (codes), BS (CS couplings) and BF (FP32 couplings), bz planes deep.
+    template <class B> static constexpr int box_rows(const B*) { return B::H; }
+    template <class E, int R> static constexpr int box_rows(const BBox<E, R>*) { return BBox<E, R>::N; }
+    template <int DIM, class BT, class BC, class BS, class BF>
+    bool box_maps(const LevelBuf<T, CS>& L, const T* b, int l, int bz, BoxMaps* m) const {
+        constexpr int H = box_rows((const BT*)nullptr);
+        bool ok = encode_level_map<T>(&m->b, b, L.g, DIM, BT::W, H, bz) &&
+                  encode_level_map<uint8_t>(&m->code, L.code, L.g, DIM, BC::W, H, bz);
+        if (l == 0) return ok;
+        ok = ok && encode_level_map<T>(&m->dg, L.dg, L.g, DIM, BT::W, H, bz);
+        if (L.c32)
+            return ok && encode_level_map<T>(&m->cx, L.cx, L.g, DIM, BF::W, H, bz) &&
+                   encode_level_map<T>(&m->cy, L.cy, L.g, DIM, BF::W, H, bz) &&
+                   (DIM == 2 || encode_level_map<T>(&m->cz, L.cz, L.g, DIM, BF::W, H, bz));
+        return ok && encode_level_map<CS>(&m->cx, L.hcx, L.g, DIM, BS::W, H, bz) &&
+               encode_level_map<CS>(&m->cy, L.hcy, L.g, DIM, BS::W, H, bz) &&
+               (DIM == 2 || encode_level_map<CS>(&m->cz, L.hcz, L.g, DIM, BS::W, H, bz));
+    }
+
     // Blocks of the whole-tile box kernels over level g: 8^3 tiles.
     static dim3 box_grid(const Geom& g) {
         return dim3((unsigned)((g.nx + kBT - 1) / kBT), (unsigned)((g.ny + kBT - 1) / kBT),
@@ -628,6 +657,15 @@ private:
             (e = smem_attr(k_level_box<T, FINE, CSL, true, false>, BPlan<T, CSL, FINE, true>::BYTES)) ||
             (e = smem_attr(k_level_box<T, FINE, CSL, true, true>, BPlan<T, CSL, FINE, true>::BYTES)))
             return e;
+        if constexpr (sizeof(T) == 4) {
+            if ((e = smem_attr(k_level_box<T, FINE, CSL, false, false, true>,
+                               BPlan<T, CSL, FINE, false, true>::BYTES)) ||
+                (e = smem_attr(k_level_box<T, FINE, CSL, true, false, true>,
+                               BPlan<T, CSL, FINE, true, true>::BYTES)) ||
+                (e = smem_attr(k_level_box<T, FINE, CSL, true, true, true>,
+                               BPlan<T, CSL, FINE, true, true>::BYTES)))
+                return e;
+        }
         return E_OK;
     }
 
@@ -641,6 +679,15 @@ private:
             (e = smem_attr(k_level_fused<DIM, T, FINE, CSL, true, true>,
                            FCfg<DIM, T, CSL, FINE, true>::BYTES)))
             return e;
+        if constexpr (sizeof(T) == 4) {
+            if ((e = smem_attr(k_level_fused<DIM, T, FINE, CSL, false, false, true>,
+                               FCfg<DIM, T, CSL, FINE, false, true>::BYTES)) ||
+                (e = smem_attr(k_level_fused<DIM, T, FINE, CSL, true, false, true>,
+                               FCfg<DIM, T, CSL, FINE, true, true>::BYTES)) ||
+                (e = smem_attr(k_level_fused<DIM, T, FINE, CSL, true, true, true>,
+                               FCfg<DIM, T, CSL, FINE, true, true>::BYTES)))
+                return e;
+        }
         return E_OK;
     }
 
@@ -664,6 +711,7 @@ private:
         // keep the reference's rule, and so do problems with Dirichlet walls (their wall
         // channel is defined by it).
         const bool cover = cover_ && !dirichlet_;
+        star_ = cover;
         const int up = cover ? 1 : 0;
         double hx = dx_, hy = dy_, hz = dz_;
         while (nx >= 2 && ny >= 2 && (DIM == 2 || nz >= 2)) {
@@ -804,47 +852,40 @@ private:
             if (ok && l > 0 && !L.c32)
                 ok = encode_level_map<CS>(&L.mcx, L.hcx, L.g, DIM, CW, BH, 1) &&
                      encode_level_map<CS>(&L.mcy, L.hcy, L.g, DIM, CW, BH, 1) &&
-                     (DIM == 2 || encode_level_map<CS>(&L.mcz, L.hcz, L.g, DIM, CW, BH, 1)) &&
-                     encode_level_map<CS>(&L.fcx, L.hcx, L.g, DIM, RBox<CS>::W, RBox<CS>::H, 1) &&
-                     encode_level_map<CS>(&L.fcy, L.hcy, L.g, DIM, RBox<CS>::W, RBox<CS>::H, 1) &&
-                     (DIM == 2 ||
-                      encode_level_map<CS>(&L.fcz, L.hcz, L.g, DIM, RBox<CS>::W, RBox<CS>::H, 1));
+                     (DIM == 2 || encode_level_map<CS>(&L.mcz, L.hcz, L.g, DIM, CW, BH, 1));
             if (ok && l > 0 && L.c32)  // FP32 couplings read as T
                 ok = encode_level_map<T>(&L.mcx, L.cx, L.g, DIM, BW, BH, 1) &&
                      encode_level_map<T>(&L.mcy, L.cy, L.g, DIM, BW, BH, 1) &&
-                     (DIM == 2 || encode_level_map<T>(&L.mcz, L.cz, L.g, DIM, BW, BH, 1)) &&
-                     encode_level_map<T>(&L.fcx, L.cx, L.g, DIM, RBox<T>::W, RBox<T>::H, 1) &&
-                     encode_level_map<T>(&L.fcy, L.cy, L.g, DIM, RBox<T>::W, RBox<T>::H, 1) &&
-                     (DIM == 2 ||
-                      encode_level_map<T>(&L.fcz, L.cz, L.g, DIM, RBox<T>::W, RBox<T>::H, 1));
+                     (DIM == 2 || encode_level_map<T>(&L.mcz, L.cz, L.g, DIM, BW, BH, 1));
             if (ok && l > 0)
                 ok = encode_level_map<T>(&L.mdg, L.dg, L.g, DIM, BW, BH, 1) &&
-                     encode_level_map<T>(&L.fdg, L.dg, L.g, DIM, RBox<T>::W, RBox<T>::H, 1) &&
                      encode_level_map<T>(&L.mxq, L.x, L.g, DIM, QBox<T>::W, QBox<T>::H, 1);
-            if (ok)
-                ok = encode_level_map<T>(&L.fb, b, L.g, DIM, RBox<T>::W, RBox<T>::H, 1) &&
-                     encode_level_map<uint8_t>(&L.fcode, L.code, L.g, DIM, RBox<uint8_t>::W,
-                                               RBox<uint8_t>::H, 1);
+            if (ok) ok = box_maps<DIM, RBox<T, 2>, RBox<uint8_t, 2>, RBox<CS, 2>, RBox<T, 2>>(L, b, l, 1, &L.f);
+            if constexpr (sizeof(T) == 4) {
+                if (ok && star_)
+                    ok = box_maps<DIM, RBox<T, 3>, RBox<uint8_t, 3>, RBox<CS, 3>, RBox<T, 3>>(L, b, l, 1, &L.fd);
+                if (ok && star_ && l > 0) {
+                    using B = SBox<T, DIM>;
+                    ok = encode_level_map<T>(&L.mxs, L.x, L.g, DIM, B::W, B::H, DIM == 3 ? 2 : 1) &&
+                         encode_level_map<uint8_t>(&L.mps, L.code, L.g, DIM, B::CW, B::CH, 1);
+                }
+            }
             if (ok && DIM == 3) {
-                // whole-tile boxes (small levels) and this level's x as the parent box of
-                // the next-finer level's box kernels
-                if (l > 0)
-                    ok = encode_level_map<T>(&L.bxq, L.x, L.g, DIM, BQBox<T>::W, 6, 6);
-                if (ok && L.box) {
-                    ok = encode_level_map<T>(&L.bb, b, L.g, DIM, BBox<T>::W, kBB, kBB) &&
-                         encode_level_map<uint8_t>(&L.bcode, L.code, L.g, DIM, BBox<uint8_t>::W, kBB,
-                                                   kBB);
-                    if (ok && l > 0) {
-                        ok = encode_level_map<T>(&L.bdg, L.dg, L.g, DIM, BBox<T>::W, kBB, kBB);
-                        if (ok && !L.c32)
-                            ok = encode_level_map<CS>(&L.bcx, L.hcx, L.g, DIM, BBox<CS>::W, kBB, kBB) &&
-                                 encode_level_map<CS>(&L.bcy, L.hcy, L.g, DIM, BBox<CS>::W, kBB, kBB) &&
-                                 encode_level_map<CS>(&L.bcz, L.hcz, L.g, DIM, BBox<CS>::W, kBB, kBB);
-                        if (ok && L.c32)
-                            ok = encode_level_map<T>(&L.bcx, L.cx, L.g, DIM, BBox<T>::W, kBB, kBB) &&
-                                 encode_level_map<T>(&L.bcy, L.cy, L.g, DIM, BBox<T>::W, kBB, kBB) &&
-                                 encode_level_map<T>(&L.bcz, L.cz, L.g, DIM, BBox<T>::W, kBB, kBB);
-                    }
+                // whole-tile boxes (small levels) and this level's x (STAR: and codes) as the
+                // parent box of the next-finer level's box kernels
+                if (l > 0) ok = encode_level_map<T>(&L.bxq, L.x, L.g, DIM, BQBox<T>::W, 6, 6);
+                if (ok && l > 0 && star_) {
+                    using B = BSBox<T>;
+                    ok = encode_level_map<T>(&L.bxs, L.x, L.g, DIM, B::W, B::N, B::N) &&
+                         encode_level_map<uint8_t>(&L.bps, L.code, L.g, DIM, B::CW, B::CN, B::CN);
+                }
+                if (ok && L.box)
+                    ok = box_maps<DIM, BBox<T, 2>, BBox<uint8_t, 2>, BBox<CS, 2>, BBox<T, 2>>(
+                        L, b, l, BBox<T, 2>::N, &L.bx);
+                if constexpr (sizeof(T) == 4) {
+                    if (ok && L.box && star_)
+                        ok = box_maps<DIM, BBox<T, 3>, BBox<uint8_t, 3>, BBox<CS, 3>, BBox<T, 3>>(
+                            L, b, l, BBox<T, 3>::N, &L.bd);
                 }
             }
             if (!ok) return E_CUDA;
@@ -902,8 +943,9 @@ private:
                          Cl.solid, Cl.cx, Cl.cy, Cl.cz, Cl.wd, Cl.dg);
         }
         for (int l = 0; l < nl; ++l)
-            UAAMG_LAUNCH((KTag{K_SETUP, l, 0.0}), k_codes<DIM>, vec_grid(lv_[l].g), dim3(32, 8),
-                         lv_[l].g, lv_[l].solid, lv_[l].code, l == 0 ? 1 : 0);
+            UAAMG_LAUNCH((KTag{K_SETUP, l, 0.0}), (k_codes<DIM, T>), vec_grid(lv_[l].g), dim3(32, 8),
+                         lv_[l].g, lv_[l].solid, lv_[l].code, l == 0 ? 1 : 0,
+                         star_ && l > 0 ? lv_[l].cx : (const T*)nullptr, lv_[l].cy, lv_[l].cz);
         if constexpr (DIM == 3) {  // trimmed boxes of the coarse box levels
             for (int l = 1; l < nl; ++l) {
                 const LevelBuf<T, CS>& Cl = lv_[l];
@@ -912,11 +954,11 @@ private:
                 if (kHalf && !Cl.c32)
                     UAAMG_LAUNCH((KTag{K_SETUP, l, 0.0}), (k_box_trim<T, CS>), box_grid(Cl.g), 256,
                                  Cl.g, Cl.code, Cl.dg, Cl.hcx, Cl.hcy, Cl.hcz, m.csx, m.csy, m.csz,
-                                 Cl.trim);
+                                 Cl.trim, star_ ? 3 : 2);
                 else
                     UAAMG_LAUNCH((KTag{K_SETUP, l, 0.0}), (k_box_trim<T, T>), box_grid(Cl.g), 256,
                                  Cl.g, Cl.code, Cl.dg, Cl.cx, Cl.cy, Cl.cz, m.csx, m.csy, m.csz,
-                                 Cl.trim);
+                                 Cl.trim, star_ ? 3 : 2);
             }
         }
         if ((e = sync_check()) != E_OK) return e;
@@ -986,6 +1028,7 @@ private:
             t.rny = 1.0f / (float)L.g.ny;
         }
         a.smem_elems = off;
+        a.star = star_ ? 1 : 0;
         return a;
     }
 
@@ -1058,7 +1101,8 @@ private:
             const std::string key = "zc|" + tune_gpu_id() + "|" + (sizeof(T) == 8 ? "f64" : mixed_ ? "mixed" : "f32") +
                                     "|" + std::to_string(L.g.nx) + "x" + std::to_string(L.g.ny) + "x" +
                                     std::to_string(L.g.nz) + "|" + (l == 0 ? "fine" : "coarse") + "|" +
-                                    (fused_ && level_nu(l) == 1 ? "fused" : "four") + (L.c32 ? "|c32" : "");
+                                    (fused_ && level_nu(l) == 1 ? star_ ? "star" : "fused" : "four") +
+                                    (L.c32 ? "|c32" : "");
             {
                 std::vector<int> v;
                 if (tune_lookup(key, &v) && v.size() == 1 && v[0] >= 2 && v[0] <= 32) { L.zc = v[0]; continue; }
@@ -1175,6 +1219,7 @@ private:
         v.csz = half ? (T)(1.0 / (lv_[0].hz * lv_[0].hz)) : T(1);
         v.dirichlet = dirichlet_;
         v.zc = L.zc;
+        v.ccode = l + 1 < (int)lv_.size() ? lv_[l + 1].code : nullptr;
         return v;
     }
 
@@ -1199,38 +1244,41 @@ private:
         return m;
     }
 
-    // Tensor maps of a fused march over level l (boxes with a 2-cell ring); up: with
-    // the next-coarser level's x as parent boxes.
+    // Tensor maps of a fused march over level l; up: the way up, with the next-coarser
+    // level's x (STAR: and codes) as parent boxes.
     FMaps fmaps(int l, bool up) const {
         const LevelBuf<T, CS>& L = lv_[l];
+        const BoxMaps& f = star_ && !up ? L.fd : L.f;
         FMaps m{};
-        m.b = L.fb;
-        m.code = L.fcode;
+        m.b = f.b;
+        m.code = f.code;
         if (l > 0) {
-            m.dg = L.fdg;
-            m.cx = L.fcx;
-            m.cy = L.fcy;
-            m.cz = L.fcz;
+            m.dg = f.dg;
+            m.cx = f.cx;
+            m.cy = f.cy;
+            m.cz = f.cz;
         }
-        if (up) m.xc = lv_[l + 1].mxq;
+        if (up) m.xc = star_ ? lv_[l + 1].mxs : lv_[l + 1].mxq;
+        if (up && star_) m.pc = lv_[l + 1].mps;
         return m;
     }
 
-    // Tensor maps of a whole-tile box kernel over level l; up: with the next-coarser
-    // level's x as parent boxes.
+    // Tensor maps of a whole-tile box kernel over level l, likewise.
     BMaps bmaps(int l, bool up) const {
         const LevelBuf<T, CS>& L = lv_[l];
+        const BoxMaps& f = star_ && !up ? L.bd : L.bx;
         BMaps m{};
-        m.b = L.bb;
-        m.code = L.bcode;
+        m.b = f.b;
+        m.code = f.code;
         if (l > 0) {
-            m.dg = L.bdg;
-            m.cx = L.bcx;
-            m.cy = L.bcy;
-            m.cz = L.bcz;
+            m.dg = f.dg;
+            m.cx = f.cx;
+            m.cy = f.cy;
+            m.cz = f.cz;
             m.trim = trim_ ? L.trim : nullptr;
         }
-        if (up) m.xc = lv_[l + 1].bxq;
+        if (up) m.xc = star_ ? lv_[l + 1].bxs : lv_[l + 1].bxq;
+        if (up && star_) m.pc = lv_[l + 1].bps;
         return m;
     }
 
@@ -1246,6 +1294,45 @@ private:
 
     int level_nu(int l) const { return l == 0 ? nu_fine_ : nu_coarse_; }
 
+    // b, code (coarse levels: diagonal, couplings) in; coarse b out; whole-tile boxes on
+    // the small 3D levels, else the march
+    template <int DIM, bool FINE, class CSL, bool STAR>
+    void down_fused(int l, const int* done) {
+        const LevelBuf<T, CS>& L = lv_[l];
+        const LevelBuf<T, CS>& Cl = lv_[l + 1];
+        const double c = cells(L.g), cc = cells(Cl.g), t = sizeof(T);
+        const double coef = FINE ? 0.0 : DIM * (double)sizeof(CSL) + t;  // couplings + diagonal
+        const KTag tag{K_DOWN, l, c * (t + 1.0 + coef) + cc * t};
+        if (DIM == 3 && L.box)
+            UAAMG_LAUNCH_SMEM(tag, (k_level_box<T, FINE, CSL, false, false, STAR>), box_grid(L.g),
+                              dim3(kThreads), (BPlan<T, CSL, FINE, false, STAR>::BYTES), bmaps(l, false),
+                              mlevel(l), Cl.b, done, err_, partials_, cg_);
+        else
+            UAAMG_LAUNCH_SMEM(tag, (k_level_fused<DIM, T, FINE, CSL, false, false, STAR>),
+                              march_grid<DIM>(L.g, L.zc), dim3(kThreads),
+                              (FCfg<DIM, T, CSL, FINE, false, STAR>::BYTES), fmaps(l, false), mlevel(l),
+                              Cl.b, done, err_, partials_, cg_);
+    }
+
+    // b, code (coarse levels: diagonal, couplings), coarse x in; x out
+    template <int DIM, bool FINE, class CSL, bool ZDOT, bool STAR>
+    void up_fused(int l, const int* done) {
+        const LevelBuf<T, CS>& L = lv_[l];
+        const double c = cells(L.g), cc = cells(lv_[l + 1].g), t = sizeof(T);
+        const double coef = FINE ? 0.0 : DIM * (double)sizeof(CSL) + t;  // couplings + diagonal
+        const KTag tag{K_UP, l, c * (2.0 * t + 1.0 + coef) + cc * t};
+        T* x = l == 0 ? z_ : L.x;
+        if (DIM == 3 && L.box)
+            UAAMG_LAUNCH_SMEM(tag, (k_level_box<T, FINE, CSL, true, ZDOT, STAR>), box_grid(L.g),
+                              dim3(kThreads), (BPlan<T, CSL, FINE, true, STAR>::BYTES), bmaps(l, true),
+                              mlevel(l), x, done, err_, partials_, cg_);
+        else
+            UAAMG_LAUNCH_SMEM(tag, (k_level_fused<DIM, T, FINE, CSL, true, ZDOT, STAR>),
+                              march_grid<DIM>(L.g, L.zc), dim3(kThreads),
+                              (FCfg<DIM, T, CSL, FINE, true, STAR>::BYTES), fmaps(l, true), mlevel(l), x,
+                              done, err_, partials_, cg_);
+    }
+
     template <int DIM, bool FINE, class CSL>
     void down_level_cs(int l, const int* done) {
         const int nu = level_nu(l);
@@ -1256,20 +1343,11 @@ private:
         const dim3 grid = march_grid<DIM>(L.g, L.zc), blk(kThreads);
         // a finest level with Dirichlet walls takes the four-march path (the fused
         // finest level's branch-free cell table holds no wall terms)
-        if (DIM == 3 && L.box && fused_ && nu == 1 && !(FINE && dirichlet_)) {
-            // whole-tile boxes: b, code (coarse levels: diagonal, couplings) in; coarse b out
-            UAAMG_LAUNCH_SMEM((KTag{K_DOWN, l, c * (t + 1.0 + coef) + cc * t}),
-                              (k_level_box<T, FINE, CSL, false, false>), box_grid(L.g), blk,
-                              (BPlan<T, CSL, FINE, false>::BYTES), bmaps(l, false), mlevel(l), Cl.b,
-                              done, err_, partials_, cg_);
-            return;
-        }
         if (fused_ && nu == 1 && !(FINE && dirichlet_)) {
-            // b, code (coarse levels: diagonal, couplings) in; coarse b out
-            UAAMG_LAUNCH_SMEM((KTag{K_DOWN, l, c * (t + 1.0 + coef) + cc * t}),
-                              (k_level_fused<DIM, T, FINE, CSL, false, false>), grid, blk,
-                              (FCfg<DIM, T, CSL, FINE, false>::BYTES), fmaps(l, false), mlevel(l),
-                              Cl.b, done, err_, partials_, cg_);
+            if constexpr (sizeof(T) == 4) {
+                if (star_) { down_fused<DIM, FINE, CSL, true>(l, done); return; }
+            }
+            down_fused<DIM, FINE, CSL, false>(l, done);
             return;
         }
         T* x = l == 0 ? z_ : L.x;
@@ -1305,31 +1383,17 @@ private:
         const double coef = FINE ? 0.0 : DIM * (double)sizeof(CSL) + t;  // couplings + diagonal
         const dim3 grid = march_grid<DIM>(L.g, L.zc), blk(kThreads);
         T* x = l == 0 ? z_ : L.x;
-        if (DIM == 3 && L.box && fused_ && nu == 1 && !(FINE && dirichlet_)) {
-            // whole-tile boxes: b, code (coarse levels: diagonal, couplings), coarse x in;
-            // x out
-            const KTag tag{K_UP, l, c * (2.0 * t + 1.0 + coef) + cc * t};
-            if (FINE && zdot)
-                UAAMG_LAUNCH_SMEM(tag, (k_level_box<T, FINE, CSL, true, true>), box_grid(L.g), blk,
-                                  (BPlan<T, CSL, FINE, true>::BYTES), bmaps(l, true), mlevel(l), x, done,
-                                  err_, partials_, cg_);
-            else
-                UAAMG_LAUNCH_SMEM(tag, (k_level_box<T, FINE, CSL, true, false>), box_grid(L.g), blk,
-                                  (BPlan<T, CSL, FINE, true>::BYTES), bmaps(l, true), mlevel(l), x, done,
-                                  err_, partials_, cg_);
-            return;
-        }
         if (fused_ && nu == 1 && !(FINE && dirichlet_)) {
-            // b, code (coarse levels: diagonal, couplings), coarse x in; x out
-            const KTag tag{K_UP, l, c * (2.0 * t + 1.0 + coef) + cc * t};
-            if (FINE && zdot)
-                UAAMG_LAUNCH_SMEM(tag, (k_level_fused<DIM, T, FINE, CSL, true, true>), grid, blk,
-                                  (FCfg<DIM, T, CSL, FINE, true>::BYTES), fmaps(l, true), mlevel(l), x,
-                                  done, err_, partials_, cg_);
-            else
-                UAAMG_LAUNCH_SMEM(tag, (k_level_fused<DIM, T, FINE, CSL, true, false>), grid, blk,
-                                  (FCfg<DIM, T, CSL, FINE, true>::BYTES), fmaps(l, true), mlevel(l), x,
-                                  done, err_, partials_, cg_);
+            const bool zd = FINE && zdot;
+            if constexpr (sizeof(T) == 4) {
+                if (star_) {
+                    if (zd) up_fused<DIM, FINE, CSL, true, true>(l, done);
+                    else up_fused<DIM, FINE, CSL, false, true>(l, done);
+                    return;
+                }
+            }
+            if (zd) up_fused<DIM, FINE, CSL, true, false>(l, done);
+            else up_fused<DIM, FINE, CSL, false, false>(l, done);
             return;
         }
         UAAMG_LAUNCH_SMEM((KTag{K_UPE, l, c * (2.0 * t + 1.0 + coef) + cc * t}),

@@ -36,54 +36,94 @@
 // just relaxed, so its residual is 0, and an odd cell's is sum_n c_n x_n over its
 // (even) neighbours, since d x = b there; cells with d < 1e-30 (skipped by the
 // smoother) keep r = b.
+//
+// STAR (the FP32 and mixed solves on covering aggregates, engine.cuh): the transfers
+// between this level and the next coarser one are not constant per aggregate but
+// reach its face neighbours.  A fine cell takes 2 (x_c + w sum_a (x_n - x_c)), x_n the
+// coarse neighbour on the cell's own side along axis a where the coarse level couples
+// the two, and the restriction is the transpose: the sum of a coarse cell's residuals
+// plus w times, over its coupled faces, the difference between the residuals on the
+// far and on the near side of the face.  Constant transfers overshoot in directions
+// the smoother is weak in; with w = 1/5 the mixed solve of 129 x 97 x 65 with spacings
+// 1 : 1.5 : 0.67 takes 15 iterations instead of 46, of 256^3 10 instead of 15.  The
+// way down then needs the residual on the tile and a 1-cell ring and one plane either
+// side of the chunk, so its boxes have a 3-cell ring; the way up needs the parent
+// level's x in boxes one cell wider, two planes deep, and the parent's codes, whose
+// low six bits say which neighbours a coarse cell is coupled to.
 #pragma once
 #include "march.cuh"
 
 namespace uaamg {
 namespace {
 
-// Box of element type E around a tile with a 2-cell ring: cells
-// i in [i0-2, i0+33], j in [j0-2, j0+17] (i0 = 1 + 32 bx, j0 = 1 + 16 by) of one
-// plane.  The start column 32 bx - A is the 16-byte boundary at or below i0 - 2.
-template <class E>
+constexpr float kStarW = 0.2f;  // weight of a coupled face neighbour (1/4 is exact for linear
+                                // fields; 1/5 took as many iterations or one fewer)
+
+// Box of element type E around a tile with an R-cell ring: cells
+// i in [i0-R, i0+31+R], j in [j0-R, j0+15+R] (i0 = 1 + 32 bx, j0 = 1 + 16 by) of one
+// plane.  The start column 32 bx - A is a 16-byte boundary at or below i0 - R.
+template <class E, int R = 2>
 struct RBox {
-    static constexpr int A = 16 / (int)sizeof(E);          // elements per 16 bytes
-    static constexpr int W = (A + 35 + A - 1) / A * A;      // row width (elements)
-    static constexpr int H = kMY + 4;
+    static constexpr int A = 16 / (int)sizeof(E);              // elements per 16 bytes
+    static constexpr int W = (A + 33 + R + A - 1) / A * A;      // row width (elements)
+    static constexpr int H = kMY + 2 * R;
     static constexpr uint32_t BYTES = (uint32_t)(W * H * sizeof(E));
-    // position of the cell (i0 + di, j0 + dj), di in [-2, 33], dj in [-2, 17]
-    __host__ __device__ static constexpr int pos(int di, int dj) { return (dj + 2) * W + A + 1 + di; }
+    // position of the cell (i0 + di, j0 + dj), di in [-R, 31+R], dj in [-R, 15+R]
+    __host__ __device__ static constexpr int pos(int di, int dj) { return (dj + R) * W + A + 1 + di; }
+    static_assert(A >= R - 1, "the ring's first column lies in the box");
+};
+
+// STAR, way up: the parent level's x under a tile with a 2-cell ring and the face
+// neighbours of those parents: coarse columns [16 bx - A, ...], of which [16 bx - 1,
+// 16 bx + 18] are read, rows [8 by - 1, 8 by + 10], and in 3D the two planes kc - 1, kc
+// (odd k) or kc, kc + 1 (even k), kc = (k + 1) / 2; and the parents' codes: columns
+// [16 bx, 16 bx + 31], rows [8 by, 8 by + 9] of plane kc.
+template <class T, int DIM>
+struct SBox {
+    static constexpr int A = 16 / (int)sizeof(T);
+    static constexpr int W = (A + 19 + A - 1) / A * A;
+    static constexpr int H = kMY / 2 + 4;
+    static constexpr int PL = W * H;
+    static constexpr uint32_t BYTES = (uint32_t)(PL * (DIM == 3 ? 2 : 1) * sizeof(T));
+    static constexpr int CW = 32, CH = kMY / 2 + 2;
+    static constexpr uint32_t CBYTES = CW * CH;
 };
 
 // Tensor maps of a fused march (boxes of RBox geometry; xc: the parent level's x
-// in QBox geometry).
+// in QBox geometry, with STAR xc and pc the parent level's x and codes in SBox geometry).
 struct FMaps {
-    CUtensorMap b, code, dg, cx, cy, cz, xc;
+    CUtensorMap b, code, dg, cx, cy, cz, xc, pc;
 };
 
-// One ring stage: b, codes, [diagonal, couplings], [parent x].
-template <int DIM, class T, class CS, bool FINE, bool UP>
+// One ring stage: b, codes, [diagonal, couplings], [parent x, [parent codes]].
+template <int DIM, class T, class CS, bool FINE, bool UP, bool STAR>
 struct FPlan {
+    static constexpr int R = STAR && !UP ? 3 : 2;  // ring cells of the boxes
+    using BT = RBox<T, R>;
+    using BC = RBox<uint8_t, R>;
+    using BS = RBox<CS, R>;
     static constexpr int NC = FINE ? 0 : (DIM == 3 ? 3 : 2);
     static constexpr size_t OFF_B = 0;
-    static constexpr size_t OFF_CODE = align128(RBox<T>::BYTES);
-    static constexpr size_t OFF_DG = OFF_CODE + align128(RBox<uint8_t>::BYTES);
-    static constexpr size_t OFF_CX = OFF_DG + (FINE ? 0 : align128(RBox<T>::BYTES));
-    static constexpr size_t CB = align128(RBox<CS>::BYTES);
+    static constexpr size_t OFF_CODE = align128(BT::BYTES);
+    static constexpr size_t OFF_DG = OFF_CODE + align128(BC::BYTES);
+    static constexpr size_t OFF_CX = OFF_DG + (FINE ? 0 : align128(BT::BYTES));
+    static constexpr size_t CB = align128(BS::BYTES);
     static constexpr size_t OFF_CY = OFF_CX + CB, OFF_CZ = OFF_CY + CB;
     static constexpr size_t OFF_XC = OFF_CX + NC * CB;
-    static constexpr size_t STAGE = OFF_XC + (UP ? align128(QBox<T>::BYTES) : 0);
-    static constexpr uint32_t TX = RBox<T>::BYTES + RBox<uint8_t>::BYTES +
-                                   (FINE ? 0u : RBox<T>::BYTES + NC * RBox<CS>::BYTES) +
-                                   (UP ? QBox<T>::BYTES : 0u);
+    static constexpr uint32_t XCB = STAR ? SBox<T, DIM>::BYTES : QBox<T>::BYTES;
+    static constexpr size_t OFF_PC = OFF_XC + align128(XCB);
+    static constexpr size_t STAGE =
+        !UP ? OFF_XC : STAR ? OFF_PC + align128(SBox<T, DIM>::CBYTES) : OFF_PC;
+    static constexpr uint32_t TX = BT::BYTES + BC::BYTES + (FINE ? 0u : BT::BYTES + NC * BS::BYTES) +
+                                   (UP ? XCB + (STAR ? SBox<T, DIM>::CBYTES : 0u) : 0u);
 };
 
 // Ring depth and shared memory.  LAG: planes behind the step that stay resident
 // (the coarse levels read the -z coupling of plane s-2 in step 3); S >= LAG + 3
 // keeps the plane of the next step in flight during the current one.
-template <int DIM, class T, class CS, bool FINE, bool UP>
+template <int DIM, class T, class CS, bool FINE, bool UP, bool STAR = false>
 struct FCfg {
-    using P = FPlan<DIM, T, CS, FINE, UP>;
+    using P = FPlan<DIM, T, CS, FINE, UP, STAR>;
     static constexpr int LAG = FINE ? 1 : 2;
     static constexpr int S = DIM == 2 ? 1 : LAG + 3 + (FINE ? (UP ? 2 : 3) : 1);
     static constexpr int NXP = DIM == 2 ? 1 : 3;  // shared x planes
@@ -93,8 +133,12 @@ struct FCfg {
     static constexpr size_t OFF_TAB = OFF_LUT + align128(64 * sizeof(T));
     static constexpr size_t OFF_RING = OFF_TAB + (LEAN ? 128 * sizeof(float2) : 0);
     static constexpr size_t OFF_X = OFF_RING + S * P::STAGE;
-    static constexpr size_t XB = align128(RBox<T>::BYTES);
-    static constexpr size_t BYTES = OFF_X + NXP * XB;
+    static constexpr size_t XB = align128(P::BT::BYTES);
+    // STAR, way down: the residuals of a coarse plane's two fine planes, summed over
+    // them, on the tile and a 1-cell ring: cell (di, dj) at (dj + 1) RW + di + 2
+    static constexpr int RW = kMX + 4;
+    static constexpr size_t OFF_R = OFF_X + NXP * XB;
+    static constexpr size_t BYTES = OFF_R + (STAR && !UP ? align128(RW * (kMY + 2) * sizeof(T)) : 0);
     // resident blocks per SM the finest FP32 level is compiled for (registers): 3D,
     // five on the way down (its shared memory fits five) and four on the way up (at 48
     // registers the compiler recomputed values: 256^3, 74.3 M against 58.0 M warp
@@ -102,7 +146,7 @@ struct FCfg {
     // 69 us); 2D, eight (a full SM of 256-thread
     // blocks; the 2D way up at five blocks and 48 registers: 2048 x 1024 solve 10.24
     // against 9.99 ms)
-    static constexpr int MINB = LEAN ? (DIM == 3 ? (UP ? 4 : 5) : 8) : 1;
+    static constexpr int MINB = LEAN ? (DIM == 3 ? (UP || STAR ? 4 : 5) : 8) : 1;
     static_assert(S <= 16, "stage barriers: 128 bytes");
 };
 
@@ -111,18 +155,29 @@ struct FCfg {
 // and its colour on plane 0 ((i + j) & 1).
 struct FCell {
     int qt, qc, qs, qq;
+    int qk, side;  // STAR: the parent's code; bits 0 / 1: the cell is on its +x / +y side
+    int qr;        // STAR: position in the residual buffer
     int gid;
     bool in;
     int par;
 };
 
-template <class T, class CS>
+template <class P, class T, int DIM, bool STAR>
 __device__ __forceinline__ FCell fcell(const Geom& g, int i0, int j0, int di, int dj) {
     FCell c;
-    c.qt = RBox<T>::pos(di, dj);
-    c.qc = RBox<uint8_t>::pos(di, dj);
-    c.qs = RBox<CS>::pos(di, dj);
-    c.qq = ((dj + 2) >> 1) * QBox<T>::W + ((di + 2) >> 1);
+    c.qt = P::BT::pos(di, dj);
+    c.qc = P::BC::pos(di, dj);
+    c.qs = P::BS::pos(di, dj);
+    if constexpr (STAR) {
+        using B = SBox<T, DIM>;
+        c.qq = (((dj + 2) >> 1) + 1) * B::W + B::A + ((di + 2) >> 1);
+        c.qk = ((dj + 2) >> 1) * B::CW + ((di + 2) >> 1);
+        c.side = (di & 1) | ((dj & 1) << 1);
+        c.qr = (dj + 1) * (kMX + 4) + di + 2;
+    } else {
+        c.qq = ((dj + 2) >> 1) * QBox<T>::W + ((di + 2) >> 1);
+        c.qk = c.side = c.qr = 0;
+    }
     const int i = i0 + di, j = j0 + dj;
     c.gid = i + j * g.sx;
     c.in = i >= 1 && i <= g.nx && j >= 1 && j <= g.ny;
@@ -144,29 +199,57 @@ __device__ __forceinline__ void ring_pair(int t, int& d1i, int& d1j, int& d2i, i
 }
 constexpr int kRing1Tasks = 50, kRingTasks = 104;
 
-template <int DIM, class T, class CS, bool FINE, bool UP>
+// STAR, way down: the ring tasks of thread t by whole warps, so that no warp mixes
+// rings and each scheduler's two warps carry about as much: the 1-cell ring (50 pairs,
+// all three phases) on warps 0 and 1, the 2-cell ring (54, two phases) on 2 and 3, the
+// 3-cell ring (58, odd values only) on 6 and 7.  Returns the ring (0: none).
+__device__ __forceinline__ int star_ring_pair(int t, int& d1i, int& d1j, int& d2i, int& d2j) {
+    if (t < kRing1Tasks) { ring_pair(t, d1i, d1j, d2i, d2j); return 1; }
+    if (t >= 64 && t < 64 + kRingTasks - kRing1Tasks) {
+        ring_pair(t - 64 + kRing1Tasks, d1i, d1j, d2i, d2j);
+        return 2;
+    }
+    if (t >= 192 && t < 192 + 58) {
+        const int q = t - 192;
+        if (q < 19) { d1i = 2 * q - 3; d2i = 2 * q - 2; d1j = d2j = -3; }
+        else if (q < 38) { const int u = q - 19; d1i = 2 * u - 3; d2i = 2 * u - 2; d1j = d2j = kMY + 2; }
+        else if (q < 48) { const int u = q - 38; d1i = d2i = -3; d1j = 2 * u - 2; d2j = 2 * u - 1; }
+        else { const int u = q - 48; d1i = d2i = kMX + 2; d1j = 2 * u - 2; d2j = 2 * u - 1; }
+        return 3;
+    }
+    return 0;
+}
+
+template <int DIM, class T, class CS, bool FINE, bool UP, bool STAR>
 __device__ __forceinline__ void f_issue(const FMaps& M, unsigned char* st, uint64_t* bar, int k) {
-    using P = FPlan<DIM, T, CS, FINE, UP>;
-    const int x0 = kMX * (int)blockIdx.x, y0 = kMY * (int)blockIdx.y - 1;
+    using P = FPlan<DIM, T, CS, FINE, UP, STAR>;
+    const int x0 = kMX * (int)blockIdx.x, y0 = kMY * (int)blockIdx.y + 1 - P::R;
     fence_proxy_async();
     mbar_expect_tx(bar, P::TX);
-    tma_load<DIM>(st + P::OFF_B, &M.b, x0 - RBox<T>::A, y0, k, bar);
-    tma_load<DIM>(st + P::OFF_CODE, &M.code, x0 - RBox<uint8_t>::A, y0, k, bar);
+    tma_load<DIM>(st + P::OFF_B, &M.b, x0 - P::BT::A, y0, k, bar);
+    tma_load<DIM>(st + P::OFF_CODE, &M.code, x0 - P::BC::A, y0, k, bar);
     if constexpr (!FINE) {
-        tma_load<DIM>(st + P::OFF_DG, &M.dg, x0 - RBox<T>::A, y0, k, bar);
-        tma_load<DIM>(st + P::OFF_CX, &M.cx, x0 - RBox<CS>::A, y0, k, bar);
-        tma_load<DIM>(st + P::OFF_CY, &M.cy, x0 - RBox<CS>::A, y0, k, bar);
-        if constexpr (DIM == 3) tma_load<DIM>(st + P::OFF_CZ, &M.cz, x0 - RBox<CS>::A, y0, k, bar);
+        tma_load<DIM>(st + P::OFF_DG, &M.dg, x0 - P::BT::A, y0, k, bar);
+        tma_load<DIM>(st + P::OFF_CX, &M.cx, x0 - P::BS::A, y0, k, bar);
+        tma_load<DIM>(st + P::OFF_CY, &M.cy, x0 - P::BS::A, y0, k, bar);
+        if constexpr (DIM == 3) tma_load<DIM>(st + P::OFF_CZ, &M.cz, x0 - P::BS::A, y0, k, bar);
     }
-    if constexpr (UP)
-        tma_load<DIM>(st + P::OFF_XC, &M.xc, x0 / 2, (y0 + 1) / 2, (k + 1) >> 1, bar);
+    if constexpr (UP) {
+        const int yc = kMY / 2 * (int)blockIdx.y, kc = (k + 1) >> 1;
+        if constexpr (STAR) {
+            tma_load<DIM>(st + P::OFF_XC, &M.xc, x0 / 2 - SBox<T, DIM>::A, yc - 1, kc - (k & 1), bar);
+            tma_load<DIM>(st + P::OFF_PC, &M.pc, x0 / 2, yc, kc, bar);
+        } else {
+            tma_load<DIM>(st + P::OFF_XC, &M.xc, x0 / 2, yc, kc, bar);
+        }
+    }
 }
 
 // Planes p0 .. plast pass through S stages; plane p uses stage (p - p0) mod S.
 // Thread 0 issues every load and is the only thread that waits on the barriers.
-template <int DIM, class T, class CS, bool FINE, bool UP, int S>
+template <int DIM, class T, class CS, bool FINE, bool UP, bool STAR, int S>
 struct FRing {
-    using P = FPlan<DIM, T, CS, FINE, UP>;
+    using P = FPlan<DIM, T, CS, FINE, UP, STAR>;
     uint64_t* bars;
     unsigned char* base;
     int p0, plast;
@@ -181,12 +264,12 @@ struct FRing {
     __device__ void start(const FMaps& M) const {
         for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
         for (int p = p0; p < p0 + S && p <= plast; ++p)
-            f_issue<DIM, T, CS, FINE, UP>(M, at(p), &bars[(p - p0) % S], p);
+            f_issue<DIM, T, CS, FINE, UP, STAR>(M, at(p), &bars[(p - p0) % S], p);
     }
     // after a block barrier: plane `freed` is no longer read; load plane freed + S
     __device__ void refill(const FMaps& M, int freed) const {
         if (freed >= p0 && freed + S <= plast)
-            f_issue<DIM, T, CS, FINE, UP>(M, at(freed + S), &bars[(freed - p0) % S], freed + S);
+            f_issue<DIM, T, CS, FINE, UP, STAR>(M, at(freed + S), &bars[(freed - p0) % S], freed + S);
     }
 };
 
@@ -206,15 +289,17 @@ struct FHist {
         return;                                                                  \
     }
 
-template <int DIM, class T, bool FINE, class CS, bool UP, bool ZDOT>
-__global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
+template <int DIM, class T, bool FINE, class CS, bool UP, bool ZDOT, bool STAR = false>
+__global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::MINB))
     k_level_fused(const __grid_constant__ FMaps M, MLevel<T> L, T* __restrict__ out,
                   const int* __restrict__ done, int* err, double* partials, CGState* cg) {
     pdl_entry();
     if (done && *done) return;
-    using C = FCfg<DIM, T, CS, FINE, UP>;
+    using C = FCfg<DIM, T, CS, FINE, UP, STAR>;
     using P = typename C::P;
-    constexpr int S = C::S, WT = RBox<T>::W, WS = RBox<CS>::W;
+    constexpr int S = C::S, WT = P::BT::W, WS = P::BS::W;
+    constexpr bool kStarDn = STAR && !UP;
+    static_assert(!STAR || sizeof(T) == 4, "the FP64 form keeps the reference's transfers");
     constexpr bool kFull = sizeof(T) == 8;  // the reference's residual expression
     UAAMG_FUSED_SMEM(sm, err)
     T* lut = reinterpret_cast<T*>(sm + C::OFF_LUT);
@@ -285,43 +370,60 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
         if (DIM == 3) nb = nb + cc[4] * vp + cc[5] * vm;
         return nb;
     };
-    auto prolong = [&](const unsigned char* st, const FCell& c) -> T {
-        return T(2) * reinterpret_cast<const T*>(st + P::OFF_XC)[c.qq];
+    // kodd: the plane is odd (3D), i.e. the cell is on its parent's -z side
+    auto prolong = [&](const unsigned char* st, const FCell& c, auto kodd) -> T {
+        const T* xc = reinterpret_cast<const T*>(st + P::OFF_XC);
+        if constexpr (STAR) {
+            using B = SBox<T, DIM>;
+            constexpr bool KO = decltype(kodd)::value;
+            constexpr int own = DIM == 3 && KO ? B::PL : 0, oth = DIM == 3 && !KO ? B::PL : 0;
+            const uint32_t pc = st[P::OFF_PC + c.qk];
+            const bool px = c.side & 1, py = c.side & 2;
+            const T xo = xc[own + c.qq];
+            T g = (pc & (px ? 1u : 2u)) ? xc[own + c.qq + (px ? 1 : -1)] - xo : T(0);
+            g += (pc & (py ? 4u : 8u)) ? xc[own + c.qq + (py ? B::W : -B::W)] - xo : T(0);
+            if constexpr (DIM == 3) g += (pc & (KO ? 32u : 16u)) ? xc[oth + c.qq] - xo : T(0);
+            return T(2) * (xo + T(kStarW) * g);
+        } else {
+            return T(2) * xc[c.qq];
+        }
     };
     // odd-colour value at plane k: pre-smoothed (b + 0)/d, plus the prolongation on
     // the way up; 0 on cells that are not interior fluid
-    auto oval = [&](const unsigned char* st, const FCell& c, int k) -> T {
+    auto oval = [&](const unsigned char* st, const FCell& c, int k, auto kodd) -> T {
         if constexpr (LEAN) {
             const uint32_t code = code_at(st, c);
             const float2 t = tab[code & 127u];
-            if constexpr (UP) return b_at(st, c) * t.x + ((code & kActive) ? prolong(st, c) : T(0));
+            if constexpr (UP) return b_at(st, c) * t.x + ((code & kActive) ? prolong(st, c, kodd) : T(0));
             else return b_at(st, c) * t.x;
         }
         const uint32_t code = code_at(st, c);
         if (!(code & kActive)) return T(0);
         const T d = diag_of(st, c, code, k);
         const T pre = d < T(1e-30) ? T(0) : mdiv<T, CS>(b_at(st, c) + T(0), d);
-        if constexpr (UP) return pre + prolong(st, c);
+        if constexpr (UP) return pre + prolong(st, c, kodd);
         else return pre;
     };
     // even-colour value at plane k from the odd values around it: forward sweep
     // (way down) or first colour of the reverse sweep (way up; a skipped cell keeps
     // 0 + the prolongation)
     auto evalc = [&](const unsigned char* st, const unsigned char* stm, const T* xv, const FCell& c,
-                     int k, T op, T om) -> T {
+                     int k, T op, T om, auto kodd) -> T {
         if constexpr (LEAN) {
             const float2 t = tab[code_at(st, c) & 127u];
             const int q = c.qt;
             T nb = L.idx2 * (xv[q + 1] + xv[q - 1]) + L.idy2 * (xv[q + WT] + xv[q - WT]);
             if (DIM == 3) nb = nb + L.idz2 * (op + om);
-            if constexpr (UP) return (b_at(st, c) + nb) * t.x + t.y * prolong(st, c);
+            if constexpr (UP && STAR)
+                return (b_at(st, c) + nb) * t.x + (t.y != 0.f ? prolong(st, c, kodd) : T(0));
+            else if constexpr (UP) return (b_at(st, c) + nb) * t.x + t.y * prolong(st, c, kodd);
             else return (b_at(st, c) + nb) * t.x;
         }
         const uint32_t code = code_at(st, c);
         if (!(code & kActive)) return T(0);
         const T d = diag_of(st, c, code, k);
         if (d < T(1e-30)) {
-            if constexpr (UP) return T(0) + prolong(st, c);
+            if constexpr (UP) return T(0) + prolong(st, c, kodd);
             else return T(0);
         }
         T cc[6];
@@ -331,15 +433,26 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
 
     // --- tasks ---------------------------------------------------------------
     // tile pair: A = (i0 + lane, j0 + 2w), B = (i0 + lane, j0 + 2w + 1)
-    const FCell cA = fcell<T, CS>(g, i0, j0, lane, 2 * w);
-    const FCell cB = fcell<T, CS>(g, i0, j0, lane, 2 * w + 1);
-    const bool ring = tid < kRingTasks, ring1 = tid < kRing1Tasks;
+    const FCell cA = fcell<P, T, DIM, STAR>(g, i0, j0, lane, 2 * w);
+    const FCell cB = fcell<P, T, DIM, STAR>(g, i0, j0, lane, 2 * w + 1);
+    // this thread's ring pair: ring: it has one; ring_e: with even values; ring_f: with
+    // final results (the 1-cell ring of a STAR way down)
+    bool ring, ring_e, ring_f = false;
     FCell cR1, cR2;
     {
         int d1i = 0, d1j = 0, d2i = 0, d2j = 0;
-        if (ring) ring_pair(tid, d1i, d1j, d2i, d2j);
-        cR1 = fcell<T, CS>(g, i0, j0, d1i, d1j);
-        cR2 = fcell<T, CS>(g, i0, j0, d2i, d2j);
+        if constexpr (kStarDn) {
+            const int r = star_ring_pair(tid, d1i, d1j, d2i, d2j);
+            ring = r > 0;
+            ring_e = r == 1 || r == 2;
+            ring_f = r == 1;
+        } else {
+            ring = tid < kRingTasks;
+            ring_e = tid < kRing1Tasks;
+            if (ring) ring_pair(tid, d1i, d1j, d2i, d2j);
+        }
+        cR1 = fcell<P, T, DIM, STAR>(g, i0, j0, d1i, d1j);
+        cR2 = fcell<P, T, DIM, STAR>(g, i0, j0, d2i, d2j);
     }
     int kb, ke;
     if constexpr (UP) zrange<DIM>(g, L.zc, kb, ke);
@@ -350,16 +463,15 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
     const int jc = kMY / 2 * (int)blockIdx.y + 1 + w;
     const bool writer = !UP && (lane & 1) == 0 && ic <= L.cg.nx && jc <= L.cg.ny;
 
-    // Final step on the tile pair at plane k, in colour order: cO / cE are the pair's
-    // odd and even cells there, vO / vE their x values, zp* / zm* their columns'
-    // values at k+1 and k-1; aOdd: A is the odd cell.  rlo: the way down's dk = 0
-    // residuals, kept from the odd plane below.
-    auto final_pair = [&](auto kodd, const unsigned char* st, const unsigned char* stm, const T* xv,
-                          int k, const FCell& cO, const FCell& cE, bool aOdd, T vO, T vE, T zpO,
-                          T zmO, T zpE, T zmE, T (&rlo)[2]) {
-        constexpr bool KODD = decltype(kodd)::value;  // plane k is odd (3D)
+    // Final values of a pair at a plane, in colour order: cO / cE are its odd and even
+    // cells there, vO / vE their x values, zp* / zm* their columns' values one plane up and
+    // down.  resO / resE: the final x (way up) or the residuals (way down).
+    auto finals = [&](const unsigned char* st, const unsigned char* stm, const T* xv, int k,
+                      const FCell& cO, const FCell& cE, T vO, T vE, T zpO, T zmO, T zpE, T zmE,
+                      T& resO, T& resE) {
         const uint32_t kO = code_at(st, cO), kE = code_at(st, cE);
-        T resO = UP ? vO : T(0), resE = UP ? vE : T(0);
+        resO = UP ? vO : T(0);
+        resE = UP ? vE : T(0);
         if constexpr (LEAN) {
             const float2 tO = tab[kO & 127u];
             const int q = cO.qt;
@@ -412,6 +524,17 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
                 }
             }
         }
+    };
+
+    // Final step on the tile pair at plane k (finals); aOdd: A is the odd cell.  rlo: the
+    // way down's dk = 0 residuals, kept from the odd plane below.
+    auto final_pair = [&](auto kodd, const unsigned char* st, const unsigned char* stm, const T* xv,
+                          int k, const FCell& cO, const FCell& cE, bool aOdd, T vO, T vE, T zpO,
+                          T zmO, T zpE, T zmE, T (&rlo)[2]) {
+        [[maybe_unused]] constexpr bool KODD = decltype(kodd)::value;  // plane k is odd (3D)
+        T resO, resE;
+        finals(st, stm, xv, k, cO, cE, vO, vE, zpO, zmO, zpE, zmE, resO, resE);
+        const uint32_t kO = code_at(st, cO), kE = code_at(st, cE);
         if constexpr (UP) {
             const int base = k * g.sxy;
             const bool inO = cO.in, inE = cE.in;
@@ -476,6 +599,22 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
         }
     };
 
+    // STAR, way down.  rbuf holds the residuals summed over a coarse plane's two fine
+    // planes on the tile and its 1-cell ring; a writer lane (an even column) forms its
+    // coarse cell's sum and adds w times, per coupled face, the far minus the near
+    // side's sums; zt: the two z faces' part, the same way.
+    T* rbuf = reinterpret_cast<T*>(sm + C::OFF_R);
+    uint32_t ccode = 0;  // code of this writer's coarse cell of the plane in progress
+    auto star_write = [&](int kc, T zt) {
+        constexpr int RW = C::RW;
+        const T* r0 = rbuf + (2 * w + 1) * RW + lane + 2;  // row dj = 2 w, column lane
+        const T a0 = r0[0], a1 = r0[1], b0 = r0[RW], b1 = r0[RW + 1];
+        T q = (ccode & 2u) ? (r0[-1] + r0[RW - 1]) - (a0 + b0) : T(0);
+        q += (ccode & 1u) ? (r0[2] + r0[RW + 2]) - (a1 + b1) : T(0);
+        q += (ccode & 8u) ? (r0[-RW] + r0[1 - RW]) - (a0 + a1) : T(0);
+        q += (ccode & 4u) ? (r0[2 * RW] + r0[2 * RW + 1]) - (b0 + b1) : T(0);
+        out[cidx(L.cg, ic, jc, kc)] = ((a0 + a1) + (b0 + b1)) + T(kStarW) * (q + zt);
+    };
     T rlo[2] = {T(0), T(0)};
     if constexpr (DIM == 2) {
         // one plane: odd values, barrier, even values, barrier, final
@@ -484,7 +623,7 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
         bool ok = true;
         if (tid == 0) {
             mbar_init(bar, 1);
-            f_issue<DIM, T, CS, FINE, UP>(M, st, bar, 0);
+            f_issue<DIM, T, CS, FINE, UP, STAR>(M, st, bar, 0);
             ok = mbar_wait(bar, 0u, kTmaWaitLimit);
         }
         if (!step_barrier(ok, err)) return;
@@ -493,22 +632,46 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
         const FCell tO = oddA ? cA : cB, tE = oddA ? cB : cA;
         const bool odd1 = cR1.par != 0;
         const FCell rO = odd1 ? cR1 : cR2, rE = odd1 ? cR2 : cR1;
-        const T ot = oval(st, tO, 0);
+        const std::false_type even;
+        const T ot = oval(st, tO, 0, even);
         xpl[tO.qt] = ot;
-        if (ring) xpl[rO.qt] = oval(st, rO, 0);
+        T otr = T(0), etr = T(0);
+        if (ring) {
+            otr = oval(st, rO, 0, even);
+            xpl[rO.qt] = otr;
+        }
         __syncthreads();
-        const T et = evalc(st, st, xpl, tE, 0, T(0), T(0));
+        const T et = evalc(st, st, xpl, tE, 0, T(0), T(0), even);
         xpl[tE.qt] = et;
-        if (ring1) xpl[rE.qt] = evalc(st, st, xpl, rE, 0, T(0), T(0));
+        if (ring_e) {
+            etr = evalc(st, st, xpl, rE, 0, T(0), T(0), even);
+            xpl[rE.qt] = etr;
+        }
         __syncthreads();
-        final_pair(std::false_type(), st, st, xpl, 0, tO, tE, oddA, ot, et, T(0), T(0), T(0), T(0),
-                   rlo);
+        if constexpr (kStarDn) {
+            T rA, rB;
+            if (writer) ccode = L.ccode[cidx(L.cg, ic, jc, 0)];
+            finals(st, st, xpl, 0, tO, tE, ot, et, T(0), T(0), T(0), T(0), rA, rB);
+            rbuf[tO.qr] = rA;
+            rbuf[tE.qr] = rB;
+            if (ring_f) {
+                finals(st, st, xpl, 0, rO, rE, otr, etr, T(0), T(0), T(0), T(0), rA, rB);
+                rbuf[rO.qr] = rA;
+                rbuf[rE.qr] = rB;
+            }
+            __syncthreads();
+            if (writer) star_write(0, T(0));
+        } else {
+            final_pair(even, st, st, xpl, 0, tO, tE, oddA, ot, et, T(0), T(0), T(0), T(0), rlo);
+        }
     } else {
         // steps s = kb-3 .. ke: odd values of planes kb-2 .. ke+1, even values of
         // kb-1 .. ke, final results of kb .. ke-1
-        const int s0 = kb - 3;
-        FRing<DIM, T, CS, FINE, UP, S> R{reinterpret_cast<uint64_t*>(sm), sm + C::OFF_RING, kb - 2,
-                                         ke + 1};
+        // (a STAR way down: final results of kb-1 .. ke, so one step more at either end)
+        constexpr int X = kStarDn ? 1 : 0;
+        const int s0 = kb - 3 - X, sl = ke + X;
+        FRing<DIM, T, CS, FINE, UP, STAR, S> R{reinterpret_cast<uint64_t*>(sm), sm + C::OFF_RING,
+                                               s0 + 1, sl + 1};
         bool ok = true;
         if (tid == 0) {
             R.start(M);
@@ -522,6 +685,10 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
         const FCell q0 = r1Role0 ? cR1 : cR2, q1 = r1Role0 ? cR2 : cR1;
         FHist<T> ht[2] = {{T(0), T(0), T(0)}, {T(0), T(0), T(0)}};
         T hr[2] = {T(0), T(0)};  // ring columns: last odd value
+        // STAR way down: the ring columns' last even value and dk = 0 residuals (by role),
+        // the tile pair's residual sum on the even plane below, and on the z face below
+        // the coarse plane in progress the difference of the two sides' sums
+        T he[2] = {T(0), T(0)}, hlo[2] = {T(0), T(0)}, te = T(0), gz = T(0);
         // stages of planes s+1, s, s-1, s-2 and the shared x planes s+1, s, s-1,
         // rotated once per step (planes below p0 are never read)
         const unsigned char* ring_end = sm + C::OFF_RING + S * P::STAGE;
@@ -539,32 +706,77 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
             constexpr int RC = decltype(R0c)::value, RO = 1 - RC, PH = decltype(PHc)::value;
             const bool run_even = PH == 0 ? s >= kb - 1 : PH >= 2;
             const bool run_final = PH == 0 ? s >= kb + 1 : PH == 3;
+            // planes s+1 and s-1 are odd, plane s is even, or the other way round (s0 is
+            // even, for a STAR way down odd)
+            using Odd1 = std::integral_constant<bool, (RC == 0) != (X != 0)>;
+            using Odd0 = std::integral_constant<bool, !Odd1::value>;
             const FCell& tc = RC == 0 ? t0 : t1;
             const FCell& qc = RC == 0 ? q0 : q1;
             // 1. odd values of plane s+1
-            const T on = oval(sp1, tc, s + 1);
+            const T on = oval(sp1, tc, s + 1, Odd1());
             xn[tc.qt] = on;
             T onr = T(0);
             if (ring) {
-                onr = oval(sp1, qc, s + 1);
+                onr = oval(sp1, qc, s + 1, Odd1());
                 xn[qc.qt] = onr;
             }
             // 2. even values of plane s
-            T en = T(0);
+            T en = T(0), enr = T(0);
             if (run_even) {
-                en = evalc(s00, sm1, xc, tc, s, on, ht[RC].o1);
+                en = evalc(s00, sm1, xc, tc, s, on, ht[RC].o1, Odd0());
                 xc[tc.qt] = en;
-                if (ring1) xc[qc.qt] = evalc(s00, sm1, xc, qc, s, onr, hr[RC]);
+                if (ring_e) {
+                    enr = evalc(s00, sm1, xc, qc, s, onr, hr[RC], Odd0());
+                    xc[qc.qt] = enr;
+                }
             }
-            // 3. final results of plane s-1: the role-RC cell is odd there (plane s-1 is
-            // odd for role 0: s0 = kb - 3 is even)
-            if (run_final) {
+            // 3. final results of plane s-1: the role-RC cell is odd there
+            if constexpr (kStarDn) {
+                if (run_final) {
+                    const int p = s - 1;
+                    constexpr bool KODD = Odd1::value;
+                    T rO, rE;
+                    finals(sm1, sm2, xo, p, tc, RC == 0 ? t1 : t0, ht[RC].o1, ht[RO].e1, en, ht[RC].e1,
+                           ht[RO].o1, ht[RO].o2, rO, rE);
+                    const T t = rO + rE;
+                    if constexpr (KODD) {  // dk = 0; the coarse plane below is complete
+                        const T g = te - t;
+                        if (p > kb) {
+                            T zt = ((ccode & 32u) ? gz : T(0)) - ((ccode & 16u) ? g : T(0));
+                            const uint32_t cn = __shfl_up_sync(0xffffffffu, ccode, 1);
+                            const T zo = ((cn & 32u) ? gz : T(0)) - ((cn & 16u) ? g : T(0));
+                            zt += __shfl_down_sync(0xffffffffu, zo, 1);
+                            if (writer) star_write((p - 1) / 2, zt);
+                        }
+                        gz = g;
+                        rlo[RC] = rO;
+                        rlo[RO] = rE;
+                    } else {  // dk = 1: the sums over both planes
+                        te = t;
+                        rbuf[tc.qr] = rlo[RC] + rO;
+                        rbuf[(RC == 0 ? t1 : t0).qr] = rlo[RO] + rE;
+                        if (writer) ccode = L.ccode[cidx(L.cg, ic, jc, p / 2)];
+                    }
+                    if (ring_f) {
+                        const FCell& qo = RC == 0 ? q1 : q0;
+                        finals(sm1, sm2, xo, p, qc, qo, T(0), T(0), enr, he[RC], T(0), T(0), rO, rE);
+                        if constexpr (KODD) {
+                            hlo[RC] = rO;
+                            hlo[RO] = rE;
+                        } else {
+                            rbuf[qc.qr] = hlo[RC] + rO;
+                            rbuf[qo.qr] = hlo[RO] + rE;
+                        }
+                    }
+                }
+                he[RC] = enr;
+            } else if (run_final) {
                 const int p = s - 1;
                 const T vR = ht[RC].o1, vO = ht[RO].e1;   // x at p
                 const T zpR = en, zmR = ht[RC].e1;         // role RC: even values at p+1, p-1
                 const T zpO = ht[RO].o1, zmO = ht[RO].o2;  // role RO: odd values at p+1, p-1
                 const FCell& to = RC == 0 ? t1 : t0;
-                final_pair(std::integral_constant<bool, RC == 0>(), sm1, sm2, xo, p, tc, to,
+                final_pair(Odd1(), sm1, sm2, xo, p, tc, to,
                            aRole0 == (RC == 0), vR, vO, zpR, zmR, zpO, zmO, rlo);
             }
             ht[RC].o2 = ht[RC].o1;
@@ -598,18 +810,18 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
                 if (s + 1 <= ke && !step(s + 1, R1(), std::integral_constant<int, 0>())) return;
             }
         } else {
-            // steps kb-3 .. kb fill the pipeline: odd and even values only (the even
-            // values of planes kb-3, kb-2 are not needed; their shared positions are
-            // written again before any read); then ke >= kb + 1 steps run all three
+            // four steps fill the pipeline: odd and even values only (the even values of
+            // the first two planes are not needed; their shared positions are written
+            // again before any read); then two or more steps run all three
 #pragma unroll 1
-            for (int s = s0; s <= kb; s += 2) {
+            for (int s = s0; s < s0 + 4; s += 2) {
                 if (!step(s, R0(), std::integral_constant<int, 2>())) return;
                 if (!step(s + 1, R1(), std::integral_constant<int, 2>())) return;
             }
 #pragma unroll 1
-            for (int s = kb + 1; s <= ke; s += 2) {
+            for (int s = s0 + 4; s <= sl; s += 2) {
                 if (!step(s, R0(), std::integral_constant<int, 3>())) return;
-                if (s + 1 <= ke && !step(s + 1, R1(), std::integral_constant<int, 3>())) return;
+                if (s + 1 <= sl && !step(s + 1, R1(), std::integral_constant<int, 3>())) return;
             }
         }
     }
@@ -629,17 +841,17 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP>::MINB))
 // the reverse sweep, the store, and on the finest level the z sums), with one block
 // barrier between the phases.  Per-cell expressions are those of k_level_fused.
 constexpr int kBT = 8;               // tile edge
-constexpr int kBB = kBT + 4;         // box edge (2-cell ring)
 
-// Box of element type E: cells i in [i0-2, i0+9] (i0 = 1 + 8 bx), the start column
-// 8 bx - A rounded to 16 bytes; rows and planes 12.
-template <class E>
+// Box of element type E: cells i in [i0-R, i0+7+R] (i0 = 1 + 8 bx; R = 2, on the STAR way
+// down 3), the start column 8 bx - A rounded to 16 bytes; 8 + 2 R rows and planes.
+template <class E, int R = 2>
 struct BBox {
     static constexpr int A = 16 / (int)sizeof(E);
-    static constexpr int W = (A + kBB - 1 + A - 1) / A * A;
-    static constexpr uint32_t BYTES = (uint32_t)(W * kBB * kBB * sizeof(E));
+    static constexpr int N = kBT + 2 * R;  // box edge
+    static constexpr int W = (A + kBT + R + 1 + A - 1) / A * A;
+    static constexpr uint32_t BYTES = (uint32_t)(W * N * N * sizeof(E));
     __host__ __device__ static constexpr int pos(int di, int dj, int dk) {
-        return ((dk + 2) * kBB + (dj + 2)) * W + A + 1 + di;
+        return ((dk + R) * N + (dj + R)) * W + A + 1 + di;
     }
 };
 // Parent box (coarse x under the box): coarse cells [4 bx, 4 bx + 5] per axis.
@@ -648,29 +860,50 @@ struct BQBox {
     static constexpr int W = (6 * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T);
     static constexpr uint32_t BYTES = (uint32_t)(W * 6 * 6 * sizeof(T));
 };
+// STAR: parent box with the parents' face neighbours: coarse columns [4 bx - 4, ...], of
+// which [4 bx - 1, 4 bx + 6] are read, rows and planes [4 by - 1, 4 by + 6]; and the
+// parents' codes: columns from the 16-byte boundary at or below 4 bx, rows and planes
+// [4 by, 4 by + 5].
+template <class T>
+struct BSBox {
+    static constexpr int W = 12, N = 8;
+    static constexpr uint32_t BYTES = (uint32_t)(W * N * N * sizeof(T));
+    static constexpr int CW = 32, CN = 6;
+    static constexpr uint32_t CBYTES = CW * CN * CN;
+};
 
-template <class T, class CS, bool FINE, bool UP>
+template <class T, class CS, bool FINE, bool UP, bool STAR = false>
 struct BPlan {
+    static constexpr int R = STAR && !UP ? 3 : 2;
+    using BT = BBox<T, R>;
+    using BC = BBox<uint8_t, R>;
+    using BS = BBox<CS, R>;
+    static constexpr uint32_t XCB = STAR ? BSBox<T>::BYTES : BQBox<T>::BYTES;
     static constexpr size_t OFF_B = 0;
-    static constexpr size_t OFF_CODE = align128(BBox<T>::BYTES);
-    static constexpr size_t OFF_DG = OFF_CODE + align128(BBox<uint8_t>::BYTES);
-    static constexpr size_t CB = align128(BBox<CS>::BYTES);
-    static constexpr size_t OFF_CX = OFF_DG + (FINE ? 0 : align128(BBox<T>::BYTES));
+    static constexpr size_t OFF_CODE = align128(BT::BYTES);
+    static constexpr size_t OFF_DG = OFF_CODE + align128(BC::BYTES);
+    static constexpr size_t CB = align128(BS::BYTES);
+    static constexpr size_t OFF_CX = OFF_DG + (FINE ? 0 : align128(BT::BYTES));
     static constexpr size_t OFF_CY = OFF_CX + CB, OFF_CZ = OFF_CY + CB;
     static constexpr size_t OFF_XC = OFF_CX + (FINE ? 0 : 3 * CB);
-    static constexpr size_t OFF_X = OFF_XC + (UP ? align128(BQBox<T>::BYTES) : 0);
-    static constexpr size_t OFF_BAR = OFF_X + align128(BBox<T>::BYTES);
+    static constexpr size_t OFF_PC = OFF_XC + (UP ? align128(XCB) : 0);
+    static constexpr size_t OFF_X = OFF_PC + (UP && STAR ? align128(BSBox<T>::CBYTES) : 0);
+    // STAR, way down: residuals on the tile and its 1-cell ring
+    static constexpr int RN = kBT + 2;
+    static constexpr size_t OFF_R = OFF_X + align128(BT::BYTES);
+    static constexpr size_t OFF_BAR = OFF_R + (STAR && !UP ? align128(RN * RN * RN * sizeof(T)) : 0);
     static constexpr size_t OFF_LUT = OFF_BAR + 128;
     static constexpr size_t BYTES = OFF_LUT + align128(64 * sizeof(T));
-    static constexpr uint32_t TX = BBox<T>::BYTES + BBox<uint8_t>::BYTES +
-                                   (FINE ? 0u : BBox<T>::BYTES + 3 * BBox<CS>::BYTES) +
-                                   (UP ? BQBox<T>::BYTES : 0u);
+    // the parent x and codes are loaded for trimmed boxes too
+    static constexpr uint32_t TXP = UP ? XCB + (STAR ? BSBox<T>::CBYTES : 0u) : 0u;
+    static constexpr uint32_t TX =
+        BT::BYTES + BC::BYTES + (FINE ? 0u : BT::BYTES + 3 * BS::BYTES) + TXP;
 };
 
 // Tensor maps of a box kernel: b, codes, diagonal, couplings (BBox geometry), and the
-// parent level's x (BQBox geometry).
+// parent level's x (BQBox geometry; STAR: x and codes in BSBox geometry).
 struct BMaps {
-    CUtensorMap b, code, dg, cx, cy, cz, xc;
+    CUtensorMap b, code, dg, cx, cy, cz, xc, pc;
     // coarse levels: per box the default stencil {d, c_x, c_y, c_z} (as T) when every
     // cell of the box and its 2-cell ring is interior fluid with that diagonal and
     // those couplings (a trimmed box), else d = 0 (k_box_trim); null: no trimming
@@ -683,7 +916,8 @@ struct BMaps {
 // diagonal and one coupling per axis needs none of its diagonal, coupling or code
 // boxes: the box kernel loads b (and the parent x) only and uses the four values.
 // The values are the stored ones, so results are identical with and without
-// trimming.  One block of 256 threads per box; rec[4 box + 0] = d or 0.
+// trimming.  One block of 256 threads per box; rec[4 box + 0] = d or 0.  ring: the ring
+// of the widest box that reads the record (2, with STAR 3).
 template <class E>
 __device__ __forceinline__ bool same_bits(E a, E b) {
     if constexpr (sizeof(E) == 2) return __half_as_ushort(a) == __half_as_ushort(b);
@@ -695,12 +929,13 @@ template <class T, class CS>
 __global__ void __launch_bounds__(256) k_box_trim(Geom g, const uint8_t* __restrict__ code,
                                                   const T* __restrict__ dg, const CS* __restrict__ cx,
                                                   const CS* __restrict__ cy, const CS* __restrict__ cz,
-                                                  T csx, T csy, T csz, T* rec) {
+                                                  T csx, T csy, T csz, T* rec, int ring) {
     pdl_entry();
     const int i0 = 1 + kBT * (int)blockIdx.x, j0 = 1 + kBT * (int)blockIdx.y,
               k0 = 1 + kBT * (int)blockIdx.z;
-    const bool inside = i0 - 2 >= 1 && j0 - 2 >= 1 && k0 - 2 >= 1 && i0 + kBT + 1 <= g.nx &&
-                        j0 + kBT + 1 <= g.ny && k0 + kBT + 1 <= g.nz;
+    const int lo = ring, hi = kBT + ring - 1, nb = kBT + 2 * ring;
+    const bool inside = i0 - lo >= 1 && j0 - lo >= 1 && k0 - lo >= 1 && i0 + hi <= g.nx &&
+                        j0 + hi <= g.ny && k0 + hi <= g.nz;
     bool ok = inside;
     T d0 = T(0);
     CS x0{}, y0{}, z0{};
@@ -711,8 +946,8 @@ __global__ void __launch_bounds__(256) k_box_trim(Geom g, const uint8_t* __restr
         y0 = cy[id0];
         z0 = cz[id0];
         ok = !(d0 < T(1e-30));
-        for (int c = threadIdx.x; ok && c < kBB * kBB * kBB; c += blockDim.x) {
-            const int i = i0 - 2 + c % kBB, j = j0 - 2 + (c / kBB) % kBB, k = k0 - 2 + c / (kBB * kBB);
+        for (int c = threadIdx.x; ok && c < nb * nb * nb; c += blockDim.x) {
+            const int i = i0 - lo + c % nb, j = j0 - lo + (c / nb) % nb, k = k0 - lo + c / (nb * nb);
             const int id = cidx(g, i, j, k);
             ok = (code[id] & kActive) && same_bits(dg[id], d0) && same_bits(cx[id], x0) &&
                  same_bits(cy[id], y0) && same_bits(cz[id], z0);
@@ -728,15 +963,21 @@ __global__ void __launch_bounds__(256) k_box_trim(Geom g, const uint8_t* __restr
     }
 }
 
-template <class T, bool FINE, class CS, bool UP, bool ZDOT>
+template <class T, bool FINE, class CS, bool UP, bool ZDOT, bool STAR = false>
 __global__ void __launch_bounds__(kThreads)
     k_level_box(const __grid_constant__ BMaps M, MLevel<T> L, T* __restrict__ out,
                 const int* __restrict__ done, int* err, double* partials, CGState* cg) {
     pdl_entry();
     if (done && *done) return;
-    using P = BPlan<T, CS, FINE, UP>;
-    constexpr int WT = BBox<T>::W, WS = BBox<CS>::W;
-    constexpr int PT = WT * kBB, PS = WS * kBB;  // plane strides
+    using P = BPlan<T, CS, FINE, UP, STAR>;
+    using BT = typename P::BT;
+    using BC = typename P::BC;
+    using BS = typename P::BS;
+    constexpr int R = P::R, BN = BT::N;          // ring, box edge
+    constexpr int WT = BT::W, WS = BS::W;
+    constexpr int PT = WT * BN, PS = WS * BN;  // plane strides
+    constexpr bool kStarDn = STAR && !UP;
+    static_assert(!STAR || sizeof(T) == 4, "the FP64 form keeps the reference's transfers");
     constexpr bool kFull = sizeof(T) == 8;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* sm = smem_raw;
@@ -769,44 +1010,65 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     const bool tr = !FINE && trim[0] != T(0);
-    // The code box starts at the 16-byte boundary at or below its first column (x0 - 1
+    // The code box starts at the 16-byte boundary at or below its first column (x0 + 1 - R
     // in the padded array): x0 - 16 when bx is even, x0 - 8 when it is odd.  Every other
     // box starts at x0 - A, a 16-byte boundary for its element size.
-    const int aC = kBT * bx - 16 * ((kBT * bx - 1) >> 4);
-    static_assert(16 + kBT + 2 < BBox<uint8_t>::W, "code box: tile and ring at the widest offset");
+    const int aC = kBT * bx - 16 * ((kBT * bx + 1 - R) >> 4);
+    static_assert(16 + kBT + R < BC::W, "code box: tile and ring at the widest offset");
+    // likewise the parents' codes (STAR): from the boundary at or below 4 bx
+    const int aP = (kBT / 2 * bx) & 15;
+    static_assert(12 + 6 <= BSBox<T>::CW, "parent code box at the widest offset");
     bool ok = true;
     if (tid == 0) {
         mbar_init(bar, 1);
-        const int x0 = kBT * bx, y0 = kBT * by - 1, z0 = kBT * bz - 1;
+        const int x0 = kBT * bx, y0 = kBT * by + 1 - R, z0 = kBT * bz + 1 - R;
         fence_proxy_async();
-        constexpr uint32_t kTrimTX = BBox<T>::BYTES + (UP ? BQBox<T>::BYTES : 0u);
+        constexpr uint32_t kTrimTX = BT::BYTES + P::TXP;
         mbar_expect_tx(bar, tr ? kTrimTX : P::TX);
-        tma_load<3>(sm + P::OFF_B, &M.b, x0 - BBox<T>::A, y0, z0, bar);
+        tma_load<3>(sm + P::OFF_B, &M.b, x0 - BT::A, y0, z0, bar);
         if (!tr) {
             tma_load<3>(sm + P::OFF_CODE, &M.code, x0 - aC, y0, z0, bar);
             if constexpr (!FINE) {
-                tma_load<3>(sm + P::OFF_DG, &M.dg, x0 - BBox<T>::A, y0, z0, bar);
-                tma_load<3>(sm + P::OFF_CX, &M.cx, x0 - BBox<CS>::A, y0, z0, bar);
-                tma_load<3>(sm + P::OFF_CY, &M.cy, x0 - BBox<CS>::A, y0, z0, bar);
-                tma_load<3>(sm + P::OFF_CZ, &M.cz, x0 - BBox<CS>::A, y0, z0, bar);
+                tma_load<3>(sm + P::OFF_DG, &M.dg, x0 - BT::A, y0, z0, bar);
+                tma_load<3>(sm + P::OFF_CX, &M.cx, x0 - BS::A, y0, z0, bar);
+                tma_load<3>(sm + P::OFF_CY, &M.cy, x0 - BS::A, y0, z0, bar);
+                tma_load<3>(sm + P::OFF_CZ, &M.cz, x0 - BS::A, y0, z0, bar);
             }
         }
-        if constexpr (UP) tma_load<3>(sm + P::OFF_XC, &M.xc, x0 / 2, (y0 + 1) / 2, (z0 + 1) / 2, bar);
+        if constexpr (UP) {
+            const int xp = kBT / 2 * bx, yp = kBT / 2 * by, zp = kBT / 2 * bz;
+            if constexpr (STAR) {
+                tma_load<3>(sm + P::OFF_XC, &M.xc, xp - 4, yp - 1, zp - 1, bar);
+                tma_load<3>(sm + P::OFF_PC, &M.pc, xp - aP, yp, zp, bar);
+            } else {
+                tma_load<3>(sm + P::OFF_XC, &M.xc, xp, yp, zp, bar);
+            }
+        }
         ok = mbar_wait(bar, 0u, kTmaWaitLimit);
     }
     if (!step_barrier(ok, err)) return;
 
-    // per-cell helpers on box offsets (di, dj, dk) in [-2, 9]
-    auto qT = [](int di, int dj, int dk) { return BBox<T>::pos(di, dj, dk); };
-    auto qC = [aC](int di, int dj, int dk) {
-        return BBox<uint8_t>::pos(di, dj, dk) - BBox<uint8_t>::A + aC;
-    };
-    auto qS = [](int di, int dj, int dk) { return BBox<CS>::pos(di, dj, dk); };
+    // per-cell helpers on box offsets (di, dj, dk) in [-R, 7 + R]
+    auto qT = [](int di, int dj, int dk) { return BT::pos(di, dj, dk); };
+    auto qC = [aC](int di, int dj, int dk) { return BC::pos(di, dj, dk) - BC::A + aC; };
+    auto qS = [](int di, int dj, int dk) { return BS::pos(di, dj, dk); };
     auto nbsum = [&](const T (&cc)[6], int q) -> T {
         return cc[0] * xs[q + 1] + cc[1] * xs[q - 1] + cc[2] * xs[q + WT] + cc[3] * xs[q - WT] +
                cc[4] * xs[q + PT] + cc[5] * xs[q - PT];
     };
     auto prolong = [&](int di, int dj, int dk) -> T {
+        if constexpr (STAR) {
+            using B = BSBox<T>;
+            const int pi = (di + 2) >> 1, pj = (dj + 2) >> 1, pk = (dk + 2) >> 1;
+            const int q = ((pk + 1) * B::N + pj + 1) * B::W + pi + 4;
+            const uint32_t pc = sm[P::OFF_PC + (pk * B::CN + pj) * B::CW + pi + aP];
+            const T xo = xcs[q];
+            T g = (pc & ((di & 1) ? 1u : 2u)) ? xcs[q + ((di & 1) ? 1 : -1)] - xo : T(0);
+            g += (pc & ((dj & 1) ? 4u : 8u)) ? xcs[q + ((dj & 1) ? B::W : -B::W)] - xo : T(0);
+            g += (pc & ((dk & 1) ? 16u : 32u)) ? xcs[q + ((dk & 1) ? B::N * B::W : -B::N * B::W)] - xo
+                                              : T(0);
+            return T(2) * (xo + T(kStarW) * g);
+        }
         return T(2) * xcs[(((dk + 2) >> 1) * 6 + ((dj + 2) >> 1)) * BQBox<T>::W + ((di + 2) >> 1)];
     };
     // colour of a box cell: (i + j + k) & 1 with i0 + j0 + k0 odd
@@ -849,13 +1111,14 @@ __global__ void __launch_bounds__(kThreads)
         // 2 m + s with s fixed by the row's parity.  A thread steps its enumeration
         // index by the block size, updating (m, row) incrementally.
         static_assert(kThreads == 256, "incremental colour enumeration assumes 256 threads");
-        // 1. odd values on the whole box: 144 rows of 12 cells, 6 odd per row; a step
-        // of 256 is 42 rows (3 planes and 6 rows) and 4 cells
+        // 1. odd values on the whole box: BN^2 rows of BN cells, H = BN / 2 odd per row; a
+        // step of 256 is SK planes, SJ rows and SM cells (BN = 12: 3, 6 and 4)
         {
-            int m = tid % 6, jj = (tid / 6) % kBB, kk = tid / (6 * kBB);
-            while (kk < kBB) {
-                const int dj = jj - 2, dk = kk - 2;
-                const int di = -2 + 2 * m + ((1 + dj + dk + par0) & 1);
+            constexpr int H = BN / 2, SM = 256 % H, SJ = 256 / H % BN, SK = 256 / H / BN;
+            int m = tid % H, jj = (tid / H) % BN, kk = tid / (H * BN);
+            while (kk < BN) {
+                const int dj = jj - R, dk = kk - R;
+                const int di = -R + 2 * m + ((1 + dj + dk + par0 + R) & 1);
                 const int q = qT(di, dj, dk);
                 const uint32_t code = code_at(di, dj, dk);
                 T v = T(0);
@@ -865,22 +1128,22 @@ __global__ void __launch_bounds__(kThreads)
                     if constexpr (UP) v = v + prolong(di, dj, dk);
                 }
                 xs[q] = v;
-                m += 4;
-                jj += 6;
-                kk += 3;
-                if (m >= 6) { m -= 6; jj += 1; }
-                if (jj >= kBB) { jj -= kBB; kk += 1; }
+                m += SM;
+                jj += SJ;
+                kk += SK;
+                if (m >= H) { m -= H; jj += 1; }
+                if (jj >= BN) { jj -= BN; kk += 1; }
             }
         }
         __syncthreads();
-        // 2. even values on the tile and the inner ring: 100 rows of 10 cells, 5 even
-        // per row; a step of 256 is 51 rows (5 planes and 1 row) and 1 cell
+        // 2. even values on the tile and all rings but the outermost: EN = BN - 2 (BN = 12:
+        // a step of 256 is 5 planes, 1 row and 1 cell)
         {
-            constexpr int R = kBT + 2;
-            int m = tid % 5, jj = (tid / 5) % R, kk = tid / (5 * R);
-            while (kk < R) {
-                const int dj = jj - 1, dk = kk - 1;
-                const int di = -1 + 2 * m + ((1 + dj + dk + par0) & 1);
+            constexpr int EN = BN - 2, H = EN / 2, SM = 256 % H, SJ = 256 / H % EN, SK = 256 / H / EN;
+            int m = tid % H, jj = (tid / H) % EN, kk = tid / (H * EN);
+            while (kk < EN) {
+                const int dj = jj - (R - 1), dk = kk - (R - 1);
+                const int di = -(R - 1) + 2 * m + ((1 + dj + dk + par0 + R) & 1);
                 const int q = qT(di, dj, dk);
                 const uint32_t code = code_at(di, dj, dk);
                 T v = T(0);
@@ -895,17 +1158,81 @@ __global__ void __launch_bounds__(kThreads)
                     }
                 }
                 xs[q] = v;
-                m += 1;
-                jj += 1;
-                kk += 5;
-                if (m >= 5) { m -= 5; jj += 1; }
-                if (jj >= R) { jj -= R; kk += 1; }
+                m += SM;
+                jj += SJ;
+                kk += SK;
+                if (m >= H) { m -= H; jj += 1; }
+                if (jj >= EN) { jj -= EN; kk += 1; }
             }
         }
         __syncthreads();
         // 3. final results on the tile: thread = the x pair (2 m, 2 m + 1) of row (dj,
         // dk); u = 0 its odd cell, u = 1 its even cell (no lane diverges on colour)
         double acc[3] = {0.0, 0.0, 0.0};
+        if constexpr (kStarDn) {
+            // residuals of the tile and the six faces of its 1-cell ring; even cells were
+            // just relaxed (0, or b where the smoother skips them)
+            constexpr int RN = P::RN;
+            T* rr = reinterpret_cast<T*>(sm + P::OFF_R);
+            auto resid = [&](int di, int dj, int dk, bool odd) {
+                const int q = qT(di, dj, dk);
+                const uint32_t code = code_at(di, dj, dk);
+                T v = T(0);
+                if (code & kActive) {
+                    if (diag(code, q) < T(1e-30)) {
+                        v = bs[q];
+                    } else if (odd) {
+                        T cc[6];
+                        coup(qS(di, dj, dk), cc);
+                        v = nbsum(cc, q);
+                    }
+                }
+                rr[((dk + 1) * RN + dj + 1) * RN + di + 1] = v;
+            };
+            {  // thread = the x pair (2 m, 2 m + 1) of row (dj, dk)
+                const int pm = tid & 3, pj = (tid >> 2) & 7, pk = tid >> 5;
+                const int sO = (1 + pj + pk + par0) & 1;  // the odd cell is di = 2 pm + sO
+                resid(2 * pm + sO, pj, pk, true);
+                resid(2 * pm + 1 - sO, pj, pk, false);
+            }
+            for (int t = tid; t < 6 * 32; t += kThreads) {  // pairs of the faces
+                const int f = t >> 5, m = (t & 31) >> 3, r = t & 7;
+                const int e = (f & 1) ? kBT : -1;
+                int di, dj, dk;
+                if (f < 2) { di = e; dj = 2 * m; dk = r; }
+                else if (f < 4) { dj = e; di = 2 * m; dk = r; }
+                else { dk = e; di = 2 * m; dj = r; }
+                const int o = (1 + di + dj + dk + par0) & 1;  // 1: the pair's second cell is odd
+                // (i + j + k and di + dj + dk + par0 have one parity)
+                const int si = f < 2 ? 0 : 1, sj = f < 2 ? 1 : 0;
+                resid(di + si * o, dj + sj * o, dk, true);
+                resid(di + si * (1 - o), dj + sj * (1 - o), dk, false);
+            }
+            __syncthreads();
+            if (tid < (kBT / 2) * (kBT / 2) * (kBT / 2)) {
+                const int ci = tid % 4, cj = (tid / 4) % 4, ck = tid / 16;
+                const int ic = kBT / 2 * bx + 1 + ci, jc = kBT / 2 * by + 1 + cj,
+                          kc = kBT / 2 * bz + 1 + ck;
+                if (ic <= L.cg.nx && jc <= L.cg.ny && kc <= L.cg.nz) {
+                    const int cid = cidx(L.cg, ic, jc, kc);
+                    const uint32_t cc = L.ccode[cid];
+                    const T* r0 = rr + ((2 * ck + 1) * RN + 2 * cj + 1) * RN + 2 * ci + 1;
+                    auto four = [&](int o, int a, int b2) {  // a face's four cells from offset o
+                        return (r0[o] + r0[o + a]) + (r0[o + b2] + r0[o + a + b2]);
+                    };
+                    constexpr int X = 1, Y = RN, Z = RN * RN;
+                    const T xl = four(0, Y, Z), xr = four(X, Y, Z);
+                    T q = (cc & 2u) ? four(-X, Y, Z) - xl : T(0);
+                    q += (cc & 1u) ? four(2 * X, Y, Z) - xr : T(0);
+                    q += (cc & 8u) ? four(-Y, X, Z) - four(0, X, Z) : T(0);
+                    q += (cc & 4u) ? four(2 * Y, X, Z) - four(Y, X, Z) : T(0);
+                    q += (cc & 32u) ? four(-Z, X, Y) - four(0, X, Y) : T(0);
+                    q += (cc & 16u) ? four(2 * Z, X, Y) - four(Z, X, Y) : T(0);
+                    out[cid] = (xl + xr) + T(kStarW) * q;
+                }
+            }
+            return;
+        }
         T* rs = reinterpret_cast<T*>(sm + P::OFF_B);  // way down: residuals replace b (tile only)
         T res[2];
         int resq[2];

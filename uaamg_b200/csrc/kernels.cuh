@@ -540,6 +540,10 @@ __global__ void k_true_residual(Geom g, const uint8_t* __restrict__ s, const dou
 // is independent of the others.  Writes r as T to rw (0 on solid cells) when
 // given, reduces r.r; mode 1 (residual replacement, gated as replacement_due) also
 // asks the next x update to fold x_lo into x_hi; mode 2: exit diagnostics.
+// Every product and sum rounds by itself, as the reference's build does, in the FP32
+// engines too (whose unit contracts multiply-adds): a residual near 1e-12 of ||b|| is
+// mostly rounding, and this way the reported one is a host's to the last digits.
+__device__ __forceinline__ double rn_sub(double a, double b) { return __dadd_rn(a, -b); }
 template <int DIM, class T>
 __global__ void __launch_bounds__(256) k_resid_x64(Geom g, const uint8_t* __restrict__ code,
                                                    const double* __restrict__ b,
@@ -579,13 +583,14 @@ __global__ void __launch_bounds__(256) k_resid_x64(Geom g, const uint8_t* __rest
             if (DIM == 3) {
                 const double vF = (c & 32u) ? xm : (k > 1 ? xc : wall);
                 const double vK = (c & 16u) ? xp : (k < g.nz ? xc : wall);
-                ax = diag * xc - (vL + vR) * idx2 - (vB + vT) * idy2 - (vF + vK) * idz2;
+                ax = rn_sub(rn_sub(rn_sub(__dmul_rn(diag, xc), __dmul_rn(vL + vR, idx2)),
+                                   __dmul_rn(vB + vT, idy2)), __dmul_rn(vF + vK, idz2));
             } else if (st.vd) {
                 ax = (c & kActive) ? var_op<double>(st, i, j, xc, vL, vR, vB, vT) : 0.0;
             } else {
-                ax = diag * xc - (vL + vR) * idx2 - (vB + vT) * idy2;
+                ax = rn_sub(rn_sub(__dmul_rn(diag, xc), __dmul_rn(vL + vR, idx2)), __dmul_rn(vB + vT, idy2));
             }
-            const double r = (c & kActive) ? bb - ax : 0.0;
+            const double r = (c & kActive) ? rn_sub(bb, ax) : 0.0;
             acc[0] += r * r;
             if (rw) rw[id] = (T)r;
             xm = xc;

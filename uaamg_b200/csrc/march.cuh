@@ -116,6 +116,7 @@ struct MLevel {
     T csx, csy, csz; // coarse levels: coupling = stored value * cs (1 when stored in T)
     int dirichlet;   // finest level: add the Dirichlet wall diagonal
     int zc;          // planes per block (even)
+    const uint8_t* ccode;  // the next-coarser level's codes
 };
 
 // A stored coupling as T: FP16 couplings hold the coupling / cs (a face count).

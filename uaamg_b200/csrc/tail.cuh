@@ -18,7 +18,7 @@
 //   reverse sweep colour 0, 1  uaamg_preconditioner_3d.cpp:123-138
 // so the FP64 engine stays bit-exact with the reference (built with -fmad=false).
 #pragma once
-#include "march.cuh"
+#include "fused.cuh"
 
 namespace uaamg {
 namespace {
@@ -57,6 +57,7 @@ template <class T>
 struct TailArgs {
     int nlev;                         // levels in the tail; the last is the coarsest
     int smem_elems;                   // shared array length (elements of T)
+    int star;                         // STAR transfers (fused.cuh; FP32 and mixed solves)
     TailLevel<T> lv[kTailMaxLevels];  // lv[0]: the first (finest) level of the tail
 };
 
@@ -72,6 +73,7 @@ struct TailView {
     const TailLevel<T>& L;
     T* x;
     T* b;
+    bool star;  // STAR transfers
     __device__ __forceinline__ int gid(int i, int j, int k) const { return cidx(L.g, i, j, k); }
     __device__ __forceinline__ int sid(int i, int j, int k) const { return i + j * L.csx + k * L.csxy; }
 };
@@ -209,6 +211,27 @@ __device__ void tail_res(const TailView<DIM, T>& F, const TailView<DIM, T>& C) {
         T s = T(0);
 #pragma unroll
         for (int q = 0; q < (DIM == 3 ? 8 : 4); ++q) s += r[q];
+        if constexpr (sizeof(T) == 4) {
+            if (C.star) {  // w times the far minus the near side's residuals of each coupled face
+                const uint32_t code = __ldg(C.L.code + C.gid(ic, jc, kc));
+                T t = T(0);
+                for (int f = 0; f < 2 * DIM; ++f) {
+                    if (!(code & (1u << f))) continue;
+                    const int ax = f >> 1, side = f & 1 ? -1 : 1;  // +x, -x, +y, -y, +z, -z
+                    const int d[3] = {ax == 0 ? side : 0, ax == 1 ? side : 0, ax == 2 ? side : 0};
+                    for (int q = 0; q < (DIM == 3 ? 8 : 4); ++q) {
+                        const int e[3] = {DIM == 3 ? q >> 2 : q >> 1, DIM == 3 ? (q >> 1) & 1 : q & 1,
+                                          DIM == 3 ? q & 1 : 0};
+                        if (e[ax] != (side > 0 ? 1 : 0)) continue;  // near side only
+                        const int i = i0 + e[0], j = j0 + e[1], k = k0 + e[2];
+                        t += tail_r(F, F.gid(i + d[0], j + d[1], k + d[2]),
+                                    F.sid(i + d[0], j + d[1], k + d[2])) -
+                             tail_r(F, F.gid(i, j, k), F.sid(i, j, k));
+                    }
+                }
+                s += T(kStarW) * t;
+            }
+        }
         C.b[C.sid(ic, jc, kc)] = (__ldg(C.L.code + C.gid(ic, jc, kc)) & kActive) ? s : T(0);
     }
 }
@@ -217,7 +240,20 @@ __device__ void tail_res(const TailView<DIM, T>& F, const TailView<DIM, T>& C) {
 // cells, so every fine cell may add it.
 template <int DIM, class T>
 __device__ __forceinline__ T tail_prol(const TailView<DIM, T>& C, int i, int j, int k) {
-    return T(2) * C.x[C.sid((i + 1) >> 1, (j + 1) >> 1, DIM == 3 ? (k + 1) >> 1 : 0)];
+    const int ic = (i + 1) >> 1, jc = (j + 1) >> 1, kc = DIM == 3 ? (k + 1) >> 1 : 0;
+    const int s = C.sid(ic, jc, kc);
+    const T xo = C.x[s];
+    if constexpr (sizeof(T) == 4) {
+        if (C.star) {  // and w times the differences to the coupled neighbours on the cell's side
+            const uint32_t c = __ldg(C.L.code + C.gid(ic, jc, kc));
+            const int sx = C.L.csx, sxy = C.L.csxy;
+            T g = (c & ((i & 1) ? 2u : 1u)) ? C.x[s + ((i & 1) ? -1 : 1)] - xo : T(0);
+            g += (c & ((j & 1) ? 8u : 4u)) ? C.x[s + ((j & 1) ? -sx : sx)] - xo : T(0);
+            if (DIM == 3) g += (c & ((k & 1) ? 32u : 16u)) ? C.x[s + ((k & 1) ? -sxy : sxy)] - xo : T(0);
+            return T(2) * (xo + T(kStarW) * g);
+        }
+    }
+    return T(2) * xo;
 }
 
 // Odd cell after the prolongation: its forward value plus 2 x_c (0 unless active
@@ -367,7 +403,9 @@ __global__ void __launch_bounds__(tail_threads<T>()) k_tail(const __grid_constan
         }
     }
     __syncthreads();
-    auto view = [&](int q) { return TailView<DIM, T>{A.lv[q], sm + A.lv[q].xs, sm + A.lv[q].bs}; };
+    auto view = [&](int q) {
+        return TailView<DIM, T>{A.lv[q], sm + A.lv[q].xs, sm + A.lv[q].bs, A.star != 0};
+    };
     for (int q = 0; q < top; ++q) {
         tail_fwd(view(q));
         __syncthreads();

@@ -173,8 +173,12 @@ __global__ void k_export(Geom g, Geom gr, const T* __restrict__ src, double* dst
 // cell, bit 7 its colour ((i+j+k) odd), and on the finest level (fine = 1) bits
 // 0-5 whether its +x,-x,+y,-y,+z,-z neighbour is an interior fluid cell --
 // exactly when the reference's coupling exists (uaamg_preconditioner_3d.cpp:50-66).
-template <int DIM>
-__global__ void k_codes(Geom g, const uint8_t* __restrict__ s, uint8_t* code, int fine) {
+// cx given (coarse levels with STAR transfers, fused.cuh): bits 0-5 whether the cell is
+// coupled to that neighbour.
+template <int DIM, class T>
+__global__ void k_codes(Geom g, const uint8_t* __restrict__ s, uint8_t* code, int fine,
+                        const T* __restrict__ cx, const T* __restrict__ cy,
+                        const T* __restrict__ cz) {
     pdl_entry();
     for_cells<DIM>(g, [&](int i, int j, int k, int id) {
         uint32_t c = ((i + j + k) & 1) ? kOdd : 0u;
@@ -189,6 +193,16 @@ __global__ void k_codes(Geom g, const uint8_t* __restrict__ s, uint8_t* code, in
                     if (k < g.nz && !s[id + g.sxy]) c |= 16u;
                     if (k > 1 && !s[id - g.sxy]) c |= 32u;
                 }
+            }
+        }
+        if (cx && !s[id]) {
+            if (i < g.nx && cx[id] > T(0)) c |= 1u;
+            if (i > 1 && cx[id - 1] > T(0)) c |= 2u;
+            if (j < g.ny && cy[id] > T(0)) c |= 4u;
+            if (j > 1 && cy[id - g.sx] > T(0)) c |= 8u;
+            if (DIM == 3) {
+                if (k < g.nz && cz[id] > T(0)) c |= 16u;
+                if (k > 1 && cz[id - g.sxy] > T(0)) c |= 32u;
             }
         }
         code[id] = (uint8_t)c;
