@@ -47,7 +47,7 @@ struct LevelBuf {
     CS *hcx = nullptr, *hcy = nullptr, *hcz = nullptr;  // couplings as the marches read them
     T *x = nullptr, *b = nullptr;  // level >= 1 only (level 0 uses the CG's r and z)
     uint8_t* code = nullptr;       // cell codes (vec.cuh k_codes)
-    int zc = 2;                    // planes per block of the z marches (march.cuh)
+    int zc = 2, zu = 2;            // planes per block of the z marches, way down and up
     // FP32 couplings on a level of a mixed engine whose face counts exceed 2048 (3D
     // levels 6 and down, 2D levels 12 and down): FP16 holds integers exactly only up
     // to 2048 and overflows above 65504
@@ -439,6 +439,7 @@ private:
     // blocks per SM of the 2D search direction: as many as are resident at once (one
     // wave: a second, partial wave left SMs idle at its end); UAAMG_PMV2D_PER_SM overrides
     int pmv2d_per_sm_ = 8;
+    int pm_zc_ = 2;   // planes per block of the 3D search direction (k_pmatvec)
     int rx_zc_ = 16;  // planes per block of the 3D replacement march (k_resid_march)
     int pmv2d_env_ = 0;
     int resid_per_sm_ = 8;  // the FP64 residual walk: resident blocks per SM (one wave)
@@ -622,12 +623,56 @@ private:
                     (unsigned)((g.nz + kBT - 1) / kBT));
     }
 
-    // Largest even chunk <= 16 planes that still gives every SM several blocks.
-    int pick_zc(const Geom& g) const {
+    // Planes per block of a z march over level g with per_sm resident blocks per SM, whose
+    // blocks walk extra planes beside their chunk: the even length with the least
+    // steps x waves.  A step of an SM's k resident blocks takes k issue-bound units, and
+    // two at least (a lone block waits on its loads and barrier for about that long), so
+    // long chunks save the extra planes, short ones fill a last wave or a small level.
+    // Against chunks halved from 16 until every SM had four blocks: 256^3 mixed, level 1
+    // 49 / 40 -> 31 / 28 us a launch down / up, level 0 85 / 91 -> 79 / 83, the solve 8.1 ->
+    // 7.55 ms; 96^3 FP64, level 0 28 / 35 -> 18 / 23 us, the solve 9.5 -> 7.9 ms.
+    int pick_zc(const Geom& g, int per_sm, int extra) const {
         const long long tiles = (long long)((g.nx + kMX - 1) / kMX) * ((g.ny + kMY - 1) / kMY);
-        int zc = 16;
-        while (zc > 2 && tiles * ((g.nz + zc - 1) / zc) < 4LL * num_sms_) zc /= 2;
-        return zc;
+        int best = 2;
+        double best_cost = 1e300;
+        for (int zc = 2; zc < g.nz + 2 && zc <= 128; zc += 2) {
+            const long long k = (tiles * ((g.nz + zc - 1) / zc) + num_sms_ - 1) / num_sms_;
+            const long long full = k / per_sm, rest = k % per_sm;
+            const double cost = (zc + extra) * ((double)full * std::max(2, per_sm) +
+                                                (rest ? std::max<double>(2.0, (double)rest) : 0.0));
+            if (cost < best_cost) { best_cost = cost; best = zc; }
+        }
+        return best;
+    }
+    template <class K>
+    static int resident(K kern, size_t smem) {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess ||
+            per_sm < 1) {
+            cudaGetLastError();
+            per_sm = 1;
+        }
+        return per_sm;
+    }
+    template <int DIM, bool FINE, class CSL, bool STAR>
+    void pick_chunks_as(LevelBuf<T, CS>& L) const {
+        L.zc = pick_zc(L.g, resident(k_level_fused<DIM, T, FINE, CSL, false, false, STAR>,
+                                     FCfg<DIM, T, CSL, FINE, false, STAR>::BYTES), STAR ? 6 : 4);
+        L.zu = pick_zc(L.g, resident(k_level_fused<DIM, T, FINE, CSL, true, FINE, STAR>,
+                                     FCfg<DIM, T, CSL, FINE, true, STAR>::BYTES), 4);
+    }
+    // Chunk lengths of level l's fused marches (the four-march kernels take the way down's)
+    // and of the search direction.
+    template <int DIM, bool STAR>
+    void pick_chunks() {
+        for (size_t l = 0; l < lv_.size(); ++l) {
+            LevelBuf<T, CS>& L = lv_[l];
+            if (l == 0) pick_chunks_as<DIM, true, CS, STAR>(L);
+            else if (L.c32) pick_chunks_as<DIM, false, T, STAR>(L);
+            else pick_chunks_as<DIM, false, CS, STAR>(L);
+        }
+        pm_zc_ = pick_zc(lv_[0].g, dirichlet_ ? resident(k_pmatvec<DIM, T, true>, PmvCfg<DIM, T>::BYTES)
+                                              : resident(k_pmatvec<DIM, T, false>, PmvCfg<DIM, T>::BYTES), 2);
     }
 
     template <class K>
@@ -749,7 +794,6 @@ private:
         int e;
         for (int l = 0; l < nl; ++l) {
             LevelBuf<T, CS>& L = lv_[l];
-            L.zc = DIM == 3 ? pick_zc(L.g) : 2;
             // largest face count of a level-l coupling: 4^l (3D), 2^l (2D)
             L.c32 = kHalf && l > 0 && (DIM == 3 ? 2 * l : l) > 11;
             L.box = DIM == 3 && cells(L.g) <= box_cells_;
@@ -831,6 +875,14 @@ private:
             rx_zc_ = 2;
             while (rx_zc_ < g.nz && tiles * ((g.nz + rx_zc_ - 1) / rx_zc_) > (long long)per_sm * num_sms_)
                 rx_zc_ *= 2;
+        }
+        if constexpr (DIM == 3) {  // (after the kernels' shared-memory attributes)
+            if constexpr (sizeof(T) == 4) {
+                if (star_) pick_chunks<DIM, true>();
+                else pick_chunks<DIM, false>();
+            } else {
+                pick_chunks<DIM, false>();
+            }
         }
         if (DIM == 3) {
             if ((e = box_attrs<true, CS>()) || (e = box_attrs<false, CS>())) return e;
@@ -1081,7 +1133,7 @@ private:
     }
 
     // Autotuner: for every level with marches, time its V-cycle marches (down and up,
-    // on the level's own buffers) for each z-chunk length in {2, 4, 8, 16, 32} and
+    // on the level's own buffers) for the rule's lengths and for each of 2, 4, ..., 128 and
     // keep the fastest; the choice is cached per GPU, precision, level shape and
     // march kind (tune_lookup / tune_store: for the process, and in the cache file
     // when one is set).  Chunk length changes only the blocks' shape, not a per-cell
@@ -1105,13 +1157,18 @@ private:
                                     (L.c32 ? "|c32" : "");
             {
                 std::vector<int> v;
-                if (tune_lookup(key, &v) && v.size() == 1 && v[0] >= 2 && v[0] <= 32) { L.zc = v[0]; continue; }
+                if (tune_lookup(key, &v) && v.size() == 1 && (v[0] == 0 || (v[0] >= 2 && v[0] <= 128))) {
+                    if (v[0]) L.zc = L.zu = v[0];
+                    continue;
+                }
             }
-            int best = L.zc;
+            const int zc0 = L.zc, zu0 = L.zu;  // the rule's own choice: candidate 0
+            int best = 0;
             float best_ms = 1e30f;
-            for (int zc = 2; zc <= 32 && e == E_OK; zc *= 2) {
+            for (int zc = 0; zc <= 128 && e == E_OK; zc = zc ? 2 * zc : 2) {
                 if (zc > 2 && zc / 2 >= L.g.nz) break;
-                L.zc = zc;
+                L.zc = zc ? zc : zc0;
+                L.zu = zc ? zc : zu0;
                 for (int rep = 0; rep < 3; ++rep) {  // rep 0 warms up
                     if (rep == 1) cudaEventRecord(a, st_);
                     if (l == 0) { down_level<DIM, true>(l, nullptr); up_level<DIM, true>(l, nullptr, false); }
@@ -1126,7 +1183,8 @@ private:
                 }
                 if (ms < best_ms) { best_ms = ms; best = zc; }
             }
-            L.zc = best;
+            L.zc = best ? best : zc0;
+            L.zu = best ? best : zu0;
             tune_store(key, {best});
         }
         prof_on_ = prof;
@@ -1204,7 +1262,7 @@ private:
         }
     }
 
-    MLevel<T> mlevel(int l) const {
+    MLevel<T> mlevel(int l, bool up = false) const {
         const LevelBuf<T, CS>& L = lv_[l];
         MLevel<T> v;
         v.g = L.g;
@@ -1218,7 +1276,7 @@ private:
         v.csy = half ? (T)(1.0 / (lv_[0].hy * lv_[0].hy)) : T(1);
         v.csz = half ? (T)(1.0 / (lv_[0].hz * lv_[0].hz)) : T(1);
         v.dirichlet = dirichlet_;
-        v.zc = L.zc;
+        v.zc = up ? L.zu : L.zc;
         v.ccode = l + 1 < (int)lv_.size() ? lv_[l + 1].code : nullptr;
         return v;
     }
@@ -1325,11 +1383,11 @@ private:
         if (DIM == 3 && L.box)
             UAAMG_LAUNCH_SMEM(tag, (k_level_box<T, FINE, CSL, true, ZDOT, STAR>), box_grid(L.g),
                               dim3(kThreads), (BPlan<T, CSL, FINE, true, STAR>::BYTES), bmaps(l, true),
-                              mlevel(l), x, done, err_, partials_, cg_);
+                              mlevel(l, true), x, done, err_, partials_, cg_);
         else
             UAAMG_LAUNCH_SMEM(tag, (k_level_fused<DIM, T, FINE, CSL, true, ZDOT, STAR>),
-                              march_grid<DIM>(L.g, L.zc), dim3(kThreads),
-                              (FCfg<DIM, T, CSL, FINE, true, STAR>::BYTES), fmaps(l, true), mlevel(l), x,
+                              march_grid<DIM>(L.g, L.zu), dim3(kThreads),
+                              (FCfg<DIM, T, CSL, FINE, true, STAR>::BYTES), fmaps(l, true), mlevel(l, true), x,
                               done, err_, partials_, cg_);
     }
 
@@ -1526,7 +1584,7 @@ private:
             pm.v[0] = lv_[0].mx;
             pm.v[1] = from_p ? map_p_ : map_p2_;
             const KTag tag{K_PMATVEC, 0, cells(g) * (4.0 * sizeof(T) + 1.0)};
-            const int zc = lv_[0].zc;
+            const int zc = pm_zc_;
             if (dirichlet_)
                 UAAMG_LAUNCH_SMEM(tag, (k_pmatvec<DIM, T, true>), march_grid<DIM>(g, zc),
                                   dim3(kThreads), (PmvCfg<DIM, T>::BYTES), pm, g, zc, pnew, ap_, st,
