@@ -630,7 +630,7 @@ private:
     // long chunks save the extra planes, short ones fill a last wave or a small level.
     // Against chunks halved from 16 until every SM had four blocks: 256^3 mixed, level 1
     // 49 / 40 -> 31 / 28 us a launch down / up, level 0 85 / 91 -> 79 / 83, the solve 8.1 ->
-    // 7.55 ms; 96^3 FP64, level 0 28 / 35 -> 18 / 23 us, the solve 9.5 -> 7.9 ms.
+    // 7.55 ms; 96^3 FP64, level 0 way down 28 -> 18 us.
     int pick_zc(const Geom& g, int per_sm, int extra) const {
         const long long tiles = (long long)((g.nx + kMX - 1) / kMX) * ((g.ny + kMY - 1) / kMY);
         int best = 2;
@@ -670,6 +670,17 @@ private:
             if (l == 0) pick_chunks_as<DIM, true, CS, STAR>(L);
             else if (L.c32) pick_chunks_as<DIM, false, T, STAR>(L);
             else pick_chunks_as<DIM, false, CS, STAR>(L);
+        }
+        if constexpr (sizeof(T) == 8) {
+            // The FP64 form's dot products are summed per block of these two kernels; their
+            // partition stays (chunks halved from 16 planes until every SM has four blocks):
+            // 256^3 on another one stops after 81 iterations instead of the reference's 82.
+            const Geom& g = lv_[0].g;
+            const long long tiles = (long long)((g.nx + kMX - 1) / kMX) * ((g.ny + kMY - 1) / kMY);
+            int zc = 16;
+            while (zc > 2 && tiles * ((g.nz + zc - 1) / zc) < 4LL * num_sms_) zc /= 2;
+            lv_[0].zu = pm_zc_ = zc;
+            return;
         }
         pm_zc_ = pick_zc(lv_[0].g, dirichlet_ ? resident(k_pmatvec<DIM, T, true>, PmvCfg<DIM, T>::BYTES)
                                               : resident(k_pmatvec<DIM, T, false>, PmvCfg<DIM, T>::BYTES), 2);
