@@ -151,9 +151,10 @@ public:
         if (cap_) cudaStreamDestroy(cap_);
     }
 
-    // A new problem.  The previous problem's device buffers are kept for reuse by size
-    // (a mask change on the same grid -- moving solids -- allocates nothing) and the
-    // ones the new hierarchy does not take are freed afterwards.
+    // A new problem.  All device buffers of a problem live in one block of memory, kept
+    // while the next problem needs about as much: a mask change on the same grid -- moving
+    // solids -- allocates nothing, and keeps the captured step too, whose kernels see the
+    // same addresses and sizes.
     int set_problem(int dim, int nx, int ny, int nz, double dx, double dy, double dz,
                     const uint8_t* d_solid, int dirichlet) override {
         release(true);
@@ -162,8 +163,12 @@ public:
         dim_ = dim; dirichlet_ = dirichlet;
         dx_ = dx; dy_ = dy; dz_ = dim == 3 ? dz : 1.0;
         int e = dim == 3 ? build<3>(nx, ny, nz, d_solid) : build<2>(nx, ny, nz, d_solid);
-        free_pool();
         if (e != E_OK) { release(); return e; }
+        std::vector<double> sig = graph_signature();
+        if (sig != gsig_) {
+            drop_graph();
+            gsig_ = std::move(sig);
+        }
         return E_OK;
     }
 
@@ -425,8 +430,11 @@ private:
     int* flag_host_ = nullptr;    // pinned, 2 slots
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaStream_t st_ = 0;
-    std::vector<std::pair<void*, size_t>> allocs_;  // device buffers and their bytes
-    std::multimap<size_t, void*> pool_;               // kept for reuse by set_problem
+    unsigned char* arena_ = nullptr;  // one block for all buffers of a problem
+    size_t arena_cap_ = 0, arena_used_ = 0;
+    bool arena_dry_ = false;          // alloc only adds up the sizes
+    std::vector<void*> extra_;        // buffers made after set_problem (vf_)
+    std::vector<double> gsig_;        // what the captured step's arguments depend on
     size_t bytes_ = 0;
     long launches_ = 0;
     int num_sms_ = 148;
@@ -452,7 +460,7 @@ private:
     int tail_nc_ = 0;        // 1: the hierarchy has a tail (0: it does not fit the kernel)
     T* dense_ = nullptr;      // the tail's cycle as a matrix (n rows, stride ld)
     int* dense_cell_ = nullptr;
-    int dense_n_ = 0, dense_ld_ = 0;
+    int dense_n_ = 0, dense_ld_ = 0, dense_cells_ = 0;  // rows in use, stride, rows planned
     size_t tail_smem_ = 0;   // its dynamic shared memory (x and b of every tail level)
     cudaStream_t cap_ = nullptr;      // capture stream
     cudaGraphExec_t gexec_ = nullptr; // two PCG iterations
@@ -522,35 +530,83 @@ private:
         return (double)g.nx * g.ny * (g.nz ? g.nz : 1);
     }
 
+    // The next count elements of the problem's block (zeroed by arena_ready).
     template <class P>
     int alloc(P*& p, size_t count) {
+        const size_t nb = (count * sizeof(P) + 255) / 256 * 256;
+        if (!arena_dry_) {
+            if (arena_used_ + nb > arena_cap_) return E_OOM;
+            p = reinterpret_cast<P*>(arena_ + arena_used_);
+        }
+        arena_used_ += nb;
+        return E_OK;
+    }
+
+    // After a dry pass of the alloc calls: a zeroed block of at least that size, the
+    // present one unless it is too small or more than a quarter too large.
+    int arena_ready() {
+        const size_t need = arena_used_;
+        arena_dry_ = false;
+        arena_used_ = 0;
+        if (!arena_ || arena_cap_ < need || arena_cap_ > need + need / 4) {
+            if (arena_) cudaFree(arena_);
+            arena_ = nullptr;
+            arena_cap_ = 0;
+            void* q = nullptr;
+            if (cudaMalloc(&q, need) != cudaSuccess) {
+                cudaGetLastError();
+                return E_OOM;
+            }
+            arena_ = static_cast<unsigned char*>(q);
+            arena_cap_ = need;
+        }
+        bytes_ = arena_cap_;
+        return cudaMemsetAsync(arena_, 0, need, st_) == cudaSuccess ? E_OK : E_CUDA;
+    }
+
+    // A zeroed buffer of its own, freed with the problem.
+    template <class P>
+    int alloc_extra(P*& p, size_t count) {
         void* q = nullptr;
-        const size_t nb = count * sizeof(P);
-        auto it = pool_.find(nb);
-        if (it != pool_.end()) {
-            q = it->second;
-            pool_.erase(it);
-        } else if (cudaMalloc(&q, nb) != cudaSuccess) {
+        if (cudaMalloc(&q, count * sizeof(P)) != cudaSuccess) {
             cudaGetLastError();
             return E_OOM;
         }
-        allocs_.push_back({q, nb});
-        bytes_ += nb;
+        extra_.push_back(q);
+        bytes_ += count * sizeof(P);
         if (cudaMemsetAsync(q, 0, count * sizeof(P), st_) != cudaSuccess) return E_CUDA;
         p = static_cast<P*>(q);
         return E_OK;
     }
 
-    // keep: the device buffers go to the reuse pool (set_problem) instead of being
-    // freed, and the pinned host words and events stay.
-    void release(bool keep = false) {
-        if (!allocs_.empty() || cg_host_) cudaStreamSynchronize(st_);
-        for (const auto& a : allocs_) {
-            if (keep) pool_.emplace(a.second, a.first);
-            else cudaFree(a.first);
+    // Every value that a captured step's launches take from the problem, beside what
+    // drops the graph by itself (operator, smoothing, V-cycle kernels, history buffer).
+    std::vector<double> graph_signature() const {
+        const Geom& g = lv_[0].g;
+        std::vector<double> v = {(double)dim_, (double)g.nx, (double)g.ny, (double)g.nz, dx_, dy_, dz_,
+                                 (double)dirichlet_, (double)(uintptr_t)arena_, (double)arena_used_,
+                                 (double)pm_zc_, (double)rx_zc_, (double)pmv2d_per_sm_,
+                                 (double)resid_per_sm_, (double)tail_lt_, (double)tail_nc_,
+                                 (double)dense_n_};
+        for (const auto& L : lv_) {
+            v.push_back(L.zc);
+            v.push_back(L.zu);
         }
-        allocs_.clear();
-        if (!keep) free_pool();
+        return v;
+    }
+
+    // keep: the buffers' block, the captured step, the pinned host words and the events
+    // stay (set_problem).
+    void release(bool keep = false) {
+        if (arena_ || cg_host_) cudaStreamSynchronize(st_);
+        for (void* q : extra_) cudaFree(q);
+        extra_.clear();
+        if (!keep && arena_) {
+            cudaFree(arena_);
+            arena_ = nullptr;
+            arena_cap_ = 0;
+        }
+        arena_used_ = 0;
         lv_.clear();
         bytes_ = 0;
         r_ = z_ = p_ = p2_ = ap_ = xlo_ = nullptr;
@@ -562,23 +618,18 @@ private:
         vconv_ = -1;
         err_ = nullptr;
         cg_ = nullptr;
-        if (!keep) {
-            if (cg_host_) { cudaFreeHost(cg_host_); cg_host_ = nullptr; }
-            if (flag_host_) { cudaFreeHost(flag_host_); flag_host_ = nullptr; }
-            for (auto& e : ev_) if (e) { cudaEventDestroy(e); e = nullptr; }
-        }
         for (auto& pr : prof_ev_) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
         prof_ev_.clear();
-        if (gexec_) { cudaGraphExecDestroy(gexec_); gexec_ = nullptr; }
-        gkey_ = -1;
-        ghist_ = nullptr;
         prof_tag_.clear();
         prof_count_ = 0;
-    }
-
-    void free_pool() {
-        for (const auto& kv : pool_) cudaFree(kv.second);
-        pool_.clear();
+        if (keep) return;
+        if (cg_host_) { cudaFreeHost(cg_host_); cg_host_ = nullptr; }
+        if (flag_host_) { cudaFreeHost(flag_host_); flag_host_ = nullptr; }
+        for (auto& e : ev_) if (e) { cudaEventDestroy(e); e = nullptr; }
+        if (gexec_) { cudaGraphExecDestroy(gexec_); gexec_ = nullptr; }
+        gkey_ = -1;
+        gsig_.clear();
+        ghist_ = nullptr;
     }
 
     int sync_check() {
@@ -747,6 +798,66 @@ private:
         return E_OK;
     }
 
+    // The problem's buffers, in order (run twice: sizes, then addresses).
+    template <int DIM>
+    int buffers() {
+        const int nl = (int)lv_.size();
+        int e;
+        for (int l = 0; l < nl; ++l) {
+            LevelBuf<T, CS>& L = lv_[l];
+            const size_t n = (size_t)L.g.n;
+            if ((e = alloc(L.solid, n))) return e;
+            if ((e = alloc(L.code, n))) return e;
+            if ((e = alloc(L.cx, n))) return e;
+            if ((e = alloc(L.cy, n))) return e;
+            if (DIM == 3 && (e = alloc(L.cz, n))) return e;
+            if (dirichlet_ && (e = alloc(L.wd, n))) return e;
+            if (l > 0) {
+                if ((e = alloc(L.x, n))) return e;
+                if ((e = alloc(L.b, n))) return e;
+                if ((e = alloc(L.dg, n))) return e;
+                if (L.box) {
+                    const dim3 bg = box_grid(L.g);
+                    if ((e = alloc(L.trim, (size_t)4 * bg.x * bg.y * bg.z))) return e;
+                }
+                if constexpr (kHalf) {
+                    if (!L.c32) {
+                        if ((e = alloc(L.hcx, n)) || (e = alloc(L.hcy, n))) return e;
+                        if (DIM == 3 && (e = alloc(L.hcz, n))) return e;
+                    }
+                } else {
+                    L.hcx = L.cx; L.hcy = L.cy; L.hcz = L.cz;
+                }
+            }
+        }
+        const Geom g0 = lv_[0].g;
+        const size_t n0 = (size_t)g0.n;
+        if ((e = alloc(r_, n0)) || (e = alloc(z_, n0))) return e;
+        if (!apply_only_ &&
+            ((e = alloc(p_, n0)) || (e = alloc(p2_, n0)) || (e = alloc(ap_, n0)) ||
+             (e = alloc(xlo_, n0)) || (e = alloc(b64_, n0)) || (e = alloc(xd_, n0))))
+            return e;
+        // reductions: the finest-level marches (one partial per block) and the
+        // row-walk kernels (vec_grid)
+        {
+            const dim3 mg = march_grid<DIM>(g0, 2);  // the most blocks any chunk length gives
+            reduce_blocks_ = (long long)mg.x * mg.y * mg.z;
+            const dim3 rg = resid_grid(g0);
+            reduce_blocks_ = std::max(reduce_blocks_, (long long)rg.x * rg.y * rg.z);
+            const dim3 bg = box_grid(g0);  // a small finest level runs as boxes
+            if (lv_[0].box) reduce_blocks_ = std::max(reduce_blocks_, (long long)bg.x * bg.y * bg.z);
+            if (reduce_blocks_ < max_reduce_blocks()) reduce_blocks_ = max_reduce_blocks();
+        }
+        if ((e = alloc(partials_, (size_t)reduce_blocks_ * 4))) return e;
+        if ((e = alloc(err_, 1))) return e;
+        if ((e = alloc(cg_, 1))) return e;
+        if (dense_cells_ > 0) {
+            if ((e = alloc(dense_, (size_t)dense_cells_ * dense_ld_))) return e;
+            if ((e = alloc(dense_cell_, (size_t)dense_cells_))) return e;
+        }
+        return E_OK;
+    }
+
     template <int DIM>
     int build(int nx, int ny, int nz, const uint8_t* d_solid) {
         gref_ = make_geom(DIM, nx, ny, nz);
@@ -808,52 +919,12 @@ private:
             // largest face count of a level-l coupling: 4^l (3D), 2^l (2D)
             L.c32 = kHalf && l > 0 && (DIM == 3 ? 2 * l : l) > 11;
             L.box = DIM == 3 && cells(L.g) <= box_cells_;
-            const size_t n = (size_t)L.g.n;
-            if ((e = alloc(L.solid, n))) return e;
-            if ((e = alloc(L.code, n))) return e;
-            if ((e = alloc(L.cx, n))) return e;
-            if ((e = alloc(L.cy, n))) return e;
-            if (DIM == 3 && (e = alloc(L.cz, n))) return e;
-            if (dirichlet_ && (e = alloc(L.wd, n))) return e;
-            if (l > 0) {
-                if ((e = alloc(L.x, n))) return e;
-                if ((e = alloc(L.b, n))) return e;
-                if ((e = alloc(L.dg, n))) return e;
-                if (L.box) {
-                    const dim3 bg = box_grid(L.g);
-                    if ((e = alloc(L.trim, (size_t)4 * bg.x * bg.y * bg.z))) return e;
-                }
-                if constexpr (kHalf) {
-                    if (!L.c32) {
-                        if ((e = alloc(L.hcx, n)) || (e = alloc(L.hcy, n))) return e;
-                        if (DIM == 3 && (e = alloc(L.hcz, n))) return e;
-                    }
-                } else {
-                    L.hcx = L.cx; L.hcy = L.cy; L.hcz = L.cz;
-                }
-            }
         }
+        if ((e = tail_setup<DIM>()) != E_OK) return e;
+        arena_dry_ = true;
+        arena_used_ = 0;
+        if ((e = buffers<DIM>()) || (e = arena_ready()) || (e = buffers<DIM>())) return e;
         const Geom g0 = lv_[0].g;
-        const size_t n0 = (size_t)g0.n;
-        if ((e = alloc(r_, n0)) || (e = alloc(z_, n0))) return e;
-        if (!apply_only_ &&
-            ((e = alloc(p_, n0)) || (e = alloc(p2_, n0)) || (e = alloc(ap_, n0)) ||
-             (e = alloc(xlo_, n0)) || (e = alloc(b64_, n0)) || (e = alloc(xd_, n0))))
-            return e;
-        // reductions: the finest-level marches (one partial per block) and the
-        // row-walk kernels (vec_grid)
-        {
-            const dim3 mg = march_grid<DIM>(g0, 2);  // the most blocks any chunk length gives
-            reduce_blocks_ = (long long)mg.x * mg.y * mg.z;
-            const dim3 rg = resid_grid(g0);
-            reduce_blocks_ = std::max(reduce_blocks_, (long long)rg.x * rg.y * rg.z);
-            const dim3 bg = box_grid(g0);  // a small finest level runs as boxes
-            if (lv_[0].box) reduce_blocks_ = std::max(reduce_blocks_, (long long)bg.x * bg.y * bg.z);
-            if (reduce_blocks_ < max_reduce_blocks()) reduce_blocks_ = max_reduce_blocks();
-        }
-        if ((e = alloc(partials_, (size_t)reduce_blocks_ * 4))) return e;
-        if ((e = alloc(err_, 1))) return e;
-        if ((e = alloc(cg_, 1))) return e;
         if (!cg_host_ && cudaMallocHost(&cg_host_, sizeof(CGState)) != cudaSuccess) return E_OOM;
         if (!flag_host_ && cudaMallocHost(&flag_host_, 2 * sizeof(int)) != cudaSuccess) return E_OOM;
         for (auto& ev : ev_)
@@ -1024,9 +1095,8 @@ private:
                                  Cl.trim, star_ ? 3 : 2);
             }
         }
-        if ((e = sync_check()) != E_OK) return e;
-        if ((e = tail_setup<DIM>()) != E_OK) return e;
         if ((e = dense_setup<DIM>()) != E_OK) return e;
+        if ((e = sync_check()) != E_OK) return e;
         if (DIM == 3 && autotune_) return tune<DIM>();
         return E_OK;
     }
@@ -1045,6 +1115,7 @@ private:
         const int nl = (int)lv_.size();
         tail_nc_ = 0;
         tail_lt_ = nl;
+        dense_cells_ = 0;
         if (nl < 2) return E_OK;
         const Geom& gc = lv_[nl - 1].g;
         size_t elems = 2 * tail_cells_padded(gc);
@@ -1062,6 +1133,10 @@ private:
         tail_lt_ = lt;
         tail_nc_ = 1;
         tail_smem_ = elems * sizeof(T);
+        if (sizeof(T) == 4 && cover_ && cells(lv_[lt].g) <= (double)kDenseCells) {
+            dense_cells_ = (int)cells(lv_[lt].g);
+            dense_ld_ = (dense_cells_ + 3) / 4 * 4;
+        }
         return E_OK;
     }
 
@@ -1101,16 +1176,12 @@ private:
     int dense_setup() {
         dense_n_ = 0;
         if constexpr (sizeof(T) == 4) {
-            if (!cover_ || tail_nc_ == 0 || cells(lv_[tail_lt_].g) > (double)kDenseCells) return E_OK;
+            if (dense_cells_ == 0) return E_OK;
             const Geom& g = lv_[tail_lt_].g;
-            const int n = (int)cells(g);
-            dense_ld_ = (n + 3) / 4 * 4;
-            int e;
-            if ((e = alloc(dense_, (size_t)n * dense_ld_)) || (e = alloc(dense_cell_, (size_t)n))) return e;
+            const int n = dense_cells_;
             UAAMG_LAUNCH((KTag{K_SETUP, tail_lt_, 0.0}), k_tail_cells<DIM>, 1, 256, g, dense_cell_);
             UAAMG_LAUNCH_SMEM((KTag{K_SETUP, tail_lt_, 0.0}), (k_tail<DIM, T>), n, tail_threads<T>(),
                               tail_smem_, tail_args<DIM>(), (const int*)nullptr, dense_, dense_ld_);
-            if ((e = sync_check()) != E_OK) return e;
             dense_n_ = n;
         }
         return E_OK;
@@ -1649,7 +1720,7 @@ private:
             // FP32 copies of the variable-coefficient operator (once per contents)
             if (!vf_[0]) {
                 for (int q = 0; q < 3; ++q)
-                    if (int e = alloc(vf_[q], (size_t)n)) return e;
+                    if (int e = alloc_extra(vf_[q], (size_t)n)) return e;
                 if (gexec_) {  // a captured step holds the copies' (null) pointers
                     cudaStreamSynchronize(st_);
                     cudaGraphExecDestroy(gexec_);
