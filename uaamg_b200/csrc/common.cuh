@@ -107,6 +107,33 @@ __device__ __forceinline__ void pdl_entry() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// The kernels of an iteration do what does not depend on their predecessor ahead of
+// this wait: index arithmetic, tables, barriers, loads of the hierarchy's constant
+// arrays, and of arrays last written two or more kernels earlier (a kernel is launched
+// only after its predecessor's own wait, so everything before the predecessor is
+// complete and visible).  Every path of every kernel executes the wait, also one that
+// has nothing to do: its successor relies on it for the kernels further back.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// A load that stays where it is written (the compiler may otherwise move it behind the
+// test of another one, and pay their latencies in turn).
+__device__ __forceinline__ int ld_now(const int* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_now(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_now(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // Host-visible launch helpers ------------------------------------------------
 

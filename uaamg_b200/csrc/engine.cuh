@@ -475,6 +475,13 @@ private:
 
     int max_reduce_blocks() const { return 4 * num_sms_; }
 
+    // Blocks of the CG update: one vector a thread on small grids (idle blocks only
+    // lengthen the reduction's end); FP64 keeps its partition of r.r.
+    unsigned update_blocks(long long nvec) const {
+        if (sizeof(T) == 8) return (unsigned)max_reduce_blocks();
+        return (unsigned)std::max<long long>(1, std::min<long long>(max_reduce_blocks(), (nvec + 255) / 256));
+    }
+
     void drop_graph() {
         if (gexec_) {
             cudaStreamSynchronize(st_);
@@ -1679,12 +1686,12 @@ private:
         const long long nvec = (long long)g.n / Vec16<T>::N;
         // x_lo, r, p, Ap in; x_lo, r out (a fold after a replacement adds x_hi in and out)
         UAAMG_LAUNCH((KTag{K_UPDATE, 0, cells(g) * (6.0 * sizeof(T))}), k_update_flat<T>,
-                     max_reduce_blocks(), 256, nvec, xlo_, r_, pnew, ap_, mixed_ ? xd_ : nullptr,
+                     update_blocks(nvec), 256, nvec, xlo_, r_, pnew, ap_, mixed_ ? xd_ : nullptr,
                      partials_, cg_, cur_.hist);
         if (mixed_) {
             // residual replacement (when due, one iteration in replace_every; the others
             // return at once): b, x_hi, x_lo, codes in; r out
-            nopdl_next_ = true;
+            nopdl_next_ = cells(g) > 1048576.0;
             const KTag tag{K_REPLACE, 0, cells(g) * (17.0 + 2.0 * sizeof(T))};
             if (DIM == 3) {
                 MarchMaps rm;

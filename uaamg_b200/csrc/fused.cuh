@@ -220,13 +220,13 @@ __device__ __forceinline__ int star_ring_pair(int t, int& d1i, int& d1j, int& d2
     return 0;
 }
 
+// Part 1 of a plane's loads: the hierarchy's constant arrays (they do not depend on the
+// kernel before); part 2: b and the parent's x.  Part 1 announces the bytes of both.
 template <int DIM, class T, class CS, bool FINE, bool UP, bool STAR>
-__device__ __forceinline__ void f_issue(const FMaps& M, unsigned char* st, uint64_t* bar, int k) {
+__device__ __forceinline__ void f_issue1(const FMaps& M, unsigned char* st, uint64_t* bar, int k) {
     using P = FPlan<DIM, T, CS, FINE, UP, STAR>;
     const int x0 = kMX * (int)blockIdx.x, y0 = kMY * (int)blockIdx.y + 1 - P::R;
-    fence_proxy_async();
     mbar_expect_tx(bar, P::TX);
-    tma_load<DIM>(st + P::OFF_B, &M.b, x0 - P::BT::A, y0, k, bar);
     tma_load<DIM>(st + P::OFF_CODE, &M.code, x0 - P::BC::A, y0, k, bar);
     if constexpr (!FINE) {
         tma_load<DIM>(st + P::OFF_DG, &M.dg, x0 - P::BT::A, y0, k, bar);
@@ -234,14 +234,20 @@ __device__ __forceinline__ void f_issue(const FMaps& M, unsigned char* st, uint6
         tma_load<DIM>(st + P::OFF_CY, &M.cy, x0 - P::BS::A, y0, k, bar);
         if constexpr (DIM == 3) tma_load<DIM>(st + P::OFF_CZ, &M.cz, x0 - P::BS::A, y0, k, bar);
     }
+    if constexpr (UP && STAR)
+        tma_load<DIM>(st + P::OFF_PC, &M.pc, x0 / 2, kMY / 2 * (int)blockIdx.y, (k + 1) >> 1, bar);
+}
+template <int DIM, class T, class CS, bool FINE, bool UP, bool STAR>
+__device__ __forceinline__ void f_issue2(const FMaps& M, unsigned char* st, uint64_t* bar, int k) {
+    using P = FPlan<DIM, T, CS, FINE, UP, STAR>;
+    const int x0 = kMX * (int)blockIdx.x, y0 = kMY * (int)blockIdx.y + 1 - P::R;
+    tma_load<DIM>(st + P::OFF_B, &M.b, x0 - P::BT::A, y0, k, bar);
     if constexpr (UP) {
         const int yc = kMY / 2 * (int)blockIdx.y, kc = (k + 1) >> 1;
-        if constexpr (STAR) {
+        if constexpr (STAR)
             tma_load<DIM>(st + P::OFF_XC, &M.xc, x0 / 2 - SBox<T, DIM>::A, yc - 1, kc - (k & 1), bar);
-            tma_load<DIM>(st + P::OFF_PC, &M.pc, x0 / 2, yc, kc, bar);
-        } else {
+        else
             tma_load<DIM>(st + P::OFF_XC, &M.xc, x0 / 2, yc, kc, bar);
-        }
     }
 }
 
@@ -261,15 +267,31 @@ struct FRing {
         const int u = p - p0;
         return mbar_wait(&bars[u % S], (uint32_t)((u / S) & 1), kTmaWaitLimit);
     }
-    __device__ void start(const FMaps& M) const {
+    // the first S planes: barriers and part 1, then part 2
+    __device__ void start1(const FMaps& M) const {
         for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
+        fence_proxy_async();
         for (int p = p0; p < p0 + S && p <= plast; ++p)
-            f_issue<DIM, T, CS, FINE, UP, STAR>(M, at(p), &bars[(p - p0) % S], p);
+            f_issue1<DIM, T, CS, FINE, UP, STAR>(M, at(p), &bars[(p - p0) % S], p);
+    }
+    __device__ void start2(const FMaps& M) const {
+        for (int p = p0; p < p0 + S && p <= plast; ++p)
+            f_issue2<DIM, T, CS, FINE, UP, STAR>(M, at(p), &bars[(p - p0) % S], p);
+    }
+    // a block that stops at once waits for the loads it started
+    __device__ bool drain() const {
+        bool ok = true;
+        for (int p = p0; p < p0 + S && p <= plast; ++p) ok = wait(p) && ok;
+        return ok;
     }
     // after a block barrier: plane `freed` is no longer read; load plane freed + S
     __device__ void refill(const FMaps& M, int freed) const {
-        if (freed >= p0 && freed + S <= plast)
-            f_issue<DIM, T, CS, FINE, UP, STAR>(M, at(freed + S), &bars[(freed - p0) % S], freed + S);
+        if (freed >= p0 && freed + S <= plast) {
+            fence_proxy_async();
+            uint64_t* bar = &bars[(freed - p0) % S];
+            f_issue1<DIM, T, CS, FINE, UP, STAR>(M, at(freed + S), bar, freed + S);
+            f_issue2<DIM, T, CS, FINE, UP, STAR>(M, at(freed + S), bar, freed + S);
+        }
     }
 };
 
@@ -286,6 +308,7 @@ struct FHist {
     unsigned char* sm = smem_raw;                                                \
     if (smem_u32(sm) & 127u) {                                                   \
         if (threadIdx.x == 0) atomicExch(err, 2);                                \
+        pdl_wait();                                                              \
         return;                                                                  \
     }
 
@@ -293,8 +316,6 @@ template <int DIM, class T, bool FINE, class CS, bool UP, bool ZDOT, bool STAR =
 __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::MINB))
     k_level_fused(const __grid_constant__ FMaps M, MLevel<T> L, T* __restrict__ out,
                   const int* __restrict__ done, int* err, double* partials, CGState* cg) {
-    pdl_entry();
-    if (done && *done) return;
     using C = FCfg<DIM, T, CS, FINE, UP, STAR>;
     using P = typename C::P;
     constexpr int S = C::S, WT = P::BT::W, WS = P::BS::W;
@@ -306,6 +327,21 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
     const Geom& g = L.g;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int i0 = 1 + kMX * (int)blockIdx.x, j0 = 1 + kMY * (int)blockIdx.y;
+    int kb, ke;
+    if constexpr (UP) zrange<DIM>(g, L.zc, kb, ke);
+    else zrange_restrict<DIM>(g, L.cg, L.zc, kb, ke);
+    // 3D: steps s = s0 .. sl: odd values of planes kb-2 .. ke+1, even values of kb-1 ..
+    // ke, final results of kb .. ke-1 (a STAR way down: final results of kb-1 .. ke, so one
+    // step more at either end); 2D: the one plane 0
+    constexpr int X = kStarDn ? 1 : 0;
+    const int s0 = kb - 3 - X, sl = ke + X;
+    const FRing<DIM, T, CS, FINE, UP, STAR, S> R{reinterpret_cast<uint64_t*>(sm), sm + C::OFF_RING,
+                                                 DIM == 3 ? s0 + 1 : 0, DIM == 3 ? sl + 1 : 0};
+    if (tid == 0) {
+        tma_prefetch(&M.b);
+        if constexpr (UP) tma_prefetch(&M.xc);
+        R.start1(M);
+    }
     if (FINE) build_lut<DIM, T>(lut, L.idx2, L.idy2, L.idz2);
     // Finest level in FP32 (no Dirichlet walls: those problems take the four-march
     // level): every cell update is a multiply-add driven by the table entry of its
@@ -454,9 +490,6 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
         cR1 = fcell<P, T, DIM, STAR>(g, i0, j0, d1i, d1j);
         cR2 = fcell<P, T, DIM, STAR>(g, i0, j0, d2i, d2j);
     }
-    int kb, ke;
-    if constexpr (UP) zrange<DIM>(g, L.zc, kb, ke);
-    else zrange_restrict<DIM>(g, L.cg, L.zc, kb, ke);
     T* xpl = reinterpret_cast<T*>(sm + C::OFF_X);
     double acc[3] = {0.0, 0.0, 0.0};
     const int ic = kMX / 2 * (int)blockIdx.x + 1 + (lane >> 1);
@@ -616,17 +649,22 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
         out[cidx(L.cg, ic, jc, kc)] = ((a0 + a1) + (b0 + b1)) + T(kStarW) * (q + zt);
     };
     T rlo[2] = {T(0), T(0)};
+    // from here on the previous kernel's results: b, the parent's x, the stop flag (read
+    // beside the loads, whose blocks then only wait for what they started)
+    pdl_wait();
+    bool ok = true;
+    const int stop = done ? ld_now(done) : 0;
+    if (tid == 0) R.start2(M);
+    pdl_launch();
+    if (stop) {
+        if (tid == 0 && !R.drain()) atomicExch(err, 1);
+        return;
+    }
+    if (tid == 0) ok = R.wait(R.p0);
+    if (!step_barrier(ok, err)) return;
     if constexpr (DIM == 2) {
         // one plane: odd values, barrier, even values, barrier, final
         unsigned char* st = sm + C::OFF_RING;
-        uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
-        bool ok = true;
-        if (tid == 0) {
-            mbar_init(bar, 1);
-            f_issue<DIM, T, CS, FINE, UP, STAR>(M, st, bar, 0);
-            ok = mbar_wait(bar, 0u, kTmaWaitLimit);
-        }
-        if (!step_barrier(ok, err)) return;
         // A is odd when i + j is odd; ring pairs likewise
         const bool oddA = cA.par != 0;
         const FCell tO = oddA ? cA : cB, tE = oddA ? cB : cA;
@@ -665,19 +703,6 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
             final_pair(even, st, st, xpl, 0, tO, tE, oddA, ot, et, T(0), T(0), T(0), T(0), rlo);
         }
     } else {
-        // steps s = kb-3 .. ke: odd values of planes kb-2 .. ke+1, even values of
-        // kb-1 .. ke, final results of kb .. ke-1
-        // (a STAR way down: final results of kb-1 .. ke, so one step more at either end)
-        constexpr int X = kStarDn ? 1 : 0;
-        const int s0 = kb - 3 - X, sl = ke + X;
-        FRing<DIM, T, CS, FINE, UP, STAR, S> R{reinterpret_cast<uint64_t*>(sm), sm + C::OFF_RING,
-                                               s0 + 1, sl + 1};
-        bool ok = true;
-        if (tid == 0) {
-            R.start(M);
-            ok = R.wait(R.p0);
-        }
-        if (!step_barrier(ok, err)) return;
         // role 0 is the cell that is even on planes s0, s0+2, ... (odd on s0+1, ...)
         const bool aRole0 = ((cA.par + s0) & 1) == 0;
         const FCell t0 = aRole0 ? cA : cB, t1 = aRole0 ? cB : cA;
@@ -967,8 +992,6 @@ template <class T, bool FINE, class CS, bool UP, bool ZDOT, bool STAR = false>
 __global__ void __launch_bounds__(kThreads)
     k_level_box(const __grid_constant__ BMaps M, MLevel<T> L, T* __restrict__ out,
                 const int* __restrict__ done, int* err, double* partials, CGState* cg) {
-    pdl_entry();
-    if (done && *done) return;
     using P = BPlan<T, CS, FINE, UP, STAR>;
     using BT = typename P::BT;
     using BC = typename P::BC;
@@ -983,6 +1006,7 @@ __global__ void __launch_bounds__(kThreads)
     unsigned char* sm = smem_raw;
     if (smem_u32(sm) & 127u) {
         if (threadIdx.x == 0) atomicExch(err, 2);
+        pdl_wait();
         return;
     }
     const Geom& g = L.g;
@@ -1025,7 +1049,9 @@ __global__ void __launch_bounds__(kThreads)
         fence_proxy_async();
         constexpr uint32_t kTrimTX = BT::BYTES + P::TXP;
         mbar_expect_tx(bar, tr ? kTrimTX : P::TX);
-        tma_load<3>(sm + P::OFF_B, &M.b, x0 - BT::A, y0, z0, bar);
+        // the hierarchy's constant arrays, ahead of the wait for the previous kernel
+        tma_prefetch(&M.b);
+        if constexpr (UP) tma_prefetch(&M.xc);
         if (!tr) {
             tma_load<3>(sm + P::OFF_CODE, &M.code, x0 - aC, y0, z0, bar);
             if constexpr (!FINE) {
@@ -1035,18 +1061,20 @@ __global__ void __launch_bounds__(kThreads)
                 tma_load<3>(sm + P::OFF_CZ, &M.cz, x0 - BS::A, y0, z0, bar);
             }
         }
-        if constexpr (UP) {
-            const int xp = kBT / 2 * bx, yp = kBT / 2 * by, zp = kBT / 2 * bz;
-            if constexpr (STAR) {
-                tma_load<3>(sm + P::OFF_XC, &M.xc, xp - 4, yp - 1, zp - 1, bar);
-                tma_load<3>(sm + P::OFF_PC, &M.pc, xp - aP, yp, zp, bar);
-            } else {
-                tma_load<3>(sm + P::OFF_XC, &M.xc, xp, yp, zp, bar);
-            }
-        }
-        ok = mbar_wait(bar, 0u, kTmaWaitLimit);
+        const int xp = kBT / 2 * bx, yp = kBT / 2 * by, zp = kBT / 2 * bz;
+        if constexpr (UP && STAR) tma_load<3>(sm + P::OFF_PC, &M.pc, xp - aP, yp, zp, bar);
+        pdl_wait();
+        tma_load<3>(sm + P::OFF_B, &M.b, x0 - BT::A, y0, z0, bar);
+        if constexpr (UP && STAR) tma_load<3>(sm + P::OFF_XC, &M.xc, xp - 4, yp - 1, zp - 1, bar);
+        else if constexpr (UP) tma_load<3>(sm + P::OFF_XC, &M.xc, xp, yp, zp, bar);
+    } else {
+        pdl_wait();
     }
+    const int stop = done ? ld_now(done) : 0;
+    pdl_launch();
+    if (tid == 0) ok = mbar_wait(bar, 0u, kTmaWaitLimit);
     if (!step_barrier(ok, err)) return;
+    if (stop) return;
 
     // per-cell helpers on box offsets (di, dj, dk) in [-R, 7 + R]
     auto qT = [](int di, int dj, int dk) { return BT::pos(di, dj, dk); };

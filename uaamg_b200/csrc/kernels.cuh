@@ -630,35 +630,61 @@ __global__ void __launch_bounds__(256) k_pmatvec_2d(Geom g, const uint8_t* __res
                                                      const T* __restrict__ pold,
                                                      T* __restrict__ pnew, T* __restrict__ ap,
                                                      Stencil st, double* partials, CGState* cg) {
-    pdl_entry();
-    if (cg->done) return;
-    const T m = (T)cg->mean_z, beta = (T)cg->beta;
     const T idx2 = (T)st.idx2, idy2 = (T)st.idy2, diag = (T)st.diag;
     double acc[1] = {0.0};
     const int sx = g.sx;
     const int nxc = (g.nx + 31) >> 5;
     const int nitems = ((g.ny + 1) >> 1) * nxc;  // < 2^26
     const double rx = 1.0 / nxc;
-    for (int it = (int)(blockIdx.x * blockDim.y + threadIdx.y); it < nitems;
-         it += (int)(gridDim.x * blockDim.y)) {
+    const int it0 = (int)(blockIdx.x * blockDim.y + threadIdx.y);
+    T zz[8], qq[8];
+    uint32_t cc[2];
+    // the pair of item it: column, first row, index, offset of its second cell (0: none)
+    // and of its eight cells: 0: below A, 1: A, 2: B (above A), 3: above B (a ghost at
+    // most), 4/5: A -x/+x, 6/7: B -x/+x
+    auto place = [&](int it, int& i, int& j, int& id, int& sb, int (&off)[8]) -> bool {
         int ch;
         const int pr = divmod_rcp(it, nxc, rx, ch);
-        const int i = 1 + (ch << 5) + (int)threadIdx.x;
-        if (i > g.nx) continue;
-        const int j = 1 + 2 * pr;
+        i = 1 + (ch << 5) + (int)threadIdx.x;
+        j = 1 + 2 * pr;
         const bool hb = j < g.ny;  // (i, j+1) is an interior cell
-        const int id = cidx(g, i, j, 0);
-        const int sb = hb ? sx : 0;            // second cell, or the first again
-        const int s2 = hb ? 2 * sx : sx;       // the row above the pair (a ghost at most)
-        // 0: below A, 1: A, 2: B (above A), 3: above B, 4/5: A -x/+x, 6/7: B -x/+x
-        const int off[8] = {-sx, 0, sb, s2, -1, 1, sb - 1, sb + 1};
-        T zz[8], qq[8];
+        id = cidx(g, i, j, 0);
+        sb = hb ? sx : 0;  // second cell, or the first again
+        const int o[8] = {-sx, 0, sb, hb ? 2 * sx : sx, -1, 1, sb - 1, sb + 1};
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            zz[e] = z[id + off[e]];
-            qq[e] = pold[id + off[e]];
+        for (int e = 0; e < 8; ++e) off[e] = o[e];
+        return i <= g.nx;
+    };
+    auto load_old = [&](int id, int sb, const int (&off)[8]) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) qq[e] = ld_now(&pold[id + off[e]]);
+        cc[0] = __ldg(&code[id]);
+        cc[1] = __ldg(&code[id + sb]);
+    };
+    auto load_z = [&](int id, const int (&off)[8]) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) zz[e] = ld_now(&z[id + off[e]]);
+    };
+    // the first item: p_old (written an iteration ago) and the codes ahead of the wait,
+    // z beside the stop flag and the scalars
+    int i, j, id, sb, off[8];
+    const bool some = it0 < nitems && place(it0, i, j, id, sb, off);
+    if (some) load_old(id, sb, off);
+    pdl_wait();
+    const int stop = ld_now(&cg->done);
+    const T m = (T)cg->mean_z, beta = (T)cg->beta;
+    if (some) load_z(id, off);
+    pdl_launch();
+    if (stop) return;
+    for (int it = it0; it < nitems; it += (int)(gridDim.x * blockDim.y)) {
+        if (it != it0) {
+            if (!place(it, i, j, id, sb, off)) continue;
+            load_old(id, sb, off);
+            load_z(id, off);
+        } else if (!some) {
+            continue;
         }
-        const uint32_t cc[2] = {code[id], code[id + sb]};
+        const bool hb = sb != 0;
         const bool var = st.vd != nullptr;  // the same for the whole launch
         T k0[2] = {T(0), T(0)}, kx[2] = {T(0), T(0)}, ky[2] = {T(0), T(0)};
         if (!var) {

@@ -139,6 +139,7 @@ __device__ __forceinline__ T coupling(CS v, T cs) {
     unsigned char* sm = smem_raw;                                                \
     if (smem_u32(sm) & 127u) {                                                   \
         if (threadIdx.x == 0) atomicExch(err, 2);                                \
+        pdl_wait();                                                              \
         return;                                                                  \
     }
 
@@ -296,6 +297,31 @@ struct MRing {
     __device__ void start(const MarchMaps& M) const {
         for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
         for (int p = p0; p < p0 + S && p <= plast; ++p) issue_plane<DIM, P>(M, at(p), &bars[(p - p0) % S], p);
+    }
+    // start in two parts: every load but slot 0's; slot 0's
+    __device__ void start1(const MarchMaps& M) const {
+        for (int s = 0; s < S; ++s) mbar_init(&bars[s], 1);
+        fence_proxy_async();
+        const int x0 = kMX * (int)blockIdx.x, y0 = kMY * (int)blockIdx.y;
+        static_assert(!P::XCB, "no parent box");
+        for (int p = p0; p < p0 + S && p <= plast; ++p) {
+            uint64_t* bar = &bars[(p - p0) % S];
+            mbar_expect_tx(bar, P::TX_BYTES);
+#pragma unroll
+            for (int q = 1; q < P::NV; ++q) tma_load<DIM>(at(p) + P::box_off(q), &M.v[q], x0, y0, p, bar);
+            tma_load<DIM>(at(p) + P::OFF_CODE, &M.code, x0, y0, p, bar);
+        }
+    }
+    __device__ void start2(const MarchMaps& M) const {
+        const int x0 = kMX * (int)blockIdx.x, y0 = kMY * (int)blockIdx.y;
+        for (int p = p0; p < p0 + S && p <= plast; ++p)
+            tma_load<DIM>(at(p) + P::box_off(0), &M.v[0], x0, y0, p, &bars[(p - p0) % S]);
+    }
+    // a block that stops at once waits for the loads it started
+    __device__ bool drain() const {
+        bool ok = true;
+        for (int p = p0; p < p0 + S && p <= plast; ++p) ok = wait(p) && ok;
+        return ok;
     }
     // thread 0, after a block barrier: refill the stage of plane `freed`
     __device__ void refill(const MarchMaps& M, int freed) const {
@@ -880,8 +906,6 @@ template <int DIM, class T, bool DIRW = true>
 __global__ void __launch_bounds__(kThreads, DIRW ? 1 : PmvCfg<DIM, T>::MINB)
     k_pmatvec(const __grid_constant__ MarchMaps M, Geom g, int zc, T* __restrict__ pnew,
               T* __restrict__ ap, Stencil st, double* partials, CGState* cg, int* err) {
-    pdl_entry();
-    if (cg->done) return;
     using C = PmvCfg<DIM, T>;
     using P = typename C::P;
     using Lay = typename C::Lay;
@@ -891,18 +915,28 @@ __global__ void __launch_bounds__(kThreads, DIRW ? 1 : PmvCfg<DIM, T>::MINB)
     T* pbuf1 = reinterpret_cast<T*>(sm + Lay::OFF_EXTRA + align128(PBox<T>::BYTES));
     const int tid = threadIdx.x;
     const Pair o = own_pair<T>(g);
-    const T m = (T)cg->mean_z, beta = (T)cg->beta;
     const T idx2 = (T)st.idx2, idy2 = (T)st.idy2, idz2 = (T)st.idz2, diag = (T)st.diag;
     double acc[1] = {0.0};
     int kb, ke;
     zrange<DIM>(g, zc, kb, ke);
     MRing<DIM, S, P> R{reinterpret_cast<uint64_t*>(sm), sm + Lay::OFF_RING,
                        DIM == 3 ? kb - 1 : 0, DIM == 3 ? ke : 0};
+    // codes and p_old (written an iteration ago) ahead of the wait, then z and the scalars
     bool ok = true;
     if (tid == 0) {
-        R.start(M);
-        ok = R.wait(R.p0) && (DIM == 2 || (R.wait(kb) && R.wait(kb + 1)));
+        tma_prefetch(&M.v[0]);
+        R.start1(M);
     }
+    pdl_wait();
+    const int stop = ld_now(&cg->done);
+    const T m = (T)cg->mean_z, beta = (T)cg->beta;
+    if (tid == 0) R.start2(M);
+    pdl_launch();
+    if (stop) {
+        if (tid == 0 && !R.drain()) atomicExch(err, 1);
+        return;
+    }
+    if (tid == 0) ok = R.wait(R.p0) && (DIM == 2 || (R.wait(kb) && R.wait(kb + 1)));
     if (!step_barrier(ok, err)) return;
     int rq = -1, ra, rr;
     if (ring_cell(tid, ra, rr)) rq = rr * W + ra;

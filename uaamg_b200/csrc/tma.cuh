@@ -121,6 +121,10 @@ __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+__device__ __forceinline__ void tma_prefetch(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
 template <int DIM>
 __device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int x, int y, int z,
                                          uint64_t* bar) {

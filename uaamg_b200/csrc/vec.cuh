@@ -17,6 +17,19 @@ struct Vec16;
 template <> struct Vec16<float> { using V = float4; static constexpr int N = 4; };
 template <> struct Vec16<double> { using V = double2; static constexpr int N = 2; };
 
+// 16-byte loads that stay where they are written (common.cuh, ld_now).
+__device__ __forceinline__ float4 ld_vec_now(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double2 ld_vec_now(const double2* p) {
+    double2 v;
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
 template <class T>
 __device__ __forceinline__ void vaxpy_rr(typename Vec16<T>::V& x, typename Vec16<T>::V& r,
                                          const typename Vec16<T>::V& p,
@@ -69,11 +82,7 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
                                                      const T* __restrict__ p,
                                                      const T* __restrict__ ap, double* xhi,
                                                      double* partials, CGState* cg, double* hist) {
-    pdl_entry();
-    if (cg->done) return;
     using V = typename Vec16<T>::V;
-    const T alpha = (T)cg->alpha;
-    const bool fold = xhi && cg->fold;
     V* xv = reinterpret_cast<V*>(x);
     V* rv = reinterpret_cast<V*>(r);
     const V* pv = reinterpret_cast<const V*>(p);
@@ -81,6 +90,28 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
     double acc[1] = {0.0};
     const long long stride = (long long)gridDim.x * blockDim.x;
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    // the first two vectors: x and r (written an iteration ago) ahead of the wait, p and
+    // Ap beside the stop flag and the scalars
+    V x0[2] = {}, r0[2] = {}, p0[2] = {}, a0[2] = {};
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        if (t + u * stride < nvec) {
+            x0[u] = ld_vec_now(&xv[t + u * stride]);
+            r0[u] = ld_vec_now(&rv[t + u * stride]);
+        }
+    pdl_wait();
+    const int stop = ld_now(&cg->done);
+    const int fold_now = xhi ? ld_now(&cg->fold) : 0;
+    const T alpha = (T)cg->alpha;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        if (t + u * stride < nvec) {
+            p0[u] = ld_vec_now(&pv[t + u * stride]);
+            a0[u] = ld_vec_now(&av[t + u * stride]);
+        }
+    pdl_launch();
+    if (stop) return;
+    const bool fold = fold_now != 0;
     if (fold) {  // after a replacement (one iteration in replace_every): one vector a trip
         for (; t < nvec; t += stride) {
             V xx = xv[t], rr_ = rv[t];
@@ -91,6 +122,14 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             rv[t] = rr_;
         }
     } else {  // two vectors a thread per trip, their loads issued together
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (t + u * stride < nvec) {
+                vaxpy_rr<T>(x0[u], r0[u], p0[u], a0[u], alpha, acc[0]);
+                xv[t + u * stride] = x0[u];
+                rv[t + u * stride] = r0[u];
+            }
+        t += 2 * stride;
         for (; t + stride < nvec; t += 2 * stride) {
             const long long t2 = t + stride;
             V xx = xv[t], rr_ = rv[t], x2 = xv[t2], r2 = rv[t2];
