@@ -188,7 +188,6 @@ uaamg_status solve_dev(uaamg_handle* h, const double* d_rhs, double* d_p, const 
     uaamg_status s = engine_for(h, opts.precision, &eng);
     if (s != UAAMG_OK) return s;
     if ((s = ensure_hist(h, opts.max_iter)) != UAAMG_OK) return s;
-    cudaMemsetAsync(h->d_hist, 0, sizeof(double) * (size_t)h->hist_cap, h->stream);
     uaamg::SolveArgs a;
     a.rhs = d_rhs;
     a.x = d_p;

@@ -69,7 +69,8 @@ struct CGState {
     double tol_abs;    // stop when sqrt(r.r) < tol_abs
     double mean_z;     // fluid mean of z (null-space projection)
     double nfluid;     // fluid cell count
-    double sum0, sum1; // scratch sums (RHS normalisation)
+    double sum0, sum1; // right-hand side: sum over the fluid cells, sum after the first
+                       // projection; sum0 also of the result's mean projection
     double bnorm;      // ||b|| of the normalised right-hand side
     double breakdown;  // p.Ap below this stops the solve (the reference's 1e-15)
     int done;          // 1 once the solve stopped; every loop kernel then returns at once
@@ -83,6 +84,7 @@ struct CGState {
     int init;          // 1 while forming p0 = z0 (beta = 0)
     int fold;          // mixed mode: the next x update first folds x_lo into x_hi
     unsigned int counter[8];  // last-block counters, one per reduction site
+    int err;           // set by a kernel whose TMA wait gave up
 };
 
 // q = a / d and r = a % d for 0 <= a < 2^31, 0 < d, from a reciprocal 1/d computed

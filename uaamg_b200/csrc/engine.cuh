@@ -176,6 +176,7 @@ public:
         if (lv_.empty()) return E_NOPROB;
         launches_ = 0;
         cudaMemsetAsync(err_, 0, sizeof(int), st_);
+        err_known_ = false;
         if (dim_ == 3) precond_impl<3>(d_r, d_z); else precond_impl<2>(d_r, d_z);
         return sync_check();
     }
@@ -241,6 +242,7 @@ public:
         int e = sync_check();
         if (e != E_OK) return e;
         const CGState& c = *cg_host_;
+        err_known_ = true;
         res->status = c.status;
         res->iterations = c.iter;
         res->replacements = c.replacements;
@@ -397,6 +399,7 @@ public:
     int timed_out() override {
         int v = 0;
         if (!err_) return 0;
+        if (err_known_) return cg_host_->err;  // a finished solve: copied with its state
         if (cudaMemcpy(&v, err_, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
         return v;
     }
@@ -416,7 +419,8 @@ private:
     long vver_ = 0, vconv_ = -1;     // contents version set / converted into vf_
     float* vf_[3] = {nullptr, nullptr, nullptr};  // FP32 forms: s, ox, oy (level layout)
     double *b64_ = nullptr, *xd_ = nullptr, *partials_ = nullptr;
-    int* err_ = nullptr;             // set by a kernel whose TMA wait gave up
+    int* err_ = nullptr;             // cg_'s error word, set by a kernel whose TMA wait gave up
+    bool err_known_ = false;         // cg_host_ holds it
     CUtensorMap map_p_, map_p2_;     // plane boxes of the two search-direction buffers
     CUtensorMap map_b64_, map_xd_, map_xlo_;  // plane boxes of b, x_hi (FP64) and x_lo (3D)
     SolveArgs cur_{};                // the solve in progress
@@ -856,8 +860,8 @@ private:
             if (reduce_blocks_ < max_reduce_blocks()) reduce_blocks_ = max_reduce_blocks();
         }
         if ((e = alloc(partials_, (size_t)reduce_blocks_ * 4))) return e;
-        if ((e = alloc(err_, 1))) return e;
         if ((e = alloc(cg_, 1))) return e;
+        err_ = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(cg_) + offsetof(CGState, err));
         if (dense_cells_ > 0) {
             if ((e = alloc(dense_, (size_t)dense_cells_ * dense_ld_))) return e;
             if ((e = alloc(dense_cell_, (size_t)dense_cells_))) return e;
@@ -947,7 +951,9 @@ private:
         }
         if (DIM == 3) {
             if ((e = smem_attr(k_resid_march<T, true>, RxCfg<T>::BYTES)) ||
-                (e = smem_attr(k_resid_march<T, false>, RxCfg<T>::BYTES)))
+                (e = smem_attr(k_resid_march<T, false>, RxCfg<T>::BYTES)) ||
+                (e = smem_attr(k_resid_march<T, true, true>, RxCfg<T>::BYTES)) ||
+                (e = smem_attr(k_resid_march<T, false, true>, RxCfg<T>::BYTES)))
                 return e;
             // planes per block of the replacement march: chunks doubled until the blocks
             // fit in one wave (256^3: 64 planes, 512 blocks; 1.31 against 1.37 ms a solve
@@ -1655,10 +1661,13 @@ private:
         }
     }
 
-    // One PCG iteration (pcg_3d.cpp:93-124); the search direction alternates between
-    // p_ and p2_ (from_p: the current one lives in p_).
+    // One PCG iteration (pcg_3d.cpp:93-124), begun at its preconditioner application: z =
+    // M r, the search direction, the update, the residual replacement when due -- so the
+    // captured step holds a solve's first application too.  The search direction
+    // alternates between p_ and p2_ (from_p: the current one lives in p_).
     template <int DIM>
     void cg_iteration(bool from_p) {
+        cg_precond<DIM>();
         const Geom& g = lv_[0].g;
         const Stencil st = stencil();
         T* pnew = from_p ? p2_ : p_;
@@ -1693,26 +1702,29 @@ private:
             // return at once): b, x_hi, x_lo, codes in; r out
             nopdl_next_ = cells(g) > 1048576.0;
             const KTag tag{K_REPLACE, 0, cells(g) * (17.0 + 2.0 * sizeof(T))};
-            if (DIM == 3) {
-                MarchMaps rm;
-                rm.v[0] = map_b64_;
-                rm.v[1] = map_xd_;
-                rm.v[2] = map_xlo_;
-                rm.code = lv_[0].mcode;
-                if (dirichlet_)
-                    UAAMG_LAUNCH_SMEM(tag, (k_resid_march<T, true>), march_grid<DIM>(g, rx_zc_),
-                                      dim3(kThreads), (RxCfg<T>::BYTES), rm, g, rx_zc_, r_, st, partials_,
-                                      cg_, 5, cur_.tol, cur_.tol_mode, err_);
-                else
-                    UAAMG_LAUNCH_SMEM(tag, (k_resid_march<T, false>), march_grid<DIM>(g, rx_zc_),
-                                      dim3(kThreads), (RxCfg<T>::BYTES), rm, g, rx_zc_, r_, st, partials_,
-                                      cg_, 5, cur_.tol, cur_.tol_mode, err_);
+            if constexpr (DIM == 3) {
+                if (dirichlet_) resid_march<true, false>(tag, nullptr);
+                else resid_march<false, false>(tag, nullptr);
             } else {
                 UAAMG_LAUNCH(tag, (k_resid_x64<DIM, T>), resid_grid(g), dim3(32, 8), g, lv_[0].code, b64_,
-                             xd_, xlo_, r_, st, kResidZc, partials_, cg_, 5, 1, cur_.tol, cur_.tol_mode);
+                             xd_, xlo_, r_, st, kResidZc, partials_, cg_, 5, 1, cur_.tol, cur_.tol_mode,
+                             gref_, (double*)nullptr);
             }
         }
-        cg_precond<DIM>();
+    }
+
+    // The FP64 residual march: a replacement, or (EXIT) a solve's end, adding x to dst.
+    template <bool DIRW, bool EXIT>
+    void resid_march(const KTag& tag, double* dst) {
+        const Geom& g = lv_[0].g;
+        MarchMaps rm;
+        rm.v[0] = map_b64_;
+        rm.v[1] = map_xd_;
+        rm.v[2] = map_xlo_;
+        rm.code = lv_[0].mcode;
+        UAAMG_LAUNCH_SMEM(tag, (k_resid_march<T, DIRW, EXIT>), march_grid<3>(g, rx_zc_), dim3(kThreads),
+                          (RxCfg<T>::BYTES), rm, g, rx_zc_, r_, stencil(), partials_, cg_, 5, cur_.tol,
+                          cur_.tol_mode, err_, gref_, dst);
     }
 
     template <int DIM>
@@ -1750,27 +1762,25 @@ private:
         *cg_host_ = init;
         if (cudaMemcpyAsync(cg_, cg_host_, sizeof(CGState), cudaMemcpyHostToDevice, st_) != cudaSuccess)
             return E_CUDA;
-        cudaMemsetAsync(err_, 0, sizeof(int), st_);
+        err_known_ = false;
 
-        // b = -(rhs - mean), re-projected; ||b|| (pcg_3d.cpp:22-36, 80-81)
-        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 16.0}), (k_import<DIM, double>), vg, vb, g, gref_, a.rhs, b64_);
-        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 9.0}), k_sum_count<DIM>, vg, vb, g, s, b64_, partials_, cg_, 3);
-        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 17.0}), k_rhs_negate<DIM>, vg, vb, g, s, b64_, b64_, cg_);
-        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 9.0}), k_sum_count<DIM>, vg, vb, g, s, b64_, partials_, cg_, 3);
-        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 17.0}), k_sub_mean<DIM>, vg, vb, g, s, b64_, cg_);
-        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 9.0}), k_norm<DIM>, vg, vb, g, s, b64_, partials_, cg_, 4);
+        // b = -(rhs - mean), re-projected; ||b|| (pcg_3d.cpp:22-36, 80-81); r, x and p
+        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 9.0}), k_rhs_sum<DIM>, vg, vb, g, gref_, s, a.rhs,
+                     partials_, cg_, 3, 0, a.hist);
+        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 9.0}), k_rhs_sum<DIM>, vg, vb, g, gref_, s, a.rhs,
+                     partials_, cg_, 3, 1, (double*)nullptr);
+        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * (25.0 + 3.0 * sizeof(T))}), (k_rhs_write<DIM, T>), vg, vb,
+                     g, gref_, s, a.rhs, b64_, a.warm ? (T*)nullptr : r_, xlo_, p_, xd_, partials_, cg_, 4,
+                     a.tol, a.tol_mode);
         if (a.warm) {  // b <- b - A x_in: the solve then finds the correction to x_in
             if (a.x_ready) cudaStreamWaitEvent(st_, a.x_ready, 0);
             UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * 16.0}), (k_import<DIM, double>), vg, vb, g, gref_, a.x, xd_);
             UAAMG_LAUNCH((KTag{K_TRUE_RESIDUAL, 0, cells(g) * 25.0}), (k_true_residual<DIM, double>), vg, vb,
                          g, s, b64_, xd_, b64_, st, partials_, cg_, 5, 3, a.tol, a.tol_mode);
+            UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * (9.0 + sizeof(T))}), (k_true_residual<DIM, T>), vg, vb, g, s,
+                         b64_, (const double*)nullptr, r_, st, partials_, cg_, 5, 0, a.tol, a.tol_mode);
+            cudaMemsetAsync(xd_, 0, (size_t)n * sizeof(double), st_);
         }
-        UAAMG_LAUNCH((KTag{K_RHS, 0, cells(g) * (9.0 + sizeof(T))}), (k_true_residual<DIM, T>), vg, vb, g, s,
-                     b64_, (const double*)nullptr, r_, st, partials_, cg_, 5, 0, a.tol, a.tol_mode);
-        cudaMemsetAsync(xlo_, 0, (size_t)n * sizeof(T), st_);
-        cudaMemsetAsync(p_, 0, (size_t)n * sizeof(T), st_);
-        cudaMemsetAsync(xd_, 0, (size_t)n * sizeof(double), st_);
-        cg_precond<DIM>();
 
         // Two iterations form one step (the search direction is back in p_ after
         // it); outside profiling the step is a CUDA graph captured once per problem
@@ -1839,16 +1849,19 @@ private:
         const dim3 vg = vec_grid(g);
         const Stencil st = stencil();
         const SolveArgs& a = cur_;
-        // the solution: x_hi + x_lo in mixed mode, else the working x alone
-        const double* xhi = mixed_ ? xd_ : nullptr;
+        // exit diagnostics, the FP64 true residual of the accumulated solution (x_hi + x_lo in
+        // mixed mode, else the working x; x_hi is 0 then), and that solution out
         const double xb = (mixed_ ? 8.0 : 0.0) + sizeof(T);
-        // exit diagnostics: FP64 true residual of the accumulated solution
-        UAAMG_LAUNCH((KTag{K_TRUE_RESIDUAL, 0, cells(g) * (9.0 + xb)}), (k_resid_x64<DIM, T>),
-                     resid_grid(g), dim3(32, 8), g, lv_[0].code, b64_, xhi, xlo_, (T*)nullptr, st,
-                     kResidZc, partials_, cg_, 5, 2, a.tol, a.tol_mode);
         if (a.x_ready) cudaStreamWaitEvent(st_, a.x_ready, 0);  // the caller's x, accumulated into
-        UAAMG_LAUNCH((KTag{K_OUTPUT, 0, cells(g) * (16.0 + xb)}), (k_export_x<DIM, T>), vg, vb, g, gref_,
-                     xhi, xlo_, a.x, 1);
+        const KTag tag{K_TRUE_RESIDUAL, 0, cells(g) * (25.0 + xb)};
+        if constexpr (DIM == 3) {
+            if (dirichlet_) resid_march<true, true>(tag, a.x);
+            else resid_march<false, true>(tag, a.x);
+        } else {
+            UAAMG_LAUNCH(tag, (k_resid_x64<DIM, T>), resid_grid(g), dim3(32, 8), g, lv_[0].code, b64_,
+                         mixed_ ? xd_ : (double*)nullptr, xlo_, (T*)nullptr, st, kResidZc, partials_, cg_,
+                         5, 2, a.tol, a.tol_mode, gref_, a.x);
+        }
         if (a.project_mean && a.ref_solid) {
             const dim3 rg = vec_grid(gref_);
             UAAMG_LAUNCH((KTag{K_OUTPUT, 0, cells(g) * 9.0}), k_sum_count<DIM>, rg, vb, gref_, a.ref_solid,

@@ -433,20 +433,6 @@ __global__ void k_sum_count(Geom g, const uint8_t* __restrict__ s, const double*
     }
 }
 
-// b = -(rhs - mean) on fluid interior cells, 0 elsewhere (pcg_3d.cpp:22-36);
-// mean = sum0/nfluid unless Dirichlet.  b may alias rhs (each cell reads its own
-// value before writing it).
-template <int DIM>
-__global__ void k_rhs_negate(Geom g, const uint8_t* __restrict__ s, const double* rhs, double* b,
-                             const CGState* cg) {
-    pdl_entry();
-    double mean = cg->nfluid > 0.0 ? cg->sum0 / cg->nfluid : 0.0;
-    if (cg->dirichlet) mean = 0.0;
-    for_cells<DIM>(g, [&](int, int, int, int id) {
-        b[id] = s[id] ? 0.0 : -(rhs[id] - mean);
-    });
-}
-
 // v -= mean over fluid cells (pcg_3d.cpp:66-77), mean = sum0/nfluid.
 template <int DIM>
 __global__ void k_sub_mean(Geom g, const uint8_t* __restrict__ s, double* v, const CGState* cg) {
@@ -490,6 +476,70 @@ __device__ __forceinline__ void true_residual_done(CGState* cg, double rr, int m
 __device__ __forceinline__ bool replacement_due(const CGState* cg) {
     return !cg->done && (cg->cand || (cg->replace_every > 0 && cg->iter > 0 &&
                                       cg->iter % cg->replace_every == 0));
+}
+
+// The right-hand side of a solve, b = -(rhs - mean) on fluid interior cells, projected
+// once more (pcg_3d.cpp:22-36, 80-81), in three passes over the caller's array (src, in
+// its layout gr), the first two of which only reduce: the sum and count of rhs; the sum
+// of -(rhs - mean); then b itself, ||b||, and what a solve starts from -- r = b and
+// zero x and p (x_lo, p, x_hi; ghost cells stay 0) -- unless a warm start still has to
+// subtract A x (r == nullptr).  Three kernels of about 60 bytes a cell where seven kernels
+// and three fills moved 106.  With the exit in one pass and the first preconditioner
+// application in the captured step, a solve without an iteration takes 50 us at 384^2
+// (was 136, with that application), 610 us at 256^3 (was 1510).
+template <int DIM>
+__device__ __forceinline__ double rhs_mean(const CGState* cg, double sum) {
+    return !cg->dirichlet && cg->nfluid > 0.0 ? sum / cg->nfluid : 0.0;
+}
+template <int DIM>
+__global__ void k_rhs_sum(Geom g, Geom gr, const uint8_t* __restrict__ s,
+                          const double* __restrict__ src, double* partials, CGState* cg, int slot,
+                          int second, double* hist) {
+    pdl_entry();
+    const double mean = second ? rhs_mean<DIM>(cg, cg->sum0) : 0.0;
+    if (hist && blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) hist[0] = 0.0;
+    double acc[2] = {0.0, 0.0};
+    for_cells<DIM>(g, [&](int i, int j, int k, int id) {
+        if (!s[id]) {
+            const double v = src[cidx(gr, i, j, k)];
+            acc[0] += second ? -(v - mean) : v;
+            acc[1] += 1.0;
+        }
+    });
+    double tot[2];
+    if (reduce_last<2>(acc, partials, &cg->counter[slot], tot)) {
+        if (second) cg->sum1 = tot[0];
+        else cg->sum0 = tot[0];
+        cg->nfluid = tot[1];
+    }
+}
+__device__ __forceinline__ void true_residual_done(CGState* cg, double rr, int mode, double tol,
+                                                   int tol_mode);
+template <int DIM, class T>
+__global__ void k_rhs_write(Geom g, Geom gr, const uint8_t* __restrict__ s,
+                            const double* __restrict__ src, double* __restrict__ b, T* __restrict__ r,
+                            T* __restrict__ x, T* __restrict__ p, double* __restrict__ xhi,
+                            double* partials, CGState* cg, int slot, double tol, int tol_mode) {
+    pdl_entry();
+    const double mean = rhs_mean<DIM>(cg, cg->sum0), mean2 = rhs_mean<DIM>(cg, cg->sum1);
+    double acc[1] = {0.0};
+    for_cells<DIM>(g, [&](int i, int j, int k, int id) {
+        double v = 0.0;
+        if (!s[id]) {
+            v = -(src[cidx(gr, i, j, k)] - mean) - mean2;
+            acc[0] += v * v;
+        }
+        b[id] = v;
+        if (r) r[id] = (T)v;
+        x[id] = T(0);
+        p[id] = T(0);
+        xhi[id] = 0.0;
+    });
+    double tot[1];
+    if (reduce_last<1>(acc, partials, &cg->counter[slot], tot)) {
+        cg->bnorm = sqrt(tot[0]);
+        if (r) true_residual_done(cg, tot[0], 0, tol, tol_mode);
+    }
 }
 
 // r = b - A x (FP64), copied into the working residual rw (type T), with
@@ -539,7 +589,8 @@ __global__ void k_true_residual(Geom g, const uint8_t* __restrict__ s, const dou
 // keeping x of the planes below, at and above in registers; every load of a step
 // is independent of the others.  Writes r as T to rw (0 on solid cells) when
 // given, reduces r.r; mode 1 (residual replacement, gated as replacement_due) also
-// asks the next x update to fold x_lo into x_hi; mode 2: exit diagnostics.
+// asks the next x update to fold x_lo into x_hi; mode 2: exit diagnostics, and x is
+// added to the caller's array dst (layout gr).
 // Every product and sum rounds by itself, as the reference's build does, in the FP32
 // engines too (whose unit contracts multiply-adds): a residual near 1e-12 of ||b|| is
 // mostly rounding, and this way the reported one is a host's to the last digits.
@@ -550,7 +601,8 @@ __global__ void __launch_bounds__(256) k_resid_x64(Geom g, const uint8_t* __rest
                                                    const double* __restrict__ xhi,
                                                    const T* __restrict__ xlo, T* __restrict__ rw,
                                                    Stencil st, int zc, double* partials, CGState* cg,
-                                                   int slot, int mode, double tol, int tol_mode) {
+                                                   int slot, int mode, double tol, int tol_mode,
+                                                   Geom gr, double* __restrict__ dst) {
     pdl_entry();
     if (mode == 1 && !replacement_due(cg)) return;
     double acc[1] = {0.0};
@@ -593,6 +645,7 @@ __global__ void __launch_bounds__(256) k_resid_x64(Geom g, const uint8_t* __rest
             const double r = (c & kActive) ? rn_sub(bb, ax) : 0.0;
             acc[0] += r * r;
             if (rw) rw[id] = (T)r;
+            if (dst) dst[cidx(gr, i, j, k)] += xc;
             xm = xc;
             xc = xp;
         }
@@ -749,19 +802,6 @@ __global__ void __launch_bounds__(256) k_pmatvec_2d(Geom g, const uint8_t* __res
         else if (pap < cg->breakdown) { cg->status = CG_BREAKDOWN; cg->done = 1; }
         else cg->alpha = cg->rz_old / pap;
     }
-}
-
-// ||b||^2 over fluid cells -> cg->bnorm (FP64).
-template <int DIM>
-__global__ void k_norm(Geom g, const uint8_t* __restrict__ s, const double* __restrict__ b,
-                       double* partials, CGState* cg, int slot) {
-    pdl_entry();
-    double acc[1] = {0.0};
-    for_cells<DIM>(g, [&](int, int, int, int id) {
-        if (!s[id]) acc[0] += b[id] * b[id];
-    });
-    double tot[1];
-    if (reduce_last<1>(acc, partials, &cg->counter[slot], tot)) cg->bnorm = sqrt(tot[0]);
 }
 
 // Null-space projection of z and the new r.z (pcg_3d.cpp:112-123), given the

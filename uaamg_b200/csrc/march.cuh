@@ -1055,13 +1055,17 @@ template <class T> struct RxCfg {
     static constexpr size_t BYTES = Lay::OFF_EXTRA + 2 * align128(PBox<double>::BYTES);
 };
 
-template <class T, bool DIRW = true>
+// EXIT: the end of a solve instead: the residual is reported only, every product and sum
+// rounded by itself as in k_resid_x64, and x is added to the caller's array dst (layout
+// gr) -- one pass for the column walk and the separate export, 152 + 109 us at 256^3.
+template <class T, bool DIRW = true, bool EXIT = false>
 __global__ void __launch_bounds__(kThreads) k_resid_march(const __grid_constant__ MarchMaps M, Geom g,
                                                           int zc, T* __restrict__ rw, Stencil st,
                                                           double* partials, CGState* cg, int slot,
-                                                          double tol, int tol_mode, int* err) {
+                                                          double tol, int tol_mode, int* err, Geom gr,
+                                                          double* __restrict__ dst) {
     pdl_entry();
-    if (!replacement_due(cg)) return;
+    if (!EXIT && !replacement_due(cg)) return;
     using C = RxCfg<T>;
     using P = typename C::P;
     using Lay = typename C::Lay;
@@ -1135,6 +1139,16 @@ __global__ void __launch_bounds__(kThreads) k_resid_march(const __grid_constant_
             const double vT = (c & 4u) ? (e ? xbc[q + WD] : xc[1]) : (!DIRW || j < g.ny ? x0 : wall);
             const double vF = (c & 32u) ? xm[e] : (!DIRW || k > 1 ? x0 : wall);
             const double vK = (c & 16u) ? xn[e] : (!DIRW || k < g.nz ? x0 : wall);
+            if constexpr (EXIT) {
+                const double ax = rn_sub(rn_sub(rn_sub(__dmul_rn(diag, x0), __dmul_rn(vL + vR, idx2)),
+                                                __dmul_rn(vB + vT, idy2)), __dmul_rn(vF + vK, idz2));
+                const double r = (c & kActive) ? rn_sub(bc[e], ax) : 0.0;
+                if (e ? o.inb : o.ina) {
+                    acc[0] += r * r;
+                    dst[cidx(gr, i, j, k)] += x0;
+                }
+                continue;
+            }
             const double ax = diag * x0 - (vL + vR) * idx2 - (vB + vT) * idy2 - (vF + vK) * idz2;
             const double r = (c & kActive) ? bc[e] - ax : 0.0;
             if (e ? o.inb : o.ina) {
@@ -1158,6 +1172,10 @@ __global__ void __launch_bounds__(kThreads) k_resid_march(const __grid_constant_
     }
     double tot[1];
     if (reduce_last<1>(acc, partials, &cg->counter[slot], tot)) {
+        if (EXIT) {
+            true_residual_done(cg, tot[0], 2, tol, tol_mode);
+            return;
+        }
         cg->fold = 1;
         true_residual_done(cg, tot[0], 1, tol, tol_mode);
         // a replacement at max_iter that did not confirm convergence ends the solve

@@ -186,18 +186,6 @@ __global__ void k_import_mask(Geom g, Geom gr, const uint8_t* __restrict__ src, 
         dst[id] = src[cidx(gr, i, j, k)] ? 1 : 0;
     });
 }
-// The solution x = x_hi + x_lo (either part may be absent) into the reference
-// layout: dst = x (overwrite) or dst += x (accumulate), interior cells.
-template <int DIM, class T>
-__global__ void k_export_x(Geom g, Geom gr, const double* __restrict__ xhi, const T* __restrict__ xlo,
-                           double* dst, int accumulate) {
-    pdl_entry();
-    for_cells<DIM>(g, [&](int i, int j, int k, int id) {
-        const double x = xhi && xlo ? xhi[id] + (double)xlo[id] : (xhi ? xhi[id] : (double)xlo[id]);
-        const int rid = cidx(gr, i, j, k);
-        dst[rid] = accumulate ? dst[rid] + x : x;
-    });
-}
 // dst (reference layout) = src on interior cells (overwrite) or += src (accumulate).
 template <int DIM, class T>
 __global__ void k_export(Geom g, Geom gr, const T* __restrict__ src, double* dst, int accumulate) {
