@@ -852,7 +852,9 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
     }
     if constexpr (UP && ZDOT) {
         double tot[3];
-        if (reduce_last<3>(acc, partials, &cg->counter[2], tot)) finish_zdot(cg, tot);
+        ZdotIn in;
+        if (reduce_last<3>(acc, partials, &cg->counter[2], tot, [&] { in.load(cg); }))
+            finish_zdot(cg, in, tot);
     }
 }
 
@@ -1338,7 +1340,9 @@ __global__ void __launch_bounds__(kThreads)
         }
         if constexpr (UP && ZDOT) {
             double tot[3];
-            if (reduce_last<3>(acc, partials, &cg->counter[2], tot)) finish_zdot(cg, tot);
+            ZdotIn in;
+        if (reduce_last<3>(acc, partials, &cg->counter[2], tot, [&] { in.load(cg); }))
+            finish_zdot(cg, in, tot);
         }
     };
     if constexpr (FINE) {

@@ -37,9 +37,19 @@ __device__ __forceinline__ int cidx(const Geom& g, int i, int j, int k) {
 // partial sums to partials[block*NV + q]; the last block to arrive (atomic
 // counter) re-reads all partials in a fixed order and returns true in its thread 0
 // with the totals in tot.  The counter is reset for the next launch.
-template <int NV>
+// The end of a reduction is a chain of latencies in one block -- arrival, partials, the
+// scalars the outcome needs -- that all later kernels wait for.  The arrival is one
+// acquire-release atomic (its release covers the partials the same thread wrote, its
+// acquire and the block barrier order the other threads' reads), and pre() runs in the
+// last block's thread 0 beside the partials' loads: the caller loads the scalars there.
+// A 384^2 iteration (three reductions) 44.2 -> 41.3 us, one of 96^3 FP64 114 -> 111.
+struct NoPre {
+    __device__ __forceinline__ void operator()() const {}
+};
+template <int NV, class Pre = NoPre>
 __device__ __forceinline__ bool reduce_last(double (&v)[NV], double* partials,
-                                            unsigned int* counter, double (&tot)[NV]) {
+                                            unsigned int* counter, double (&tot)[NV],
+                                            Pre&& pre = NoPre()) {
     __shared__ double sm[32][NV];
     __shared__ int am_last;
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
@@ -61,13 +71,13 @@ __device__ __forceinline__ bool reduce_last(double (&v)[NV], double* partials,
             for (int w = 0; w < nwarp; ++w) s += sm[w][q];
             partials[(size_t)bid * NV + q] = s;
         }
-        __threadfence();
-        unsigned prev = atomicAdd(counter, 1u);
+        unsigned prev;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(counter) : "memory");
         am_last = (prev == nblk - 1) ? 1 : 0;
     }
     __syncthreads();
     if (!am_last) return false;
-    __threadfence();
+    if (tid == 0) pre();
     double acc[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q] = 0.0;
@@ -795,26 +805,40 @@ __global__ void __launch_bounds__(256) k_pmatvec_2d(Geom g, const uint8_t* __res
         }
     }
     double tot[1];
-    if (reduce_last<1>(acc, partials, &cg->counter[0], tot)) {
+    double rz_old = 0.0, breakdown = 0.0;
+    if (reduce_last<1>(acc, partials, &cg->counter[0], tot, [&] {
+            rz_old = ld_now(&cg->rz_old);
+            breakdown = ld_now(&cg->breakdown);
+        })) {
         const double pap = tot[0];
         cg->pap = pap;
         if (!(pap == pap)) { cg->status = CG_NAN; cg->done = 1; }
-        else if (pap < cg->breakdown) { cg->status = CG_BREAKDOWN; cg->done = 1; }
-        else cg->alpha = cg->rz_old / pap;
+        else if (pap < breakdown) { cg->status = CG_BREAKDOWN; cg->done = 1; }
+        else cg->alpha = rz_old / pap;
     }
 }
 
 // Null-space projection of z and the new r.z (pcg_3d.cpp:112-123), given the
 // fluid sums of z, r*z and r: with m = mean_fluid(z), r.(z - m) = r.z - m*sum(r).
 // Sets beta = rz/rz_old (0 when forming p0) and rz_old = rz.
-__device__ __forceinline__ void finish_zdot(CGState* cg, const double (&tot)[3]) {
+struct ZdotIn {
+    double nfluid, rz_old;
+    int dirichlet, init;
+    __device__ __forceinline__ void load(const CGState* cg) {
+        nfluid = ld_now(&cg->nfluid);
+        rz_old = ld_now(&cg->rz_old);
+        dirichlet = ld_now(&cg->dirichlet);
+        init = ld_now(&cg->init);
+    }
+};
+__device__ __forceinline__ void finish_zdot(CGState* cg, const ZdotIn& in, const double (&tot)[3]) {
     double m = 0.0, rz = tot[1];
-    if (!cg->dirichlet) {
-        m = cg->nfluid > 0.0 ? tot[0] / cg->nfluid : 0.0;
+    if (!in.dirichlet) {
+        m = in.nfluid > 0.0 ? tot[0] / in.nfluid : 0.0;
         rz = tot[1] - m * tot[2];
     }
     cg->mean_z = m;
-    cg->beta = cg->init ? 0.0 : rz / cg->rz_old;
+    cg->beta = in.init ? 0.0 : rz / in.rz_old;
     cg->rz_old = rz;
     cg->init = 0;
     if (!(rz == rz)) { cg->status = CG_NAN; cg->done = 1; }
@@ -837,7 +861,9 @@ __global__ void k_zdot(Geom g, const uint8_t* __restrict__ s, const T* __restric
         }
     });
     double tot[3];
-    if (reduce_last<3>(acc, partials, &cg->counter[2], tot)) finish_zdot(cg, tot);
+    ZdotIn in;
+        if (reduce_last<3>(acc, partials, &cg->counter[2], tot, [&] { in.load(cg); }))
+            finish_zdot(cg, in, tot);
 }
 
 }  // namespace

@@ -867,7 +867,9 @@ __global__ void __launch_bounds__(kThreads) k_up_odd(const __grid_constant__ Mar
     }
     if (ZDOT) {
         double tot[3];
-        if (reduce_last<3>(acc, partials, &cg->counter[2], tot)) finish_zdot(cg, tot);
+        ZdotIn in;
+        if (reduce_last<3>(acc, partials, &cg->counter[2], tot, [&] { in.load(cg); }))
+            finish_zdot(cg, in, tot);
     }
 }
 
@@ -1016,12 +1018,16 @@ __global__ void __launch_bounds__(kThreads, DIRW ? 1 : PmvCfg<DIM, T>::MINB)
         if (tid == 0) R.refill(M, k + 1);
     }
     double tot[1];
-    if (reduce_last<1>(acc, partials, &cg->counter[0], tot)) {
+    double rz_old = 0.0, breakdown = 0.0;
+    if (reduce_last<1>(acc, partials, &cg->counter[0], tot, [&] {
+            rz_old = ld_now(&cg->rz_old);
+            breakdown = ld_now(&cg->breakdown);
+        })) {
         const double pap = tot[0];
         cg->pap = pap;
         if (!(pap == pap)) { cg->status = CG_NAN; cg->done = 1; }
-        else if (pap < cg->breakdown) { cg->status = CG_BREAKDOWN; cg->done = 1; }
-        else cg->alpha = cg->rz_old / pap;
+        else if (pap < breakdown) { cg->status = CG_BREAKDOWN; cg->done = 1; }
+        else cg->alpha = rz_old / pap;
     }
 }
 

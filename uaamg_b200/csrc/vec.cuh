@@ -150,26 +150,32 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
         }
     }
     double tot[1];
-    if (reduce_last<1>(acc, partials, &cg->counter[1], tot)) {
+    double tol_abs = 0.0, first = 0.0;
+    int it = 0, every = 0, max_iter = 0, cand = 0;
+    if (reduce_last<1>(acc, partials, &cg->counter[1], tot, [&] {
+            tol_abs = ld_now(&cg->tol_abs);
+            first = ld_now(&cg->r0);
+            it = ld_now(&cg->iter);
+            every = ld_now(&cg->replace_every);
+            max_iter = ld_now(&cg->max_iter);
+            cand = ld_now(&cg->cand);
+        })) {
         if (fold) cg->fold = 0;  // every other block has finished its loop
         const double rr = tot[0];
         cg->rr = rr;
-        cg->iter += 1;
+        cg->iter = ++it;
         if (hist) {
-            if (cg->iter == 1) hist[0] = cg->r0;
-            hist[cg->iter] = sqrt(rr);
+            if (it == 1) hist[0] = first;
+            hist[it] = sqrt(rr);
         }
-        if (!(rr == rr)) { cg->status = CG_NAN; cg->done = 1; }
-        else if (sqrt(rr) < cg->tol_abs) {
-            if (cg->replace_every > 0) cg->cand = 1;
-            else { cg->status = CG_CONVERGED; cg->done = 1; }
-        } else if (cg->iter >= cg->max_iter && cg->replace_every == 0) {
-            cg->status = CG_MAXITER; cg->done = 1;
-        }
-        if (cg->replace_every > 0 && !cg->done && cg->iter >= cg->max_iter && !cg->cand) {
-            cg->status = CG_MAXITER;
-            cg->done = 1;
-        }
+        int status = CG_RUNNING;
+        if (!(rr == rr)) status = CG_NAN;
+        else if (sqrt(rr) < tol_abs) {
+            if (every > 0) { cand = 1; cg->cand = 1; }
+            else status = CG_CONVERGED;
+        } else if (it >= max_iter && every == 0) status = CG_MAXITER;
+        if (every > 0 && status == CG_RUNNING && it >= max_iter && !cand) status = CG_MAXITER;
+        if (status != CG_RUNNING) { cg->status = status; cg->done = 1; }
     }
 }
 
