@@ -85,7 +85,20 @@ struct CGState {
     int fold;          // mixed mode: the next x update first folds x_lo into x_hi
     unsigned int counter[8];  // last-block counters, one per reduction site
     int err;           // set by a kernel whose TMA wait gave up
+    int epoch;         // number of this solve (its progress words carry it)
+    unsigned long long* progress;  // pinned host word: where the solve is (publish)
 };
+
+// A solve's progress word in pinned host memory: epoch, completed updates, stopped.  The
+// host reads it instead of queueing a copy of the stop flag and an event behind every
+// step (two stream operations a step, and a gap before the next step).
+__host__ __device__ inline unsigned long long progress_word(int epoch, int iter, int done) {
+    return ((unsigned long long)(epoch & 0xffff) << 48) | ((unsigned long long)(unsigned)iter << 1) |
+           (done ? 1u : 0u);
+}
+__device__ __forceinline__ void publish(unsigned long long* to, int epoch, int iter, int done) {
+    if (to) *(volatile unsigned long long*)to = progress_word(epoch, iter, done);
+}
 
 // q = a / d and r = a % d for 0 <= a < 2^31, 0 < d, from a reciprocal 1/d computed
 // once (rd): the double-precision estimate is off by at most one and one exact
@@ -124,6 +137,11 @@ __device__ __forceinline__ void pdl_launch() {
 __device__ __forceinline__ int ld_now(const int* p) {
     int v;
     asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned long long* ld_now(unsigned long long* const* p) {
+    unsigned long long* v;
+    asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ float ld_now(const float* p) {

@@ -192,20 +192,26 @@ public:
         return dim_ == 3 ? step_impl<3>() : step_impl<2>();
     }
 
-    // The device is known to have stopped once the flag copied after some step
-    // reads 1, or once every queued step has finished after max_iter was reached.
+    // The progress word (common.cuh) says how many updates are done and whether the device
+    // has stopped; a step is seen once its second update is.  Now and then the stream is
+    // asked too: a failed launch ends in E_CUDA, and steps that ran without advancing the
+    // word (a kernel gave up on its loads) count as seen, so that max_iter ends the solve.
     int solve_poll(bool wait, bool* stopped) override {
         while (!stopped_ && seen_ < nstep_) {
-            const int slot = seen_ & 1;
-            if (wait) {
-                if (cudaEventSynchronize(ev_[slot]) != cudaSuccess) return E_CUDA;
-            } else {
-                const cudaError_t q = cudaEventQuery(ev_[slot]);
-                if (q == cudaErrorNotReady) break;
-                if (q != cudaSuccess) return E_CUDA;
+            const unsigned long long w = *(volatile unsigned long long*)flag_host_;
+            if ((w >> 48) == (unsigned long long)(epoch_ & 0xffff)) {
+                if (w & 1) { stopped_ = true; break; }
+                if ((long long)((w & 0xffffffffffffull) >> 1) >= 2LL * (seen_ + 1)) { ++seen_; continue; }
             }
-            if (flag_host_[slot]) stopped_ = true;
-            ++seen_;
+            if ((++polls_ & 0xffff) == 0) {
+                const cudaError_t q = cudaStreamQuery(st_);
+                if (q == cudaSuccess && w == *(volatile unsigned long long*)flag_host_) {
+                    seen_ = nstep_;
+                    break;
+                }
+                if (q != cudaSuccess && q != cudaErrorNotReady) return E_CUDA;
+            }
+            if (!wait) break;
         }
         if (!stopped_ && seen_ == nstep_ && it_ >= cur_.max_iter) stopped_ = true;
         *stopped = stopped_;
@@ -431,8 +437,9 @@ private:
     long long reduce_blocks_ = 0;    // partials_ capacity in blocks (4 doubles each)
     CGState* cg_ = nullptr;
     CGState* cg_host_ = nullptr;  // pinned
-    int* flag_host_ = nullptr;    // pinned, 2 slots
-    cudaEvent_t ev_[2] = {nullptr, nullptr};
+    unsigned long long* flag_host_ = nullptr;  // pinned: the progress word
+    int epoch_ = 0;               // solves begun
+    unsigned polls_ = 0;
     cudaStream_t st_ = 0;
     unsigned char* arena_ = nullptr;  // one block for all buffers of a problem
     size_t arena_cap_ = 0, arena_used_ = 0;
@@ -606,8 +613,8 @@ private:
         return v;
     }
 
-    // keep: the buffers' block, the captured step, the pinned host words and the events
-    // stay (set_problem).
+    // keep: the buffers' block, the captured step and the pinned host words stay
+    // (set_problem).
     void release(bool keep = false) {
         if (arena_ || cg_host_) cudaStreamSynchronize(st_);
         for (void* q : extra_) cudaFree(q);
@@ -636,7 +643,6 @@ private:
         if (keep) return;
         if (cg_host_) { cudaFreeHost(cg_host_); cg_host_ = nullptr; }
         if (flag_host_) { cudaFreeHost(flag_host_); flag_host_ = nullptr; }
-        for (auto& e : ev_) if (e) { cudaEventDestroy(e); e = nullptr; }
         if (gexec_) { cudaGraphExecDestroy(gexec_); gexec_ = nullptr; }
         gkey_ = -1;
         gsig_.clear();
@@ -937,9 +943,7 @@ private:
         if ((e = buffers<DIM>()) || (e = arena_ready()) || (e = buffers<DIM>())) return e;
         const Geom g0 = lv_[0].g;
         if (!cg_host_ && cudaMallocHost(&cg_host_, sizeof(CGState)) != cudaSuccess) return E_OOM;
-        if (!flag_host_ && cudaMallocHost(&flag_host_, 2 * sizeof(int)) != cudaSuccess) return E_OOM;
-        for (auto& ev : ev_)
-            if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return E_CUDA;
+        if (!flag_host_ && cudaMallocHost(&flag_host_, sizeof(*flag_host_)) != cudaSuccess) return E_OOM;
         // dynamic shared memory of the marches
         if ((e = march_attrs<DIM, true, CS>()) || (e = march_attrs<DIM, false, CS>()) ||
             (e = smem_attr(k_pmatvec<DIM, T, true>, PmvCfg<DIM, T>::BYTES)) ||
@@ -1759,6 +1763,9 @@ private:
         init.breakdown = a.tol_mode == 0 ? 1e-15 : 1e-300;
         init.dirichlet = dirichlet_;
         init.init = 1;
+        init.epoch = ++epoch_;
+        init.progress = flag_host_;
+        *flag_host_ = progress_word(epoch_, 0, 0);
         *cg_host_ = init;
         if (cudaMemcpyAsync(cg_, cg_host_, sizeof(CGState), cudaMemcpyHostToDevice, st_) != cudaSuccess)
             return E_CUDA;
@@ -1820,12 +1827,11 @@ private:
         return E_OK;
     }
 
-    // Queues one step (two iterations) unless max_iter is reached, then the copy of
-    // the device 'done' flag into slot step % 2 and that slot's event.  Kernels
-    // queued after the solve stopped return at once.
+    // Queues one step (two iterations) unless max_iter is reached.  Kernels queued after
+    // the solve stopped return at once.
     template <int DIM>
     int step_impl() {
-        // two flag slots: a third step waits until the oldest one has been polled
+        // at most two steps ahead of what has been polled
         if (it_ >= cur_.max_iter || nstep_ - seen_ >= 2) return E_OK;
         if (use_graph_) {
             if (cudaGraphLaunch(gexec_, st_) != cudaSuccess) return E_CUDA;
@@ -1835,9 +1841,6 @@ private:
             if (it_ + 1 < cur_.max_iter) cg_iteration<DIM>(false);
         }
         it_ += 2;
-        const int slot = nstep_ & 1;
-        cudaMemcpyAsync(&flag_host_[slot], &cg_->done, sizeof(int), cudaMemcpyDeviceToHost, st_);
-        cudaEventRecord(ev_[slot], st_);
         ++nstep_;
         return E_OK;
     }

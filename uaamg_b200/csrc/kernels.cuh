@@ -669,6 +669,7 @@ __global__ void __launch_bounds__(256) k_resid_x64(Geom g, const uint8_t* __rest
             cg->status = CG_MAXITER;
             cg->done = 1;
         }
+        if (mode == 1) publish(cg->progress, cg->epoch, cg->iter, cg->done);
     }
 }
 

@@ -110,7 +110,10 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             a0[u] = ld_vec_now(&av[t + u * stride]);
         }
     pdl_launch();
-    if (stop) return;
+    if (stop) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) publish(cg->progress, cg->epoch, cg->iter, 1);
+        return;
+    }
     const bool fold = fold_now != 0;
     if (fold) {  // after a replacement (one iteration in replace_every): one vector a trip
         for (; t < nvec; t += stride) {
@@ -151,7 +154,8 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
     }
     double tot[1];
     double tol_abs = 0.0, first = 0.0;
-    int it = 0, every = 0, max_iter = 0, cand = 0;
+    int it = 0, every = 0, max_iter = 0, cand = 0, epoch = 0;
+    unsigned long long* progress = nullptr;
     if (reduce_last<1>(acc, partials, &cg->counter[1], tot, [&] {
             tol_abs = ld_now(&cg->tol_abs);
             first = ld_now(&cg->r0);
@@ -159,6 +163,8 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             every = ld_now(&cg->replace_every);
             max_iter = ld_now(&cg->max_iter);
             cand = ld_now(&cg->cand);
+            epoch = ld_now(&cg->epoch);
+            progress = ld_now(&cg->progress);
         })) {
         if (fold) cg->fold = 0;  // every other block has finished its loop
         const double rr = tot[0];
@@ -176,6 +182,7 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
         } else if (it >= max_iter && every == 0) status = CG_MAXITER;
         if (every > 0 && status == CG_RUNNING && it >= max_iter && !cand) status = CG_MAXITER;
         if (status != CG_RUNNING) { cg->status = status; cg->done = 1; }
+        publish(progress, epoch, it, status != CG_RUNNING);
     }
 }
 
