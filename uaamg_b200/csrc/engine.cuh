@@ -694,8 +694,9 @@ private:
     // Planes per block of a z march over level g with per_sm resident blocks per SM, whose
     // blocks walk extra planes beside their chunk: the even length with the least
     // steps x waves.  A step of an SM's k resident blocks takes k issue-bound units, and
-    // two at least (a lone block waits on its loads and barrier for about that long), so
-    // long chunks save the extra planes, short ones fill a last wave or a small level.
+    // four at least (up to four blocks it is bound by its chain of loads, shared-memory
+    // round trips and barrier), so long chunks save the extra planes, short ones fill a
+    // last wave or a small level.
     // Against chunks halved from 16 until every SM had four blocks: 256^3 mixed, level 1
     // 49 / 40 -> 31 / 28 us a launch down / up, level 0 85 / 91 -> 79 / 83, the solve 8.1 ->
     // 7.55 ms; 96^3 FP64, level 0 way down 28 -> 18 us.
@@ -706,8 +707,8 @@ private:
         for (int zc = 2; zc < g.nz + 2 && zc <= 128; zc += 2) {
             const long long k = (tiles * ((g.nz + zc - 1) / zc) + num_sms_ - 1) / num_sms_;
             const long long full = k / per_sm, rest = k % per_sm;
-            const double cost = (zc + extra) * ((double)full * std::max(2, per_sm) +
-                                                (rest ? std::max<double>(2.0, (double)rest) : 0.0));
+            const double cost = (zc + extra) * ((double)full * std::max(4, per_sm) +
+                                                (rest ? std::max<double>(4.0, (double)rest) : 0.0));
             if (cost < best_cost) { best_cost = cost; best = zc; }
         }
         return best;
@@ -833,7 +834,7 @@ private:
                 if ((e = alloc(L.x, n))) return e;
                 if ((e = alloc(L.b, n))) return e;
                 if ((e = alloc(L.dg, n))) return e;
-                if (L.box) {
+                if (L.box && !cover_) {
                     const dim3 bg = box_grid(L.g);
                     if ((e = alloc(L.trim, (size_t)4 * bg.x * bg.y * bg.z))) return e;
                 }
@@ -1100,16 +1101,18 @@ private:
         if constexpr (DIM == 3) {  // trimmed boxes of the coarse box levels
             for (int l = 1; l < nl; ++l) {
                 const LevelBuf<T, CS>& Cl = lv_[l];
-                if (!Cl.box) continue;
+                // (not for the solves' covering hierarchy: their dozen iterations took the same
+                // time with it and without, and finding the boxes costs 65 us of set-up)
+                if (!Cl.box || !Cl.trim) continue;
                 const MLevel<T> m = mlevel(l);
                 if (kHalf && !Cl.c32)
                     UAAMG_LAUNCH((KTag{K_SETUP, l, 0.0}), (k_box_trim<T, CS>), box_grid(Cl.g), 256,
                                  Cl.g, Cl.code, Cl.dg, Cl.hcx, Cl.hcy, Cl.hcz, m.csx, m.csy, m.csz,
-                                 Cl.trim, star_ ? 3 : 2);
+                                 Cl.trim);
                 else
                     UAAMG_LAUNCH((KTag{K_SETUP, l, 0.0}), (k_box_trim<T, T>), box_grid(Cl.g), 256,
                                  Cl.g, Cl.code, Cl.dg, Cl.cx, Cl.cy, Cl.cz, m.csx, m.csy, m.csz,
-                                 Cl.trim, star_ ? 3 : 2);
+                                 Cl.trim);
             }
         }
         if ((e = dense_setup<DIM>()) != E_OK) return e;

@@ -943,8 +943,8 @@ struct BMaps {
 // diagonal and one coupling per axis needs none of its diagonal, coupling or code
 // boxes: the box kernel loads b (and the parent x) only and uses the four values.
 // The values are the stored ones, so results are identical with and without
-// trimming.  One block of 256 threads per box; rec[4 box + 0] = d or 0.  ring: the ring
-// of the widest box that reads the record (2, with STAR 3).
+// trimming.  One block of 256 threads per box; rec[4 box + 0] = d or 0.  (Boxes with a
+// 2-cell ring: the solves' STAR boxes are not trimmed.)
 template <class E>
 __device__ __forceinline__ bool same_bits(E a, E b) {
     if constexpr (sizeof(E) == 2) return __half_as_ushort(a) == __half_as_ushort(b);
@@ -956,11 +956,11 @@ template <class T, class CS>
 __global__ void __launch_bounds__(256) k_box_trim(Geom g, const uint8_t* __restrict__ code,
                                                   const T* __restrict__ dg, const CS* __restrict__ cx,
                                                   const CS* __restrict__ cy, const CS* __restrict__ cz,
-                                                  T csx, T csy, T csz, T* rec, int ring) {
+                                                  T csx, T csy, T csz, T* rec) {
     pdl_entry();
     const int i0 = 1 + kBT * (int)blockIdx.x, j0 = 1 + kBT * (int)blockIdx.y,
               k0 = 1 + kBT * (int)blockIdx.z;
-    const int lo = ring, hi = kBT + ring - 1, nb = kBT + 2 * ring;
+    constexpr int lo = 2, hi = kBT + 1, nb = BBox<T>::N;
     const bool inside = i0 - lo >= 1 && j0 - lo >= 1 && k0 - lo >= 1 && i0 + hi <= g.nx &&
                         j0 + hi <= g.ny && k0 + hi <= g.nz;
     bool ok = inside;
