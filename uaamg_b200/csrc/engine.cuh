@@ -26,6 +26,7 @@
 #include "engine.h"
 #include "fused.cuh"
 #include "kernels.cuh"
+#include "quad.cuh"
 #include "tail.cuh"
 #include "tma.cuh"
 #include "vec.cuh"
@@ -725,10 +726,15 @@ private:
     }
     template <int DIM, bool FINE, class CSL, bool STAR>
     void pick_chunks_as(LevelBuf<T, CS>& L) const {
-        L.zc = pick_zc(L.g, resident(k_level_fused<DIM, T, FINE, CSL, false, false, STAR>,
-                                     FCfg<DIM, T, CSL, FINE, false, STAR>::BYTES), STAR ? 6 : 4);
-        L.zu = pick_zc(L.g, resident(k_level_fused<DIM, T, FINE, CSL, true, FINE, STAR>,
-                                     FCfg<DIM, T, CSL, FINE, true, STAR>::BYTES), 4);
+        if constexpr (FINE && STAR) {
+            L.zc = pick_zc(L.g, resident(k_level_quad<DIM, CSL, false, false>, QCfg<DIM, CSL, false>::BYTES), 6);
+            L.zu = pick_zc(L.g, resident(k_level_quad<DIM, CSL, true, true>, QCfg<DIM, CSL, true>::BYTES), 4);
+        } else {
+            L.zc = pick_zc(L.g, resident(k_level_fused<DIM, T, FINE, CSL, false, false, STAR>,
+                                         FCfg<DIM, T, CSL, FINE, false, STAR>::BYTES), STAR ? 6 : 4);
+            L.zu = pick_zc(L.g, resident(k_level_fused<DIM, T, FINE, CSL, true, FINE, STAR>,
+                                         FCfg<DIM, T, CSL, FINE, true, STAR>::BYTES), 4);
+        }
     }
     // Chunk lengths of level l's fused marches (the four-march kernels take the way down's)
     // and of the search direction.
@@ -804,7 +810,12 @@ private:
             (e = smem_attr(k_level_fused<DIM, T, FINE, CSL, true, true>,
                            FCfg<DIM, T, CSL, FINE, true>::BYTES)))
             return e;
-        if constexpr (sizeof(T) == 4) {
+        if constexpr (sizeof(T) == 4 && FINE) {
+            if ((e = smem_attr(k_level_quad<DIM, CSL, false, false>, QCfg<DIM, CSL, false>::BYTES)) ||
+                (e = smem_attr(k_level_quad<DIM, CSL, true, false>, QCfg<DIM, CSL, true>::BYTES)) ||
+                (e = smem_attr(k_level_quad<DIM, CSL, true, true>, QCfg<DIM, CSL, true>::BYTES)))
+                return e;
+        } else if constexpr (sizeof(T) == 4) {
             if ((e = smem_attr(k_level_fused<DIM, T, FINE, CSL, false, false, true>,
                                FCfg<DIM, T, CSL, FINE, false, true>::BYTES)) ||
                 (e = smem_attr(k_level_fused<DIM, T, FINE, CSL, true, false, true>,
@@ -1467,6 +1478,10 @@ private:
             UAAMG_LAUNCH_SMEM(tag, (k_level_box<T, FINE, CSL, false, false, STAR>), box_grid(L.g),
                               dim3(kThreads), (BPlan<T, CSL, FINE, false, STAR>::BYTES), bmaps(l, false),
                               mlevel(l), Cl.b, done, err_, partials_, cg_);
+        else if constexpr (FINE && STAR)
+            UAAMG_LAUNCH_SMEM(tag, (k_level_quad<DIM, CSL, false, false>), march_grid<DIM>(L.g, L.zc),
+                              dim3(kThreads), (QCfg<DIM, CSL, false>::BYTES), fmaps(l, false), mlevel(l),
+                              Cl.b, done, err_, partials_, cg_);
         else
             UAAMG_LAUNCH_SMEM(tag, (k_level_fused<DIM, T, FINE, CSL, false, false, STAR>),
                               march_grid<DIM>(L.g, L.zc), dim3(kThreads),
@@ -1485,6 +1500,10 @@ private:
         if (DIM == 3 && L.box)
             UAAMG_LAUNCH_SMEM(tag, (k_level_box<T, FINE, CSL, true, ZDOT, STAR>), box_grid(L.g),
                               dim3(kThreads), (BPlan<T, CSL, FINE, true, STAR>::BYTES), bmaps(l, true),
+                              mlevel(l, true), x, done, err_, partials_, cg_);
+        else if constexpr (FINE && STAR)
+            UAAMG_LAUNCH_SMEM(tag, (k_level_quad<DIM, CSL, true, ZDOT>), march_grid<DIM>(L.g, L.zu),
+                              dim3(kThreads), (QCfg<DIM, CSL, true>::BYTES), fmaps(l, true),
                               mlevel(l, true), x, done, err_, partials_, cg_);
         else
             UAAMG_LAUNCH_SMEM(tag, (k_level_fused<DIM, T, FINE, CSL, true, ZDOT, STAR>),
