@@ -1211,8 +1211,11 @@ private:
             const Geom& g = lv_[tail_lt_].g;
             const int n = dense_cells_;
             UAAMG_LAUNCH((KTag{K_SETUP, tail_lt_, 0.0}), k_tail_cells<DIM>, 1, 256, g, dense_cell_);
-            UAAMG_LAUNCH_SMEM((KTag{K_SETUP, tail_lt_, 0.0}), (k_tail<DIM, T>), n, tail_threads<T>(),
-                              tail_smem_, tail_args<DIM>(), (const int*)nullptr, dense_, dense_ld_);
+            // small blocks, five a SM, unless the coarsest level needs more threads (two cells
+            // each): the phases are latency-bound
+            const int nt = cells(lv_.back().g) <= 512.0 ? 256 : tail_threads<T>();
+            UAAMG_LAUNCH_SMEM((KTag{K_SETUP, tail_lt_, 0.0}), (k_tail<DIM, T>), n, nt, tail_smem_,
+                              tail_args<DIM>(), (const int*)nullptr, dense_, dense_ld_);
             dense_n_ = n;
         }
         return E_OK;

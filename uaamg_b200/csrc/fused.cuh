@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
             bool okk = true;
             if (tid == 0 && s + 2 <= R.plast) okk = R.wait(s + 2);
             if (!step_barrier(okk, err)) return false;
-            if (tid == 0) R.refill(M, s - C::LAG);
+            if (tid == kRefill) R.refill(M, s - C::LAG);
             return true;
         };
         using R0 = std::integral_constant<int, 0>;

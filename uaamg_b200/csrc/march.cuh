@@ -47,6 +47,10 @@ namespace {
 constexpr int kMX = 32, kMY = 16;                  // column tile
 constexpr int kThreads = 256;                      // one thread per x-pair of the tile
 constexpr int kHaloOdd = 2 * (kMX / 2 + 1) + kMY;  // odd cells of the 1-cell ring: 50
+// The thread that issues the next plane's loads after a step's barrier: of another warp
+// than thread 0's, which waits for a plane before it, since either delays its warp and
+// with it the next barrier (256^3, k_level_quad: an iteration 451 -> 440 us).
+constexpr int kRefill = kThreads - 32;
 
 __host__ __device__ constexpr size_t align128(size_t b) { return (b + 127) / 128 * 128; }
 
@@ -964,7 +968,7 @@ __global__ void __launch_bounds__(kThreads, DIRW ? 1 : PmvCfg<DIM, T>::MINB)
     }
     form(R.at(kb), pbuf0, pc, cc);
     __syncthreads();
-    if (DIM == 3 && tid == 0) {
+    if (DIM == 3 && tid == kRefill) {
         R.refill(M, kb - 1);
         R.refill(M, kb);
     }
@@ -1015,7 +1019,7 @@ __global__ void __launch_bounds__(kThreads, DIRW ? 1 : PmvCfg<DIM, T>::MINB)
         pbn = t;
         if (tid == 0 && k + 2 <= R.plast) ok = R.wait(k + 2);
         if (!step_barrier(ok, err)) return;
-        if (tid == 0) R.refill(M, k + 1);
+        if (tid == kRefill) R.refill(M, k + 1);
     }
     double tot[1];
     double rz_old = 0.0, breakdown = 0.0;
@@ -1123,7 +1127,7 @@ __global__ void __launch_bounds__(kThreads) k_resid_march(const __grid_constant_
     }
     form(R.at(kb), xbuf0, xc, bc, cc);
     __syncthreads();
-    if (tid == 0) {
+    if (tid == kRefill) {
         R.refill(M, kb - 1);
         R.refill(M, kb);
     }
@@ -1174,7 +1178,7 @@ __global__ void __launch_bounds__(kThreads) k_resid_march(const __grid_constant_
         xbn = t;
         if (tid == 0 && k + 2 <= R.plast) ok = R.wait(k + 2);
         if (!step_barrier(ok, err)) return;
-        if (tid == 0) R.refill(M, k + 1);
+        if (tid == kRefill) R.refill(M, k + 1);
     }
     double tot[1];
     if (reduce_last<1>(acc, partials, &cg->counter[slot], tot)) {

@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, DIM == 3 ? (UP ? 3 : 4) : 5)
             bool okk = true;
             if (tid == 0 && s + 2 <= RG.plast) okk = RG.wait(s + 2);
             if (!step_barrier(okk, err)) return false;
-            if (tid == 0) RG.refill(M, s + 1);
+            if (tid == kRefill) RG.refill(M, s + 1);
             st += P::STAGE;
             if (st == sm + C::OFF_RING + S * P::STAGE) st = sm + C::OFF_RING;
             return true;
