@@ -460,6 +460,7 @@ private:
     // wave: a second, partial wave left SMs idle at its end); UAAMG_PMV2D_PER_SM overrides
     int pmv2d_per_sm_ = 8;
     int pm_zc_ = 2;   // planes per block of the 3D search direction (k_pmatvec)
+    int zdot_zc_ = 2;  // FP64, 3D: of the z sums' partition (k_zdot_tiles)
     int rx_zc_ = 16;  // planes per block of the 3D replacement march (k_resid_march)
     int pmv2d_env_ = 0;
     int resid_per_sm_ = 8;  // the FP64 residual walk: resident blocks per SM (one wave)
@@ -604,7 +605,7 @@ private:
         const Geom& g = lv_[0].g;
         std::vector<double> v = {(double)dim_, (double)g.nx, (double)g.ny, (double)g.nz, dx_, dy_, dz_,
                                  (double)dirichlet_, (double)(uintptr_t)arena_, (double)arena_used_,
-                                 (double)pm_zc_, (double)rx_zc_, (double)pmv2d_per_sm_,
+                                 (double)pm_zc_, (double)zdot_zc_, (double)rx_zc_, (double)pmv2d_per_sm_,
                                  (double)resid_per_sm_, (double)tail_lt_, (double)tail_nc_,
                                  (double)dense_n_};
         for (const auto& L : lv_) {
@@ -747,14 +748,14 @@ private:
             else pick_chunks_as<DIM, false, CS, STAR>(L);
         }
         if constexpr (sizeof(T) == 8) {
-            // The FP64 form's dot products are summed per block of these two kernels; their
+            // The FP64 form's dot products are summed per block (search direction, z sums); their
             // partition stays (chunks halved from 16 planes until every SM has four blocks):
             // 256^3 on another one stops after 81 iterations instead of the reference's 82.
             const Geom& g = lv_[0].g;
             const long long tiles = (long long)((g.nx + kMX - 1) / kMX) * ((g.ny + kMY - 1) / kMY);
             int zc = 16;
             while (zc > 2 && tiles * ((g.nz + zc - 1) / zc) < 4LL * num_sms_) zc /= 2;
-            lv_[0].zu = pm_zc_ = zc;
+            zdot_zc_ = pm_zc_ = zc;
             return;
         }
         pm_zc_ = pick_zc(lv_[0].g, dirichlet_ ? resident(k_pmatvec<DIM, T, true>, PmvCfg<DIM, T>::BYTES)
@@ -1571,6 +1572,15 @@ private:
                 if (star_) {
                     if (zd) up_fused<DIM, FINE, CSL, true, true>(l, done);
                     else up_fused<DIM, FINE, CSL, false, true>(l, done);
+                    return;
+                }
+            }
+            if constexpr (DIM == 3 && sizeof(T) == 8) {
+                if (zd && !L.box) {
+                    up_fused<DIM, FINE, CSL, false, false>(l, done);
+                    UAAMG_LAUNCH((KTag{K_ZDOT, 0, c * (2.0 * t + 1.0)}), (k_zdot_tiles<T>),
+                                 march_grid<DIM>(L.g, zdot_zc_), dim3(256), L.g, zdot_zc_, L.code, r_, z_,
+                                 partials_, cg_);
                     return;
                 }
             }

@@ -845,6 +845,56 @@ __device__ __forceinline__ void finish_zdot(CGState* cg, const ZdotIn& in, const
     if (!(rz == rz)) { cg->status = CG_NAN; cg->done = 1; }
 }
 
+// The same sums with a z march's partition and order: block (bx, by, bz) sums the tile
+// 32 x 16 and zc planes of a march, thread (lane, w) its pair (i, j), (i, j + 1), per plane
+// the odd cell first.  The FP64 form's way up takes longer chunks than its dot products'
+// partition allows (engine.cuh, pick_chunks), so they are summed here, in the same order:
+// 96^3 FP64, the way up in chunks of 2 planes with the sums took 30.8 us, and the solve
+// 7.5 ms (now 7.0, with the coarsest level's shorter divisions, tail.cuh).
+template <class T>
+__global__ void __launch_bounds__(256) k_zdot_tiles(Geom g, int zc, const uint8_t* __restrict__ code,
+                                                    const T* __restrict__ r, const T* __restrict__ z,
+                                                    double* partials, CGState* cg) {
+    pdl_wait();
+    const int stop = ld_now(&cg->done);
+    pdl_launch();
+    if (stop) return;
+    double acc[3] = {0.0, 0.0, 0.0};
+    const int i = 1 + 32 * (int)blockIdx.x + (int)(threadIdx.x & 31);
+    const int j = 1 + 16 * (int)blockIdx.y + 2 * (int)(threadIdx.x >> 5);
+    const int kb = 1 + (int)blockIdx.z * zc, ke = min(kb + zc, g.nz + 1);
+    if (i <= g.nx) {
+#pragma unroll 2
+        for (int k = kb; k < ke; ++k) {
+            const int first = ((i + j + k) & 1) ? 0 : 1;  // the pair's odd cell
+            const int id = cidx(g, i, j, k);
+            uint32_t c[2];
+            double zv[2], rv[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const bool in = j + e <= g.ny;
+                c[e] = in ? code[id + e * g.sx] : 0u;
+                zv[e] = in ? (double)z[id + e * g.sx] : 0.0;
+                rv[e] = in ? (double)r[id + e * g.sx] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool b = (first ^ u) != 0;  // the second cell of the pair
+                if ((b ? c[1] : c[0]) & kActive) {
+                    const double zz = b ? zv[1] : zv[0], rr = b ? rv[1] : rv[0];
+                    acc[0] += zz;
+                    acc[1] += rr * zz;
+                    acc[2] += rr;
+                }
+            }
+        }
+    }
+    double tot[3];
+    ZdotIn in;
+    if (reduce_last<3>(acc, partials, &cg->counter[2], tot, [&] { in.load(cg); }))
+        finish_zdot(cg, in, tot);
+}
+
 // The sums above as a separate pass (used with the per-level sweep V-cycle; the
 // fused V-cycle computes them in its last kernel).
 template <int DIM, class T>

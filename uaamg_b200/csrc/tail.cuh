@@ -329,6 +329,19 @@ __device__ __forceinline__ void tail_warps_sync(int nw) {
     else asm volatile("bar.sync 1, %0;" ::"r"(nw * 32) : "memory");
 }
 
+// a / d, correctly rounded, from y = 1/d correctly rounded (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990: one corrected step of
+// a quotient within an ulp): the coarsest solve divides by the same d forty times, each
+// on the chain of the one before.  Outside the range where the correction is exact the
+// division itself.
+__device__ __forceinline__ double tail_div(double a, double d, double y) {
+    const double m = fabs(a);
+    if (!(m > 1e-250 && m < 1e250)) return a / d;
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, d, a), y, q);
+}
+__device__ __forceinline__ float tail_div(float a, float d, float) { return a / d; }
+
 // Coarsest level: 10 x (forward + reverse) sweeps from x = 0 (x zeroed by the
 // caller) by the first ceil(n / 64) warps, two cells a thread held in registers.
 template <int DIM, class T>
@@ -339,7 +352,7 @@ __device__ void tail_coarsest(const TailView<DIM, T>& V) {
     if ((int)threadIdx.x >= nw * 32) return;
     const int nthr = nw * 32;
     int sd2[2] = {-1, -1}, par2[2] = {0, 0};
-    T d2[2] = {T(1), T(1)}, c2[2][6];
+    T d2[2] = {T(1), T(1)}, y2[2] = {T(1), T(1)}, b2[2] = {T(0), T(0)}, c2[2][6];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         const int c = threadIdx.x + s * nthr;
@@ -355,6 +368,8 @@ __device__ void tail_coarsest(const TailView<DIM, T>& V) {
                 sd2[s] = V.sid(i, j, k);
                 par2[s] = (i + j + k) & 1;
                 d2[s] = d;
+                y2[s] = T(1) / d;
+                b2[s] = V.b[sd2[s]];
                 tail_coup<DIM>(V.L, id, c2[s]);
             }
         }
@@ -370,7 +385,7 @@ __device__ void tail_coarsest(const TailView<DIM, T>& V) {
                     const T nb = tail_nb<DIM, T>(c2[s], x[sd + 1], x[sd - 1], x[sd + sx], x[sd - sx],
                                                  DIM == 3 ? x[sd + sxy] : T(0),
                                                  DIM == 3 ? x[sd - sxy] : T(0));
-                    x[sd] = (V.b[sd] + nb) / d2[s];
+                    x[sd] = tail_div(b2[s] + nb, d2[s], y2[s]);
                 }
             }
             tail_warps_sync(nw);
