@@ -67,3 +67,31 @@ def test_few_iterations_next_to_solids_and_on_odd_sizes(handle):
     assert st.iterations <= 20
     st64 = handle.solve(rhs, np.zeros_like(rhs), handle.options("fp64", 1e-6, 200, "rel"), strict=True)
     assert st64.iterations > st.iterations
+
+
+def test_inconsistent_chambers_fall_back(handle):
+    """Two chambers with a net source each: no solution exists, the covering aggregates
+    join the chambers on coarse levels, CG's residual grows and the solve is repeated on
+    the reference's hierarchy.  It ends unconverged and finite, alone and in a batch the
+    same, and a consistent right-hand side on the same mask converges before and after."""
+    n, m = 90, 70
+    solid = np.zeros((m + 2, n + 2), np.uint8)
+    solid[:, 45] = 1
+    rng = np.random.default_rng(3)
+    b = np.zeros(solid.shape)
+    fl = fluid_interior(solid)
+    b[fl] = rng.standard_normal(int(fl.sum()))
+    b[fl] -= b[fl].mean()
+    c = b.copy()
+    for sl in (slice(1, 45), slice(46, n + 1)):
+        c[1:-1, sl] -= c[1:-1, sl].mean()
+    opts = handle.options("mixed", 1e-6, 100, "rel")
+    handle.set_problem(solid, 1.0, 1.0)
+    pc = [np.zeros_like(b) for _ in range(2)]
+    assert handle.solve(c, pc[0], opts).status == 0
+    p, q = np.zeros_like(b), np.zeros_like(b)
+    st = handle.solve(b, p, opts)
+    assert st.status == 1 and st.iterations == 100 and np.isfinite(p).all()
+    sb = handle.solve_batch([(solid, b, q, 1.0, 1.0, 1.0)], opts)[0]
+    assert sb.status == 1 and sb.iterations == 100 and np.array_equal(p, q)
+    assert handle.solve(c, pc[1], opts).status == 0 and np.array_equal(*pc)

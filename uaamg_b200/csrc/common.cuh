@@ -54,6 +54,7 @@ enum : int {
     CG_MAXITER = 2,
     CG_BREAKDOWN = 3,
     CG_NAN = 4,
+    CG_DIVERGED = 5,  // covering aggregates only: the solve is repeated on the reference's
 };
 
 // Device-resident PCG state.  All scalars are FP64; the loop never copies a
@@ -86,18 +87,29 @@ struct CGState {
     unsigned int counter[8];  // last-block counters, one per reduction site
     int err;           // set by a kernel whose TMA wait gave up
     int epoch;         // number of this solve (its progress words carry it)
+    int cover;         // 1: covering aggregates; a residual that grew ends the solve
     unsigned long long* progress;  // pinned host word: where the solve is (publish)
 };
 
-// A solve's progress word in pinned host memory: epoch, completed updates, stopped.  The
+// A solve's progress word in pinned host memory: epoch, completed updates, status.  The
 // host reads it instead of queueing a copy of the stop flag and an event behind every
 // step (two stream operations a step, and a gap before the next step).
-__host__ __device__ inline unsigned long long progress_word(int epoch, int iter, int done) {
-    return ((unsigned long long)(epoch & 0xffff) << 48) | ((unsigned long long)(unsigned)iter << 1) |
-           (done ? 1u : 0u);
+__host__ __device__ inline unsigned long long progress_word(int epoch, int iter, int status) {
+    return ((unsigned long long)(epoch & 0xffff) << 48) | ((unsigned long long)(unsigned)iter << 3) |
+           (unsigned)(status & 7);
 }
-__device__ __forceinline__ void publish(unsigned long long* to, int epoch, int iter, int done) {
-    if (to) *(volatile unsigned long long*)to = progress_word(epoch, iter, done);
+__device__ __forceinline__ void publish(unsigned long long* to, int epoch, int iter, int status) {
+    if (to) *(volatile unsigned long long*)to = progress_word(epoch, iter, status);
+}
+
+// Whether a residual (squared norm rr) has grown `times` (squared) over where the solve
+// began, or over a thousandth of ||b|| when it began below that.  A right-hand side that
+// is inconsistent on separate parts of the fluid (a chamber with a net source) has no
+// solution; the covering aggregates join such parts on coarse levels and CG then runs
+// away instead of stalling at the inconsistency.
+__device__ __forceinline__ bool residual_grew(double rr, double r0, double bnorm, double times) {
+    const double f = fmax(r0, 1e-3 * bnorm);
+    return rr > times * f * f;
 }
 
 // q = a / d and r = a % d for 0 <= a < 2^31, 0 < d, from a reciprocal 1/d computed

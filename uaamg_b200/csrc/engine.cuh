@@ -18,6 +18,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <new>
 #include <tuple>
 #include <type_traits>
 #include <utility>
@@ -148,6 +149,7 @@ public:
         trim_ = !(nt && nt[0] == '1');
     }
     ~EngineT() override {
+        delete fb_;
         release();
         if (cap_) cudaStreamDestroy(cap_);
     }
@@ -158,6 +160,9 @@ public:
     // same addresses and sizes.
     int set_problem(int dim, int nx, int ny, int nz, double dx, double dy, double dz,
                     const uint8_t* d_solid, int dirichlet) override {
+        delete fb_;
+        fb_ = nullptr;
+        fb_on_ = false;
         release(true);
         if (dim != 2 && dim != 3) { release(); return E_ARG; }
         if (nx < 2 || ny < 2 || (dim == 3 && nz < 2)) { release(); return E_ARG; }
@@ -185,10 +190,12 @@ public:
     int solve_begin(const SolveArgs& a) override {
         if (lv_.empty() || apply_only_) return E_NOPROB;
         launches_ = 0;
+        fb_on_ = false;
         return dim_ == 3 ? begin_impl<3>(a) : begin_impl<2>(a);
     }
 
     int solve_step() override {
+        if (fb_on_) return fb_->solve_step();
         if (stopped_) return E_OK;
         return dim_ == 3 ? step_impl<3>() : step_impl<2>();
     }
@@ -198,11 +205,16 @@ public:
     // asked too: a failed launch ends in E_CUDA, and steps that ran without advancing the
     // word (a kernel gave up on its loads) count as seen, so that max_iter ends the solve.
     int solve_poll(bool wait, bool* stopped) override {
+        if (fb_on_) return fb_->solve_poll(wait, stopped);
         while (!stopped_ && seen_ < nstep_) {
             const unsigned long long w = *(volatile unsigned long long*)flag_host_;
             if ((w >> 48) == (unsigned long long)(epoch_ & 0xffff)) {
-                if (w & 1) { stopped_ = true; break; }
-                if ((long long)((w & 0xffffffffffffull) >> 1) >= 2LL * (seen_ + 1)) { ++seen_; continue; }
+                if (w & 7) {
+                    stopped_ = true;
+                    if ((w & 7) == CG_DIVERGED) return fall_back(stopped);
+                    break;
+                }
+                if ((long long)((w & 0xffffffffffffull) >> 3) >= 2LL * (seen_ + 1)) { ++seen_; continue; }
             }
             if ((++polls_ & 0xffff) == 0) {
                 const cudaError_t q = cudaStreamQuery(st_);
@@ -220,14 +232,17 @@ public:
     }
 
     // Steps queued but not yet seen by solve_poll (at most two are useful).
-    int solve_inflight() const override { return nstep_ - seen_; }
+    int solve_inflight() const override { return fb_on_ ? fb_->solve_inflight() : nstep_ - seen_; }
 
     int solve_end(SolveResult* res) override {
         int e = solve_end_enqueue();
         return e != E_OK ? e : solve_end_collect(res);
     }
 
-    int solve_end_enqueue() override { return dim_ == 3 ? end_enqueue<3>() : end_enqueue<2>(); }
+    int solve_end_enqueue() override {
+        if (fb_on_) return fb_->solve_end_enqueue();
+        return dim_ == 3 ? end_enqueue<3>() : end_enqueue<2>();
+    }
 
     int enqueue_step(cudaStream_t s, int* flag_dst) override {
         if (lv_.empty()) return E_NOPROB;
@@ -246,6 +261,11 @@ public:
     }
 
     int solve_end_collect(SolveResult* res) override {
+        if (fb_on_) {
+            const int e = fb_->solve_end_collect(res);
+            cuda_error = fb_->cuda_error;
+            return e;
+        }
         int e = sync_check();
         if (e != E_OK) return e;
         const CGState& c = *cg_host_;
@@ -269,8 +289,7 @@ public:
         bool stopped = false;
         while (!stopped) {
             if ((e = solve_step()) != E_OK) return e;
-            if ((e = solve_poll(solve_inflight() >= 2 || it_ >= cur_.max_iter, &stopped)) != E_OK)
-                return e;
+            if ((e = solve_poll(solve_inflight() >= 2 || queued_all(), &stopped)) != E_OK) return e;
         }
         return solve_end(res);
     }
@@ -333,8 +352,8 @@ public:
     }
 
     void set_stream(cudaStream_t s) override { st_ = s; }
-    size_t device_bytes() const override { return bytes_; }
-    long launches() const override { return launches_; }
+    size_t device_bytes() const override { return bytes_ + (fb_ ? fb_->device_bytes() : 0); }
+    long launches() const override { return launches_ + (fb_on_ ? fb_->launches() : 0); }
     void set_vcycle_sweeps(bool on) override { sweeps_ = on; }
     void set_graphs(bool on) override { graphs_ = on; }
     void set_autotune(bool on) override { autotune_ = on; }
@@ -404,6 +423,7 @@ public:
     }
 
     int timed_out() override {
+        if (fb_on_) return fb_->timed_out();
         int v = 0;
         if (!err_) return 0;
         if (err_known_) return cg_host_->err;  // a finished solve: copied with its state
@@ -412,6 +432,45 @@ public:
     }
 
 private:
+    bool queued_all() const { return fb_on_ ? fb_->queued_all() : it_ >= cur_.max_iter; }
+
+    // The residual of a solve on covering aggregates grew (common.cuh, residual_grew): the
+    // same solve from its beginning on the reference's hierarchy, by an engine of its own
+    // (made here, kept while the mask stays); the stages then go to it.  Nothing has been
+    // added to the caller's x yet.
+    int fall_back(bool* stopped) {
+        *stopped = true;
+        if (!cur_.ref_solid) return E_OK;
+        if (!fb_) {
+            fb_ = new (std::nothrow) EngineT<T, CS>(mixed_);
+            if (!fb_) return E_OK;
+            fb_->st_ = st_;
+            fb_->sweeps_ = sweeps_;
+            fb_->tail_on_ = tail_on_;
+            fb_->fused_ = fused_;
+            fb_->graphs_ = graphs_;
+            fb_->nu_fine_ = nu_fine_;
+            fb_->nu_coarse_ = nu_coarse_;
+            const Geom& g = lv_[0].g;
+            if (fb_->set_problem(dim_, g.nx, g.ny, g.nz, dx_, dy_, dz_, cur_.ref_solid, dirichlet_) != E_OK) {
+                delete fb_;  // no room for it: the diverged result stands
+                fb_ = nullptr;
+                return E_OK;
+            }
+        }
+        fb_->st_ = st_;
+        fb_->set_operator(vd_, vox_, voy_, vsx_, vver_);
+        fb_->set_smoothing(nu_fine_, nu_coarse_);
+        fb_->prof_on_ = false;
+        const int e = fb_->solve_begin(cur_);
+        if (e != E_OK) return e;
+        fb_on_ = true;
+        *stopped = false;
+        return E_OK;
+    }
+
+    EngineT<T, CS>* fb_ = nullptr;
+    bool fb_on_ = false;
     bool mixed_;
     bool cover_ = false, apply_only_ = false;
     bool star_ = false;  // the current hierarchy covers and its transfers reach face neighbours
@@ -1800,6 +1859,7 @@ private:
         init.init = 1;
         init.epoch = ++epoch_;
         init.progress = flag_host_;
+        init.cover = star_ ? 1 : 0;
         *flag_host_ = progress_word(epoch_, 0, 0);
         *cg_host_ = init;
         if (cudaMemcpyAsync(cg_, cg_host_, sizeof(CGState), cudaMemcpyHostToDevice, st_) != cudaSuccess)

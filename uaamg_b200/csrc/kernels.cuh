@@ -477,7 +477,12 @@ __device__ __forceinline__ void true_residual_done(CGState* cg, double rr, int m
             cg->cand = 0;
             if (sqrt(rr) < cg->tol_abs) { cg->status = CG_CONVERGED; cg->done = 1; }
         }
-        if (!(rr == rr)) { cg->status = CG_NAN; cg->done = 1; }
+        if (!(rr == rr)) { cg->status = cg->cover ? CG_DIVERGED : CG_NAN; cg->done = 1; }
+        else if (!cg->done && cg->cover &&
+                 residual_grew(rr, cg->r0, cg->bnorm, cg->iter >= cg->max_iter ? 1.0 : 1e4)) {
+            cg->status = CG_DIVERGED;
+            cg->done = 1;
+        }
     }
 }
 
@@ -669,7 +674,7 @@ __global__ void __launch_bounds__(256) k_resid_x64(Geom g, const uint8_t* __rest
             cg->status = CG_MAXITER;
             cg->done = 1;
         }
-        if (mode == 1) publish(cg->progress, cg->epoch, cg->iter, cg->done);
+        if (mode == 1) publish(cg->progress, cg->epoch, cg->iter, cg->status);
     }
 }
 

@@ -1193,7 +1193,7 @@ __global__ void __launch_bounds__(kThreads) k_resid_march(const __grid_constant_
             cg->status = CG_MAXITER;
             cg->done = 1;
         }
-        publish(cg->progress, cg->epoch, cg->iter, cg->done);
+        publish(cg->progress, cg->epoch, cg->iter, cg->status);
     }
 }
 

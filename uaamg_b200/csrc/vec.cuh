@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
         }
     pdl_launch();
     if (stop) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) publish(cg->progress, cg->epoch, cg->iter, 1);
+        if (blockIdx.x == 0 && threadIdx.x == 0) publish(cg->progress, cg->epoch, cg->iter, cg->status);
         return;
     }
     const bool fold = fold_now != 0;
@@ -153,8 +153,8 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
         }
     }
     double tot[1];
-    double tol_abs = 0.0, first = 0.0;
-    int it = 0, every = 0, max_iter = 0, cand = 0, epoch = 0;
+    double tol_abs = 0.0, first = 0.0, bnorm = 0.0;
+    int it = 0, every = 0, max_iter = 0, cand = 0, epoch = 0, cover = 0;
     unsigned long long* progress = nullptr;
     if (reduce_last<1>(acc, partials, &cg->counter[1], tot, [&] {
             tol_abs = ld_now(&cg->tol_abs);
@@ -163,6 +163,8 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             every = ld_now(&cg->replace_every);
             max_iter = ld_now(&cg->max_iter);
             cand = ld_now(&cg->cand);
+            cover = ld_now(&cg->cover);
+            bnorm = ld_now(&cg->bnorm);
             epoch = ld_now(&cg->epoch);
             progress = ld_now(&cg->progress);
         })) {
@@ -181,8 +183,11 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             else status = CG_CONVERGED;
         } else if (it >= max_iter && every == 0) status = CG_MAXITER;
         if (every > 0 && status == CG_RUNNING && it >= max_iter && !cand) status = CG_MAXITER;
+        if (cover && ((status == CG_MAXITER && residual_grew(rr, first, bnorm, 1.0)) || status == CG_NAN ||
+                      (status == CG_RUNNING && residual_grew(rr, first, bnorm, 1e6))))
+            status = CG_DIVERGED;
         if (status != CG_RUNNING) { cg->status = status; cg->done = 1; }
-        publish(progress, epoch, it, status != CG_RUNNING);
+        publish(progress, epoch, it, status);
     }
 }
 
