@@ -109,8 +109,11 @@ UAAMG_API uaamg_status uaamg_set_stream(uaamg_handle* h, void* stream);
  * FP64 solves, and every V-cycle applied by itself (uaamg_precond_apply) or level
  * inspected, use the reference's hierarchy.  FP32 and mixed solves precondition with
  * the same Galerkin sums over aggregates that cover every fluid cell (a coarse cell is
- * fluid when any child is, odd sizes round up), which needs far fewer iterations next
- * to solids and on odd sizes; with Dirichlet walls they use the reference's. */
+ * fluid when any child is, odd sizes round up) and transfers that reach the coarse face
+ * neighbours, which needs far fewer iterations next to solids and on odd sizes; with
+ * Dirichlet walls they use the reference's.  A solve whose residual grows on that
+ * hierarchy (a right-hand side inconsistent on separate parts of the fluid) is repeated
+ * on the reference's; grouped batches (uaamg_set_batch_group) do not repeat it. */
 UAAMG_API uaamg_status uaamg_set_problem_2d(uaamg_handle* h, int nx, int ny, double dx, double dy,
                                   const uint8_t* solid);
 UAAMG_API uaamg_status uaamg_set_problem_3d(uaamg_handle* h, int nx, int ny, int nz, double dx,
@@ -230,7 +233,8 @@ UAAMG_API uaamg_status uaamg_copy_level(uaamg_handle* h, int precision, int l, u
  * 2-cell ring are interior fluid with one diagonal and one coupling per axis, which
  * the box kernels run without loading diagonals, couplings or codes (the reference's
  * tile trimming, cuda_uaamg_preconditioner_3d.cu:81-99 and :357-375; results are
- * identical either way).  UAAMG_NO_TRIM=1 in the environment turns trimming off for
+ * identical either way).  It describes the reference's hierarchy; the FP32 and mixed
+ * solves' own hierarchy is not trimmed.  UAAMG_NO_TRIM=1 in the environment turns trimming off for
  * engines created afterwards. */
 UAAMG_API uaamg_status uaamg_level_trim(uaamg_handle* h, int precision, int l, int* boxes,
                                         int* trimmed);
