@@ -113,7 +113,7 @@ UAAMG_API uaamg_status uaamg_set_stream(uaamg_handle* h, void* stream);
  * neighbours, which needs far fewer iterations next to solids and on odd sizes; with
  * Dirichlet walls they use the reference's.  A solve whose residual grows on that
  * hierarchy (a right-hand side inconsistent on separate parts of the fluid) is repeated
- * on the reference's; grouped batches (uaamg_set_batch_group) do not repeat it. */
+ * on the reference's. */
 UAAMG_API uaamg_status uaamg_set_problem_2d(uaamg_handle* h, int nx, int ny, double dx, double dy,
                                   const uint8_t* solid);
 UAAMG_API uaamg_status uaamg_set_problem_3d(uaamg_handle* h, int nx, int ny, int nz, double dx,

@@ -95,3 +95,33 @@ def test_inconsistent_chambers_fall_back(handle):
     sb = handle.solve_batch([(solid, b, q, 1.0, 1.0, 1.0)], opts)[0]
     assert sb.status == 1 and sb.iterations == 100 and np.array_equal(p, q)
     assert handle.solve(c, pc[1], opts).status == 0 and np.array_equal(*pc)
+
+
+@pytest.mark.parametrize("members", [2, 5])
+def test_inconsistent_member_of_a_group_falls_back(handle, members):
+    """In a grouped batch (one graph a step) the inconsistent member, repeated by itself
+    after the group, ends as the same problem solved alone; the others converge."""
+    n, m = 90, 70
+    solid = np.zeros((m + 2, n + 2), np.uint8)
+    solid[:, 45] = 1
+    fl = fluid_interior(solid)
+    rng = np.random.default_rng(4)
+    b = np.zeros(solid.shape)
+    b[fl] = rng.standard_normal(int(fl.sum()))
+    c = b.copy()
+    b[fl] -= b[fl].mean()
+    for sl in (slice(1, 45), slice(46, n + 1)):
+        c[1:-1, sl] -= c[1:-1, sl].mean()
+    opts = handle.options("mixed", 1e-6, 60, "rel")
+    handle.set_problem(solid, 1.0, 1.0)
+    alone = np.zeros_like(b)
+    ref = handle.solve(b, alone, opts)
+    ps = [np.zeros_like(b) for _ in range(members)]
+    handle.set_batch_group(1 << 20)
+    try:
+        st = handle.solve_batch([(solid, b if k == 1 else c, ps[k], 1.0, 1.0, 1.0) for k in range(members)], opts)
+    finally:
+        handle.set_batch_group(0)
+    assert st[1].status == ref.status == 1 and st[1].iterations == ref.iterations
+    assert np.array_equal(ps[1], alone)
+    assert all(st[k].status == 0 for k in range(members) if k != 1)

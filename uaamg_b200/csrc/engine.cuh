@@ -260,6 +260,13 @@ public:
         return E_OK;
     }
 
+    int steps_done(bool* stopped) override {
+        const unsigned long long w = *(volatile unsigned long long*)flag_host_;
+        *stopped = true;
+        if ((w >> 48) != (unsigned long long)(epoch_ & 0xffff) || (w & 7) != CG_DIVERGED) return E_OK;
+        return fall_back(stopped);
+    }
+
     int solve_end_collect(SolveResult* res) override {
         if (fb_on_) {
             const int e = fb_->solve_end_collect(res);

@@ -85,6 +85,10 @@ public:
     // For capturing the steps of many engines into one CUDA graph (batches); the
     // engine's own step bookkeeping (solve_step / solve_poll) is not used then.
     virtual int enqueue_step(cudaStream_t s, int* flag_dst) = 0;
+    // Once the steps queued so are done and the engine's stream follows them: *stopped is
+    // false when the solve goes on by solve_step / solve_poll (a residual that grew, see
+    // residual_grew in common.cuh).
+    virtual int steps_done(bool* stopped) = 0;
     virtual int solve_end_collect(SolveResult* res) = 0;
     virtual int nlevels() const = 0;
     virtual void level_dims(int l, int* nx, int* ny, int* nz) const = 0;

@@ -409,7 +409,9 @@ uaamg_status uaamg_solve_batch(uaamg_handle* h, int n, const uaamg_problem* prob
             bool stopped = false;
             int e = E_OK;
             if (grouped[i]) {
-                stopped = group_joined;
+                if (!group_joined) continue;
+                e = d.eng->steps_done(&stopped);
+                grouped[i] = 0;  // a solve that starts again goes on by itself
             } else {
                 e = d.eng->solve_step();
                 if (e == E_OK) e = d.eng->solve_poll(false, &stopped);
