@@ -87,7 +87,7 @@ struct CGState {
     unsigned int counter[8];  // last-block counters, one per reduction site
     int err;           // set by a kernel whose TMA wait gave up
     int epoch;         // number of this solve (its progress words carry it)
-    int cover;         // 1: covering aggregates; a residual that grew ends the solve
+    int cover;         // 1: preconditioned on covering aggregates; a residual that grew ends the solve
     unsigned long long* progress;  // pinned host word: where the solve is (publish)
 };
 

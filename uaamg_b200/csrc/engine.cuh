@@ -1866,7 +1866,7 @@ private:
         init.init = 1;
         init.epoch = ++epoch_;
         init.progress = flag_host_;
-        init.cover = star_ ? 1 : 0;
+        init.cover = star_ && a.precond ? 1 : 0;  // (plain CG applies no hierarchy)
         *flag_host_ = progress_word(epoch_, 0, 0);
         *cg_host_ = init;
         if (cudaMemcpyAsync(cg_, cg_host_, sizeof(CGState), cudaMemcpyHostToDevice, st_) != cudaSuccess)
