@@ -41,3 +41,42 @@ def test_plain_cg_is_never_repeated(handle, precision):
         assert st.status == 1 and st.iterations == max_iter
         assert handle.device_bytes() == held
     assert grew  # the case is one where it happens
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp32"])
+@pytest.mark.parametrize("shape", [(200, 60), (40, 30, 30)])
+def test_consistent_solves_cut_off_early_are_not_repeated(handle, shape, precision):
+    """A consistent right-hand side and a max_iter of one to four iterations: the residual may
+    lie above the first one, and the solve ends there."""
+    solid, b = _smooth(shape, 1)
+    handle.set_problem(solid, 1.0, 1.0, 1.0)
+    handle.solve(b, np.zeros_like(b), handle.options(precision, 0.9, 9, "rel"), strict=True)
+    held, grew = handle.device_bytes(), False
+    for max_iter in (1, 2, 3, 4):
+        st = handle.solve(b, np.zeros_like(b), handle.options(precision, 1e-12, max_iter, "rel"))
+        hist = handle.residual_history(max_iter + 1)
+        grew |= hist[max_iter] > hist[0]
+        assert st.status == 1 and st.iterations == max_iter
+        assert handle.device_bytes() == held
+    assert grew
+
+
+@pytest.mark.parametrize("shape", [(20000, 6), (8, 30000), (5, 5, 20000)])
+def test_consistent_channels_are_not_repeated(handle, shape):
+    """Long channels with a smooth right-hand side: the residual rises several thousand times
+    before it falls, and the solve goes on where it is."""
+    padded = tuple(n + 2 for n in shape[::-1])
+    solid = np.zeros(padded, np.uint8)
+    ax = int(np.argmax(padded))
+    v = np.linspace(0, 1, padded[ax]).reshape([-1 if a == ax else 1 for a in range(len(padded))])
+    fl = fluid_interior(solid)
+    b = np.where(fl, np.cos(np.pi * v), 0.0)
+    b[fl] -= b[fl].mean()
+    handle.set_problem(solid, 1.0, 1.0, 1.0)
+    rough = np.where(fl, np.random.default_rng(2).standard_normal(padded), 0.0)
+    handle.solve(rough, np.zeros_like(b), handle.options("mixed", 0.9, 60, "rel"), strict=True)
+    held = handle.device_bytes()
+    handle.solve(b, np.zeros_like(b), handle.options("mixed", 1e-4, 60, "rel"))
+    hist = handle.residual_history(61)
+    assert hist.max() > 1e3 * hist[0]
+    assert handle.device_bytes() == held

@@ -479,7 +479,7 @@ __device__ __forceinline__ void true_residual_done(CGState* cg, double rr, int m
         }
         if (!(rr == rr)) { cg->status = cg->cover ? CG_DIVERGED : CG_NAN; cg->done = 1; }
         else if (!cg->done && cg->cover &&
-                 residual_grew(rr, cg->r0, cg->bnorm, cg->iter >= cg->max_iter ? 1.0 : 1e4)) {
+                 residual_grew(rr, cg->rr_peak, cg->r0, cg->bnorm, cg->iter, cg->iter >= cg->max_iter)) {
             cg->status = CG_DIVERGED;
             cg->done = 1;
         }
