@@ -74,7 +74,8 @@ struct CGState {
                        // projection; sum0 also of the result's mean projection
     double bnorm;      // ||b|| of the normalised right-hand side
     double breakdown;  // p.Ap below this stops the solve (the reference's 1e-15)
-    double rr_peak;    // the largest rr of the solve's iterations
+    double rr_best;    // the least rr of the solve's iterations
+    double rz0, rz_peak;  // rz_old of its first one, the largest rz_old so far
     int done;          // 1 once the solve stopped; every loop kernel then returns at once
     int status;        // CG_* above
     int iter;          // completed x/r updates
@@ -103,20 +104,29 @@ __device__ __forceinline__ void publish(unsigned long long* to, int epoch, int i
     if (to) *(volatile unsigned long long*)to = progress_word(epoch, iter, status);
 }
 
-// Whether the residual (squared norm rr, the largest so far peak) of iteration it shows
-// that a solve on covering aggregates runs away.  A right-hand side that is inconsistent on
+// Whether the residual of iteration it shows that a solve on covering aggregates runs away
+// (squared norms: rr, the least so far best; rz, the preconditioner's norm r.Mr one
+// iteration before, its first value rz0 and the largest so far).  A right-hand side that is inconsistent on
 // separate parts of the fluid (a chamber with a net source) has no solution; the covering
 // aggregates join such parts on coarse levels, and CG then runs away instead of stalling
 // at the inconsistency: 1e6 times where it began (or a thousandth of ||b|| when it began
 // below that) within 8 to 15 iterations.  A consistent solve also rises first when its
 // right-hand side is smooth, since the 2-norm weighs the rough error that the coarse
 // levels bring in: 130 times at 2048 x 1024 with scattered solids, 420 at 2000 x 6, 9400
-// at 60000 x 8, from the second iteration on falling again.  At max_iter (last) a smaller
-// growth will do, from the fifth iteration on and while it has not fallen again.
-__device__ __forceinline__ bool residual_grew(double rr, double peak, double r0, double bnorm, int it,
-                                              bool last) {
+// at 60000 x 8, falling again from the second iteration on.  Its rz does not rise, but in
+// channels some 25 times as long as wide, and there falls again too; that of an inconsistent
+// one rises on from the third iteration, which is what counts when max_iter ends a solve
+// (last).
+// With a small inconsistent share of b the residual falls to it first and rises from there
+// (share 1e-4: to 1e-3 in 6 iterations, past 1 in 15).  Once it has been below half of r0,
+// 1000 times the best ends the solve, three times at max_iter; consistent solves rise 28
+// times over their best at most there (1000 x 5 x 5; other shapes 3, few past 5).
+__device__ __forceinline__ bool residual_grew(double rr, double best, double r0, double bnorm, double rz,
+                                              double rz0, double rz_peak, int it, bool last) {
     const double f = fmax(r0, 1e-3 * bnorm);
-    return rr > 1e12 * f * f || (last && it > 4 && rr > 1e4 * f * f && 4.0 * rr > peak);
+    return rr > 1e12 * f * f ||
+           (last && it > 1 && rr > 4.0 * f * f && rz > rz0 && 4.0 * rz > rz_peak) ||
+           (4.0 * best < r0 * r0 && rr > (last ? 9.0 : 1e6) * best);
 }
 
 // q = a / d and r = a % d for 0 <= a < 2^31, 0 < d, from a reciprocal 1/d computed

@@ -1866,6 +1866,7 @@ private:
         init.init = 1;
         init.epoch = ++epoch_;
         init.progress = flag_host_;
+        init.rr_best = 1e300;
         init.cover = star_ && a.precond ? 1 : 0;  // (plain CG applies no hierarchy)
         *flag_host_ = progress_word(epoch_, 0, 0);
         *cg_host_ = init;

@@ -470,7 +470,12 @@ __device__ __forceinline__ void true_residual_done(CGState* cg, double rr, int m
         // recurrence drifted: the next search direction restarts (beta = 0),
         // since beta = r.z / r.z_old would mix the replaced residual with
         // directions built for the drifted one
-        if (rr > 4.0 * cg->rr) cg->init = 1;
+        // (and the least residual so far is the true one: below it the recurrence measured
+        // its own rounding)
+        if (rr > 4.0 * cg->rr) {
+            cg->init = 1;
+            cg->rr_best = rr;
+        }
         cg->rr = rr;
         cg->replacements += 1;
         if (cg->cand) {
@@ -479,7 +484,8 @@ __device__ __forceinline__ void true_residual_done(CGState* cg, double rr, int m
         }
         if (!(rr == rr)) { cg->status = cg->cover ? CG_DIVERGED : CG_NAN; cg->done = 1; }
         else if (!cg->done && cg->cover &&
-                 residual_grew(rr, cg->rr_peak, cg->r0, cg->bnorm, cg->iter, cg->iter >= cg->max_iter)) {
+                 residual_grew(rr, cg->rr_best, cg->r0, cg->bnorm, cg->rz_old, cg->rz0, cg->rz_peak,
+                               cg->iter, cg->iter >= cg->max_iter)) {
             cg->status = CG_DIVERGED;
             cg->done = 1;
         }

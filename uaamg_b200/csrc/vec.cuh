@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
         }
     }
     double tot[1];
-    double tol_abs = 0.0, first = 0.0, bnorm = 0.0, peak = 0.0;
+    double tol_abs = 0.0, first = 0.0, bnorm = 0.0, best = 0.0, rz = 0.0, rz0 = 0.0, rz_peak = 0.0;
     int it = 0, every = 0, max_iter = 0, cand = 0, epoch = 0, cover = 0;
     unsigned long long* progress = nullptr;
     if (reduce_last<1>(acc, partials, &cg->counter[1], tot, [&] {
@@ -165,7 +165,10 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             cand = ld_now(&cg->cand);
             cover = ld_now(&cg->cover);
             bnorm = ld_now(&cg->bnorm);
-            peak = ld_now(&cg->rr_peak);
+            best = ld_now(&cg->rr_best);
+            rz = ld_now(&cg->rz_old);
+            rz0 = ld_now(&cg->rz0);
+            rz_peak = ld_now(&cg->rz_peak);
             epoch = ld_now(&cg->epoch);
             progress = ld_now(&cg->progress);
         })) {
@@ -185,9 +188,12 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
         } else if (it >= max_iter && every == 0) status = CG_MAXITER;
         if (every > 0 && status == CG_RUNNING && it >= max_iter && !cand) status = CG_MAXITER;
         if (cover) {
-            cg->rr_peak = peak = fmax(peak, rr);
+            cg->rr_best = best = fmin(best, rr);
+            if (it == 1) cg->rz0 = rz0 = rz;
+            cg->rz_peak = rz_peak = fmax(rz_peak, rz);
             if (status == CG_NAN || ((status == CG_RUNNING || status == CG_MAXITER) &&
-                                     residual_grew(rr, peak, first, bnorm, it, status == CG_MAXITER)))
+                                     residual_grew(rr, best, first, bnorm, rz, rz0, rz_peak, it,
+                                                   status == CG_MAXITER)))
                 status = CG_DIVERGED;
         }
         if (status != CG_RUNNING) { cg->status = status; cg->done = 1; }
