@@ -125,3 +125,36 @@ def test_inconsistent_share_ends_as_on_the_reference_hierarchy(handle, dim, shar
     st = handle.solve(b, np.zeros_like(b), handle.options(precision, 1e-7, max_iter, "rel"))
     assert st.rel_residual <= max(6.0 * ref.rel_residual, 1e-5)
     assert st.status == 0 or st.iterations == max_iter
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_a_run_away_that_overflows_is_repeated(handle, dim):
+    """A large right-hand side: the run-away iterates overflow FP32 before the residual has
+    grown enough, and the solve used to end with NaN.  On the reference's hierarchy it ends
+    at max_iter, finite."""
+    solid, lab = _rooms(dim)
+    b = _inconsistent(solid, lab, 1e-2) * 1e32
+    handle.set_problem(solid, 1.0, 1.0, 1.0)
+    p = np.zeros_like(b)
+    st = handle.solve(b, p, handle.options("fp32", 1e-8, 40, "rel"))
+    assert st.status == 1 and st.iterations == 40
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp32"])
+def test_not_finite_and_tiny_right_hand_sides_are_not_repeated(handle, precision):
+    """NaN in the right-hand side ends as NaN, and one whose p.Ap lies below the absolute
+    threshold as a breakdown, in one engine."""
+    solid, b = _smooth((70, 50), 3)
+    handle.set_problem(solid, 1.0, 1.0)
+    handle.solve(b, np.zeros_like(b), handle.options(precision, 1e-3, 30, "rel"), strict=True)
+    held = handle.device_bytes()
+    st = handle.solve(1e-12 * b, np.zeros_like(b), handle.options(precision, 1e-20, 30, "abs"))
+    assert st.status == 2
+    bad = b.copy()
+    bad[20, 20] = np.nan
+    with pytest.raises(Exception, match="nan"):
+        handle.solve(bad, np.zeros_like(b), handle.options(precision, 1e-6, 30, "rel"))
+    bad[20, 20] = np.inf
+    with pytest.raises(Exception, match="nan"):
+        handle.solve(bad, np.zeros_like(b), handle.options(precision, 1e-6, 30, "rel"))
+    assert handle.device_bytes() == held

@@ -454,6 +454,34 @@ __global__ void k_sub_mean(Geom g, const uint8_t* __restrict__ s, double* v, con
     });
 }
 
+// Whether a NaN ends a solve on covering aggregates that ran away (to infinity and on to
+// NaN, 1e32 times as large a right-hand side within FP32's range) rather than one whose
+// right-hand side was not finite: only the first is repeated.
+__device__ __forceinline__ int nan_status(const CGState* cg) {
+    return cg->cover && cg->r0 <= 1.7e308 ? CG_DIVERGED : CG_NAN;
+}
+
+// p.Ap, reduced: alpha, or the end of the solve.  On covering aggregates a breakdown is one
+// of a run-away solve when the direction is nearly a null vector (a consistent solve's
+// alpha = r.z / p.Ap is the inverse of an eigenvalue of M A, 1 to 230 measured up to 3000 x
+// 6) or when the residual shows it; a right-hand side so small that p.Ap is below the
+// absolute threshold ends as it is.
+__device__ __forceinline__ void finish_pap(CGState* cg, double pap, double rz, double breakdown) {
+    cg->pap = pap;
+    if (pap == pap && !(pap < breakdown)) {
+        cg->alpha = rz / pap;
+        return;
+    }
+    int status = CG_BREAKDOWN;
+    if (!(pap == pap)) status = nan_status(cg);
+    else if (cg->cover && cg->iter > 0 &&
+             ((rz > 1e4 * pap && cg->rr > 1e-24 * cg->r0 * cg->r0) ||
+              residual_grew(cg->rr, cg->rr_best, cg->r0, cg->bnorm, rz, cg->rz0, cg->rz_peak, cg->iter, true)))
+        status = CG_DIVERGED;
+    cg->status = status;
+    cg->done = 1;
+}
+
 // The last block's bookkeeping of a true residual r.r (rr): mode 0 the initial
 // residual (r0, the absolute tolerance); mode 1 a residual replacement; 2 and 3
 // record it only.
@@ -482,7 +510,7 @@ __device__ __forceinline__ void true_residual_done(CGState* cg, double rr, int m
             cg->cand = 0;
             if (sqrt(rr) < cg->tol_abs) { cg->status = CG_CONVERGED; cg->done = 1; }
         }
-        if (!(rr == rr)) { cg->status = cg->cover ? CG_DIVERGED : CG_NAN; cg->done = 1; }
+        if (!(rr == rr)) { cg->status = nan_status(cg); cg->done = 1; }
         else if (!cg->done && cg->cover &&
                  residual_grew(rr, cg->rr_best, cg->r0, cg->bnorm, cg->rz_old, cg->rz0, cg->rz_peak,
                                cg->iter, cg->iter >= cg->max_iter)) {
@@ -822,11 +850,7 @@ __global__ void __launch_bounds__(256) k_pmatvec_2d(Geom g, const uint8_t* __res
             rz_old = ld_now(&cg->rz_old);
             breakdown = ld_now(&cg->breakdown);
         })) {
-        const double pap = tot[0];
-        cg->pap = pap;
-        if (!(pap == pap)) { cg->status = CG_NAN; cg->done = 1; }
-        else if (pap < breakdown) { cg->status = CG_BREAKDOWN; cg->done = 1; }
-        else cg->alpha = rz_old / pap;
+        finish_pap(cg, tot[0], rz_old, breakdown);
     }
 }
 
@@ -853,7 +877,7 @@ __device__ __forceinline__ void finish_zdot(CGState* cg, const ZdotIn& in, const
     cg->beta = in.init ? 0.0 : rz / in.rz_old;
     cg->rz_old = rz;
     cg->init = 0;
-    if (!(rz == rz)) { cg->status = CG_NAN; cg->done = 1; }
+    if (!(rz == rz)) { cg->status = nan_status(cg); cg->done = 1; }
 }
 
 // The same sums with a z march's partition and order: block (bx, by, bz) sums the tile

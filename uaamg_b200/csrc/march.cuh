@@ -1027,11 +1027,7 @@ __global__ void __launch_bounds__(kThreads, DIRW ? 1 : PmvCfg<DIM, T>::MINB)
             rz_old = ld_now(&cg->rz_old);
             breakdown = ld_now(&cg->breakdown);
         })) {
-        const double pap = tot[0];
-        cg->pap = pap;
-        if (!(pap == pap)) { cg->status = CG_NAN; cg->done = 1; }
-        else if (pap < breakdown) { cg->status = CG_BREAKDOWN; cg->done = 1; }
-        else cg->alpha = rz_old / pap;
+        finish_pap(cg, tot[0], rz_old, breakdown);
     }
 }
 

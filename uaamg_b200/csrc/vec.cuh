@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             hist[it] = sqrt(rr);
         }
         int status = CG_RUNNING;
-        if (!(rr == rr)) status = CG_NAN;
+        if (!(rr == rr)) status = nan_status(cg);
         else if (sqrt(rr) < tol_abs) {
             if (every > 0) { cand = 1; cg->cand = 1; }
             else status = CG_CONVERGED;
@@ -191,9 +191,8 @@ __global__ void __launch_bounds__(256) k_update_flat(long long nvec, T* x, T* r,
             cg->rr_best = best = fmin(best, rr);
             if (it == 1) cg->rz0 = rz0 = rz;
             cg->rz_peak = rz_peak = fmax(rz_peak, rz);
-            if (status == CG_NAN || ((status == CG_RUNNING || status == CG_MAXITER) &&
-                                     residual_grew(rr, best, first, bnorm, rz, rz0, rz_peak, it,
-                                                   status == CG_MAXITER)))
+            if ((status == CG_RUNNING || status == CG_MAXITER) &&
+                residual_grew(rr, best, first, bnorm, rz, rz0, rz_peak, it, status == CG_MAXITER))
                 status = CG_DIVERGED;
         }
         if (status != CG_RUNNING) { cg->status = status; cg->done = 1; }
