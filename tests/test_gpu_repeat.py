@@ -158,3 +158,62 @@ def test_not_finite_and_tiny_right_hand_sides_are_not_repeated(handle, precision
     with pytest.raises(Exception, match="nan"):
         handle.solve(bad, np.zeros_like(b), handle.options(precision, 1e-6, 30, "rel"))
     assert handle.device_bytes() == held
+
+
+def _two_chambers():
+    """Two chambers with a net source each (no solution exists)."""
+    solid = np.zeros((72, 92), np.uint8)
+    solid[:, 45] = 1
+    fl = fluid_interior(solid)
+    b = np.where(fl, np.random.default_rng(3).standard_normal(solid.shape), 0.0)
+    b[:, :45][fl[:, :45]] += 1.0
+    b[fl] -= b[fl].mean()
+    return solid, b
+
+
+@pytest.mark.parametrize("modes", [(0, 1), (0, 4), (3, 0), (2, 1)])
+def test_repeat_follows_the_kernel_mode(handle, modes):
+    """The repeat's engine, kept while the mask stays, runs the V-cycle kernels that are set
+    now: as many launches as in a handle where it was made with them."""
+    from uaamg_b200.solver import Handle
+    solid, b = _two_chambers()
+    opts = handle.options("mixed", 1e-6, 40, "rel")
+    other = Handle(0)
+    try:
+        got = []
+        for h, ms in ((handle, modes), (other, modes[1:])):
+            h.set_problem(solid, 1.0, 1.0)
+            for m in ms:
+                h.set_vcycle_kernels(m)
+                p = np.zeros_like(b)
+                st = h.solve(b, p, opts)
+            assert st.status == 1 and st.iterations == 40
+            got.append((st.kernel_launches, p))
+        assert got[0][0] == got[1][0]
+        assert np.array_equal(got[0][1], got[1][1])
+    finally:
+        handle.set_vcycle_kernels(0)
+        other.close()
+
+
+def test_repeat_follows_the_stream(handle):
+    """The stream a solve was repeated on is gone before the next mask and the next repeat."""
+    from cuda.bindings import runtime as rt
+    solid, b = _two_chambers()
+    opts = handle.options("mixed", 1e-6, 40, "rel")
+    handle.set_problem(solid, 1.0, 1.0)
+    p, q = np.zeros_like(b), np.zeros_like(b)
+    handle.solve(b, p, opts)
+    err, stream = rt.cudaStreamCreate()
+    assert err == rt.cudaError_t.cudaSuccess
+    try:
+        handle.set_stream(int(stream))
+        st = handle.solve(b, q, opts)
+        assert st.status == 1 and np.array_equal(p, q)
+    finally:
+        handle.set_stream(0)
+        rt.cudaStreamDestroy(stream)
+    handle.set_problem(solid, 1.0, 1.0)  # releases the repeat's engine
+    q[:] = 0
+    st = handle.solve(b, q, opts)
+    assert st.status == 1 and np.array_equal(p, q)

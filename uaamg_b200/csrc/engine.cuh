@@ -358,7 +358,10 @@ public:
         return E_OK;
     }
 
-    void set_stream(cudaStream_t s) override { st_ = s; }
+    void set_stream(cudaStream_t s) override {
+        st_ = s;
+        if (fb_) fb_->st_ = s;  // (its next use may be its release)
+    }
     size_t device_bytes() const override { return bytes_ + (fb_ ? fb_->device_bytes() : 0); }
     long launches() const override { return launches_ + (fb_on_ ? fb_->launches() : 0); }
     void set_vcycle_sweeps(bool on) override { sweeps_ = on; }
@@ -452,12 +455,6 @@ private:
             fb_ = new (std::nothrow) EngineT<T, CS>(mixed_);
             if (!fb_) return E_OK;
             fb_->st_ = st_;
-            fb_->sweeps_ = sweeps_;
-            fb_->tail_on_ = tail_on_;
-            fb_->fused_ = fused_;
-            fb_->graphs_ = graphs_;
-            fb_->nu_fine_ = nu_fine_;
-            fb_->nu_coarse_ = nu_coarse_;
             const Geom& g = lv_[0].g;
             if (fb_->set_problem(dim_, g.nx, g.ny, g.nz, dx_, dy_, dz_, cur_.ref_solid, dirichlet_) != E_OK) {
                 delete fb_;  // no room for it: the diverged result stands
@@ -466,6 +463,10 @@ private:
             }
         }
         fb_->st_ = st_;
+        fb_->set_vcycle_sweeps(sweeps_);
+        fb_->set_small_levels(tail_on_);
+        fb_->set_fused(fused_);
+        fb_->set_graphs(graphs_);
         fb_->set_operator(vd_, vox_, voy_, vsx_, vver_);
         fb_->set_smoothing(nu_fine_, nu_coarse_);
         fb_->prof_on_ = false;
