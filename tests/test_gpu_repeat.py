@@ -217,3 +217,46 @@ def test_repeat_follows_the_stream(handle):
     q[:] = 0
     st = handle.solve(b, q, opts)
     assert st.status == 1 and np.array_equal(p, q)
+
+
+def test_repeat_without_room_for_a_second_engine(handle):
+    """With the device's memory taken, a run-away solve is repeated in its own engine: the
+    same result as with a second one, and the next mask is on covering aggregates again."""
+    import torch
+    solid = np.zeros((1502, 2002), np.uint8)
+    solid[:, 1000] = 1
+    fl = fluid_interior(solid)
+    rng = np.random.default_rng(8)
+    b = np.where(fl, rng.standard_normal(solid.shape), 0.0)
+    c = b.copy()
+    b[:, :1000][fl[:, :1000]] += 1.0
+    b[fl] -= b[fl].mean()
+    for sl in (slice(1, 1000), slice(1001, 2001)):
+        c[1:-1, sl] -= c[1:-1, sl].mean()
+    opts = handle.options("mixed", 1e-6, 40, "rel")
+    handle.set_problem(solid, 1.0, 1.0)
+    want, good = np.zeros_like(b), np.zeros_like(b)
+    ref = handle.solve(b, want, opts)
+    st = handle.solve(c, good, opts, strict=True)
+    two = handle.device_bytes()
+    handle.set_problem(solid, 1.0, 1.0)  # the second engine is gone
+    q = np.zeros_like(b)
+    handle.solve(c, q, opts, strict=True)
+    one = handle.device_bytes()
+    assert two > one and np.array_equal(q, good)
+    torch.cuda.init()
+    free, _ = torch.cuda.mem_get_info(0)
+    hog = torch.empty(free - (two - one) // 2, dtype=torch.uint8, device="cuda:0")
+    try:
+        p = np.zeros_like(b)
+        got = handle.solve(b, p, opts)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert handle.device_bytes() <= one
+    assert got.status == ref.status == 1 and got.iterations == ref.iterations
+    assert np.array_equal(p, want)
+    handle.set_problem(solid, 1.0, 1.0)
+    q[:] = 0
+    again = handle.solve(c, q, opts, strict=True)
+    assert again.iterations == st.iterations and np.array_equal(q, good)

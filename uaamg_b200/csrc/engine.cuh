@@ -160,6 +160,11 @@ public:
     // same addresses and sizes.
     int set_problem(int dim, int nx, int ny, int nz, double dx, double dy, double dz,
                     const uint8_t* d_solid, int dirichlet) override {
+        plain_ = false;
+        return set_problem_now(dim, nx, ny, nz, dx, dy, dz, d_solid, dirichlet);
+    }
+    int set_problem_now(int dim, int nx, int ny, int nz, double dx, double dy, double dz,
+                        const uint8_t* d_solid, int dirichlet) {
         delete fb_;
         fb_ = nullptr;
         fb_on_ = false;
@@ -446,41 +451,54 @@ private:
 
     // The residual of a solve on covering aggregates grew (common.cuh, residual_grew): the
     // same solve from its beginning on the reference's hierarchy, by an engine of its own
-    // (made here, kept while the mask stays); the stages then go to it.  Nothing has been
-    // added to the caller's x yet.
+    // (made here, kept while the mask stays); the stages then go to it.  Without room for
+    // one, this engine takes the reference's hierarchy until the next mask (its buffers are
+    // no larger).  Nothing has been added to the caller's x yet.
     int fall_back(bool* stopped) {
         *stopped = true;
         if (!cur_.ref_solid) return E_OK;
+        const Geom g = lv_[0].g;
+        const SolveArgs a = cur_;
+        int e = E_OK;
         if (!fb_) {
             fb_ = new (std::nothrow) EngineT<T, CS>(mixed_);
-            if (!fb_) return E_OK;
+            if (fb_) fb_->st_ = st_;
+            e = fb_ ? fb_->set_problem(dim_, g.nx, g.ny, g.nz, dx_, dy_, dz_, a.ref_solid, dirichlet_) : E_OOM;
+        }
+        if (e == E_OK) {
             fb_->st_ = st_;
-            const Geom& g = lv_[0].g;
-            if (fb_->set_problem(dim_, g.nx, g.ny, g.nz, dx_, dy_, dz_, cur_.ref_solid, dirichlet_) != E_OK) {
-                delete fb_;  // no room for it: the diverged result stands
-                fb_ = nullptr;
+            fb_->set_vcycle_sweeps(sweeps_);
+            fb_->set_small_levels(tail_on_);
+            fb_->set_fused(fused_);
+            fb_->set_graphs(graphs_);
+            fb_->set_operator(vd_, vox_, voy_, vsx_, vver_);
+            fb_->set_smoothing(nu_fine_, nu_coarse_);
+            fb_->prof_on_ = false;
+            e = fb_->solve_begin(a);
+            if (e == E_OK) {
+                fb_on_ = true;
+                *stopped = false;
                 return E_OK;
             }
         }
-        fb_->st_ = st_;
-        fb_->set_vcycle_sweeps(sweeps_);
-        fb_->set_small_levels(tail_on_);
-        fb_->set_fused(fused_);
-        fb_->set_graphs(graphs_);
-        fb_->set_operator(vd_, vox_, voy_, vsx_, vver_);
-        fb_->set_smoothing(nu_fine_, nu_coarse_);
-        fb_->prof_on_ = false;
-        const int e = fb_->solve_begin(cur_);
-        if (e != E_OK) return e;
-        fb_on_ = true;
-        *stopped = false;
-        return E_OK;
+        if (e != E_OOM) {
+            cuda_error = fb_->cuda_error;
+            return e;
+        }
+        const long before = launches_;
+        plain_ = true;
+        e = set_problem_now(dim_, g.nx, g.ny, g.nz, dx_, dy_, dz_, a.ref_solid, dirichlet_);
+        if (e == E_OK) e = solve_begin(a);
+        launches_ += before;
+        if (e == E_OK) *stopped = false;
+        return e;
     }
 
     EngineT<T, CS>* fb_ = nullptr;
     bool fb_on_ = false;
     bool mixed_;
     bool cover_ = false, apply_only_ = false;
+    bool plain_ = false;  // this mask on the reference's hierarchy (fall_back without room)
     bool star_ = false;  // the current hierarchy covers and its transfers reach face neighbours
     int dim_ = 0, dirichlet_ = 0;
     double dx_ = 1, dy_ = 1, dz_ = 1;
@@ -674,7 +692,7 @@ private:
                                  (double)dirichlet_, (double)(uintptr_t)arena_, (double)arena_used_,
                                  (double)pm_zc_, (double)zdot_zc_, (double)rx_zc_, (double)pmv2d_per_sm_,
                                  (double)resid_per_sm_, (double)tail_lt_, (double)tail_nc_,
-                                 (double)dense_n_};
+                                 (double)dense_n_, (double)star_};
         for (const auto& L : lv_) {
             v.push_back(L.zc);
             v.push_back(L.zu);
@@ -974,7 +992,7 @@ private:
         // 129 x 97 x 65 204 -> 46 (19.6 -> 5.0 ms).  The FP64 form and every V-cycle applied by itself
         // keep the reference's rule, and so do problems with Dirichlet walls (their wall
         // channel is defined by it).
-        const bool cover = cover_ && !dirichlet_;
+        const bool cover = cover_ && !plain_ && !dirichlet_;
         star_ = cover;
         const int up = cover ? 1 : 0;
         double hx = dx_, hy = dy_, hz = dz_;
@@ -1232,7 +1250,7 @@ private:
         tail_lt_ = lt;
         tail_nc_ = 1;
         tail_smem_ = elems * sizeof(T);
-        if (sizeof(T) == 4 && cover_ && cells(lv_[lt].g) <= (double)kDenseCells) {
+        if (sizeof(T) == 4 && cover_ && !plain_ && cells(lv_[lt].g) <= (double)kDenseCells) {
             dense_cells_ = (int)cells(lv_[lt].g);
             dense_ld_ = (dense_cells_ + 3) / 4 * 4;
         }
