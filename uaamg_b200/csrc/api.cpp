@@ -163,7 +163,6 @@ uaamg_status set_problem(uaamg_handle* h, int dim, int nx, int ny, int nz, doubl
 }
 
 uaamg_status ensure_hist(uaamg_handle* h, int max_iter) {
-    h->has_hist = true;
     if (max_iter + 1 <= h->hist_cap) return UAAMG_OK;
     cudaFree(h->d_hist);
     h->d_hist = nullptr;
@@ -187,6 +186,7 @@ uaamg_status solve_dev(uaamg_handle* h, const double* d_rhs, double* d_p, const 
     uaamg::Engine* eng = nullptr;
     uaamg_status s = engine_for(h, opts.precision, &eng);
     if (s != UAAMG_OK) return s;
+    h->has_hist = false;  // until this solve has filled it
     if ((s = ensure_hist(h, opts.max_iter)) != UAAMG_OK) return s;
     uaamg::SolveArgs a;
     a.rhs = d_rhs;
@@ -208,6 +208,7 @@ uaamg_status solve_dev(uaamg_handle* h, const double* d_rhs, double* d_p, const 
     if (eng->timed_out())
         return fail(h, UAAMG_TIMEOUT, "solve: a kernel gave up waiting for its tile loads");
     h->last_iters = r.iterations;
+    h->has_hist = true;
     return uaamg::api::fill_stats(eng, r, st);
 }
 

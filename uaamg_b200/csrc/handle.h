@@ -25,7 +25,7 @@ struct uaamg_handle {
     cudaEvent_t p_ready = nullptr;
     size_t face_n[3] = {0, 0, 0};
     int hist_cap = 0;
-    bool has_hist = false;  // a solve of the current problem has filled d_hist
+    bool has_hist = false;  // the last solve of the current problem has filled d_hist
     int last_iters = 0;
     // by precision; 3 and 4: FP32 and mixed on the reference's hierarchy (V-cycles applied
     // by themselves and level inspection; made on first use)
