@@ -260,3 +260,60 @@ def test_repeat_without_room_for_a_second_engine(handle):
     q[:] = 0
     again = handle.solve(c, q, opts, strict=True)
     assert again.iterations == st.iterations and np.array_equal(q, good)
+
+
+def _serve(srv, sim_id, solid, b):
+    t = srv.submit(sim_id, solid, b, 1.0, 1.0)
+    srv.drain()
+    return srv.poll(t)
+
+
+def test_server_counts_the_engine_of_a_repeat(handle):
+    """The resident bytes grow by the repeat's engine, and idle ids make room for it."""
+    from uaamg_b200.solver import Server
+    solid, b = _two_chambers()
+    c = np.zeros_like(b)
+    for sl in (slice(1, 45), slice(46, 91)):
+        c[1:-1, sl] = np.random.default_rng(4).standard_normal(c[1:-1, sl].shape)
+        c[1:-1, sl] -= c[1:-1, sl].mean()
+    srv = Server(0, "mixed", 1e-6, 40)
+    try:
+        assert _serve(srv, 1, solid, c)["status"] == 0
+        one = srv.info()["device_bytes"]
+        assert _serve(srv, 1, solid, b)["status"] == 1
+        two = srv.info()["device_bytes"]
+        assert two > 1.2 * one
+    finally:
+        srv.stop()
+    # room for two ids, not for a third engine
+    srv = Server(0, "mixed", 1e-6, 40, hbm_budget_bytes=2 * one + (two - one) // 2)
+    try:
+        assert _serve(srv, 1, solid, c)["status"] == 0
+        assert _serve(srv, 2, solid, c)["status"] == 0
+        assert srv.info()["device_bytes"] <= 2 * one
+        assert _serve(srv, 2, solid, b)["status"] == 1
+        info = srv.info()
+        assert info["resident"] == 1 and info["device_bytes"] == two
+    finally:
+        srv.stop()
+
+
+@pytest.mark.parametrize("shape", [(48, 48), (64, 64), (70, 33)])
+def test_server_budget_holds_for_small_ids(shape):
+    """Small grids hold the dense tail's matrix, many times the grid: a budget for one and a
+    half of them admits one at a time."""
+    from uaamg_b200.solver import Server
+    solid, b = _smooth(shape, 2)
+    srv = Server(0, "mixed", 1e-6, 100)
+    try:
+        assert _serve(srv, 1, solid, b)["status"] == 0
+        one = srv.info()["device_bytes"]
+    finally:
+        srv.stop()
+    srv = Server(0, "mixed", 1e-6, 100, hbm_budget_bytes=one + one // 2)
+    try:
+        for sim in (1, 2, 3):
+            assert _serve(srv, sim, solid, b)["status"] == 0
+            assert srv.info()["device_bytes"] <= one + one // 2
+    finally:
+        srv.stop()

@@ -10,6 +10,11 @@
 
 namespace uaamg {
 
+// Largest small-level part of the V-cycle that the FP32 and mixed solves keep as a dense
+// matrix (tail.cuh, k_tail_dense): 4 MB, every level the tail takes by its cell count; a
+// larger first level (a long thin coarsest level) keeps the one-block kernel.
+constexpr int kDenseCells = 1024;
+
 // Engine precision modes (match uaamg_precision in include/uaamg.h).
 enum Precision : int { PREC_FP64 = 0, PREC_FP32 = 1, PREC_MIXED = 2 };
 

@@ -518,10 +518,20 @@ struct StageBuf {
 };
 
 // Device bytes a new id of this shape is expected to hold (engine + staging),
-// used for admission before its hierarchy exists.
+// used for admission before its hierarchy exists.  The FP32 and mixed engines hold the
+// matrix of the dense tail too: up to 4 MB, which outweighs the grid of a small id.
 size_t estimate_bytes(int prec, int dim, int nx, int ny, int nz) {
     const size_t n = padded_cells(dim, nx, ny, nz);
-    return n * (prec == PREC_FP64 ? 200 : 120);
+    if (prec == PREC_FP64) return n * 200;
+    size_t tail = 0;
+    while (!tail && nx > 4 && ny > 4 && (dim == 2 || nz > 4)) {
+        nx = (nx + 1) / 2;
+        ny = (ny + 1) / 2;
+        nz = (nz + 1) / 2;
+        const size_t c = (size_t)nx * ny * (dim == 3 ? nz : 1);
+        if (c <= kDenseCells) tail = c * (c + 3) * 4;
+    }
+    return n * 120 + tail;
 }
 
 }  // namespace
@@ -595,6 +605,17 @@ void finish(uaamg_server* s, Ticket* t, int status) {
     if (t->sim) {
         t->sim->busy = false;
         t->sim->last_used = ++s->tick;
+        // a solve that was repeated has made an engine more
+        const size_t now = t->sim->dp.bytes(), was = t->sim->bytes;
+        t->sim->bytes = now;
+        if (now != was) {
+            {
+                std::lock_guard<std::mutex> lk(s->mu);
+                s->resident_bytes += now - was;
+            }
+            make_room(s, 0);  // (may release this id too)
+            t->sim = nullptr;
+        }
     }
     std::lock_guard<std::mutex> lk(s->mu);
     t->done = true;

@@ -33,11 +33,6 @@ constexpr size_t kTailSmemBytes = 200 * 1024;    // x and b of every tail level
 template <class T>
 constexpr int tail_threads() { return sizeof(T) == 8 ? 512 : 1024; }
 
-// Largest tail level whose whole cycle is kept as a dense matrix (k_tail_dense): 4 MB,
-// every level the tail takes by its cell count; a larger first level (a long thin
-// coarsest level) keeps the one-block kernel.
-constexpr int kDenseCells = 1024;
-
 template <class T>
 struct TailLevel {
     Geom g;          // the level's global (pitched) layout
@@ -449,7 +444,7 @@ __global__ void __launch_bounds__(tail_threads<T>()) k_tail(const __grid_constan
 }
 
 // The same cycle as one product x = M b.  From the tail's first level down the cycle is
-// a fixed linear map of its n <= kDenseCells cells, so the FP32 and mixed solves apply
+// a fixed linear map of its n <= kDenseCells (engine.h) cells, so the FP32 and mixed solves apply
 // its matrix, formed at set-up by running k_tail on every unit vector (n blocks, 40-90
 // us once per mask), instead of some 60 dependent phases in one block.  M is symmetric
 // (forward and reverse sweeps are adjoint), so its rows as written serve as its rows as
