@@ -931,7 +931,7 @@ private:
                 if ((e = alloc(L.x, n))) return e;
                 if ((e = alloc(L.b, n))) return e;
                 if ((e = alloc(L.dg, n))) return e;
-                if (L.box && !cover_) {
+                if (L.box && !star_ && !plain_) {
                     const dim3 bg = box_grid(L.g);
                     if ((e = alloc(L.trim, (size_t)4 * bg.x * bg.y * bg.z))) return e;
                 }
@@ -1198,8 +1198,8 @@ private:
         if constexpr (DIM == 3) {  // trimmed boxes of the coarse box levels
             for (int l = 1; l < nl; ++l) {
                 const LevelBuf<T, CS>& Cl = lv_[l];
-                // (not for the solves' covering hierarchy: their dozen iterations took the same
-                // time with it and without, and finding the boxes costs 65 us of set-up)
+                // (not for the covering hierarchy: its dozen iterations took the same time with
+                // trimming and without, and finding the boxes costs 65 us of set-up)
                 if (!Cl.box || !Cl.trim) continue;
                 const MLevel<T> m = mlevel(l);
                 if (kHalf && !Cl.c32)
