@@ -78,7 +78,7 @@ typedef struct uaamg_stats {
     int status;                 /* uaamg_status of the solve */
     int iterations;             /* x/r updates performed */
     int replacements;           /* FP64 residual replacements (UAAMG_MIXED) */
-    int levels;                 /* multigrid levels */
+    int levels;                 /* multigrid levels (as uaamg_num_levels) */
     double residual;            /* FP64 true ||b - A p|| at exit (fluid cells) */
     double rel_residual;        /* residual / ||b|| */
     double recursive_residual;  /* the CG's recursive ||r|| at exit */

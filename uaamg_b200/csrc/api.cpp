@@ -37,6 +37,23 @@ uaamg_status map_engine(uaamg_handle* h, int e, const char* where, const uaamg::
     }
 }
 
+namespace {
+// Levels of the reference's hierarchy (uaamg_num_levels) over the engine's grid; the covering
+// aggregates round odd sizes up and can have one more.
+int reference_levels(const uaamg::Engine* eng) {
+    int nx = 0, ny = 0, nz = 0, n = 1;
+    eng->level_dims(0, &nx, &ny, &nz);
+    const bool flat = nz == 0;
+    while (nx > 4 && ny > 4 && (flat || nz > 4)) {
+        nx /= 2;
+        ny /= 2;
+        nz /= 2;
+        ++n;
+    }
+    return n;
+}
+}  // namespace
+
 uaamg_status fill_stats(const uaamg::Engine* eng, const uaamg::SolveResult& r, uaamg_stats* st) {
     uaamg_status out;
     switch (r.status) {
@@ -49,7 +66,7 @@ uaamg_status fill_stats(const uaamg::Engine* eng, const uaamg::SolveResult& r, u
         st->status = out;
         st->iterations = r.iterations;
         st->replacements = r.replacements;
-        st->levels = eng->nlevels();
+        st->levels = reference_levels(eng);
         st->residual = r.rr_true >= 0 ? __builtin_sqrt(r.rr_true) : 0.0;
         st->rhs_norm = r.bnorm;
         st->rel_residual = r.bnorm > 0 ? st->residual / r.bnorm : st->residual;
