@@ -162,8 +162,10 @@ UAAMG_API uaamg_status uaamg_set_vcycle_kernels(uaamg_handle* h, int sweeps);
  * is the reference's V(1,1) (UAAMGPreconditioner3D::vCycle, uaamg_preconditioner_3d.cpp:
  * 183-196; its CUDA path fixes NU = 1, cuda_uaamg_preconditioner_3d_opt_f.cu:444).  More
  * sweeps make a different (still symmetric) preconditioner; the batch autotuner
- * (uaamg_set_autotune) may choose them per problem class.  Takes effect at the next
- * solve. */
+ * (uaamg_set_autotune) may choose them per problem class.  A level with more than one
+ * sweep has constant transfers to the next coarser one in every precision, and the levels
+ * of the small-level kernel (at most 1024 cells; uaamg_set_vcycle_kernels) keep one sweep.
+ * Takes effect at the next solve. */
 UAAMG_API uaamg_status uaamg_set_smoothing(uaamg_handle* h, int sweeps_fine, int sweeps_coarse);
 
 /* Solve lap(p) = rhs with HOST FP64 arrays (padded): the Solver::solve /

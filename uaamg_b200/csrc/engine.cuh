@@ -1673,15 +1673,12 @@ private:
             else up_fused<DIM, FINE, CSL, false, false>(l, done);
             return;
         }
-        UAAMG_LAUNCH_SMEM((KTag{K_UPE, l, c * (2.0 * t + 1.0 + coef) + cc * t}),
-                          (k_up_even<DIM, T, FINE, CSL>), grid, blk, (UpeCfg<DIM, T, FINE, CSL>::BYTES),
-                          maps<DIM>(l, false, true), mlevel(l), x, done, err_);
-        if (nu > 1) {  // first reverse sweep, further reverse sweeps (colour 0, then 1), z sums
-            UAAMG_LAUNCH_SMEM((KTag{K_UPO, l, c * (2.5 * t + 1.0 + coef)}),
-                              (k_up_odd<DIM, T, FINE, false, CSL>), grid, blk, (UpoCfg<DIM, T, FINE, CSL>::BYTES),
-                              maps<DIM>(l, true, false), mlevel(l), x, done, err_, partials_, cg_);
+        if (nu > 1) {  // (the marches' first colour starts from x of a single forward sweep)
             const LevelView<T> v = view(l, r_, z_);
-            for (int q = 1; q < nu; ++q) {
+            UAAMG_LAUNCH((KTag{K_PROLONG, l, c * (2.0 * t + 1.0) + cc * (t + 1.0)}), (k_prolong<DIM, T>),
+                         cell_grid<DIM>(Cl.g.nx, Cl.g.ny, Cl.g.nz), cell_block<DIM>(), Cl.g, Cl.solid, Cl.x,
+                         v.g, v.solid, v.x, done);
+            for (int q = 0; q < nu; ++q) {  // reverse sweeps: colour 0, then 1
                 sweep<DIM>(v, 0, done, l);
                 sweep<DIM>(v, 1, done, l);
             }
@@ -1690,6 +1687,9 @@ private:
                              dim3(32, 8), L.g, L.solid, r_, z_, partials_, cg_);
             return;
         }
+        UAAMG_LAUNCH_SMEM((KTag{K_UPE, l, c * (2.0 * t + 1.0 + coef) + cc * t}),
+                          (k_up_even<DIM, T, FINE, CSL>), grid, blk, (UpeCfg<DIM, T, FINE, CSL>::BYTES),
+                          maps<DIM>(l, false, true), mlevel(l), x, done, err_);
         if (zdot)
             UAAMG_LAUNCH_SMEM((KTag{K_UPO, l, c * (2.5 * t + 1.0 + coef)}),
                               (k_up_odd<DIM, T, FINE, true, CSL>), grid, blk, (UpoCfg<DIM, T, FINE, CSL>::BYTES),

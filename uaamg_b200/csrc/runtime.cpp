@@ -148,8 +148,8 @@ std::vector<int> tune_schedule(DevProblem& d, const uaamg_problem& p, const uaam
                 ++inner;
             }
     const int bucket = (int)(20.0 * (double)solid / (double)(inner ? inner : 1) + 0.5);
-    // (v2: schedules timed on the covering aggregates)
-    const std::string key = "nu|v2|" + tune_gpu_id() + "|" +
+    // (v3: schedules timed on the covering aggregates, with every forward sweep kept)
+    const std::string key = "nu|v3|" + tune_gpu_id() + "|" +
                             (o.precision == PREC_MIXED ? "mixed" : "f32") + "|" + std::to_string(p.dim) +
                             "|" + std::to_string(p.nx) + "x" + std::to_string(p.ny) + "x" +
                             std::to_string(p.dim == 3 ? p.nz : 0) + "|s" + std::to_string(bucket);
