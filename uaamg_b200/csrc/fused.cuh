@@ -146,7 +146,7 @@ struct FCfg {
     // 69 us); 2D, eight (a full SM of 256-thread
     // blocks; the 2D way up at five blocks and 48 registers: 2048 x 1024 solve 10.24
     // against 9.99 ms)
-    static constexpr int MINB = LEAN ? (DIM == 3 ? (UP || STAR ? 4 : 5) : 8) : 1;
+    static constexpr int MINB = LEAN ? (DIM == 3 ? (UP ? 4 : 5) : 8) : 1;
     static_assert(S <= 16, "stage barriers: 128 bytes");
 };
 
@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
     constexpr int S = C::S, WT = P::BT::W, WS = P::BS::W;
     constexpr bool kStarDn = STAR && !UP;
     static_assert(!STAR || sizeof(T) == 4, "the FP64 form keeps the reference's transfers");
+    static_assert(!STAR || !FINE, "quad.cuh runs the finest level with STAR transfers");
     constexpr bool kFull = sizeof(T) == 8;  // the reference's residual expression
     UAAMG_FUSED_SMEM(sm, err)
     T* lut = reinterpret_cast<T*>(sm + C::OFF_LUT);
@@ -450,9 +451,7 @@ __global__ void __launch_bounds__(kThreads, (FCfg<DIM, T, CS, FINE, UP, STAR>::M
             const int q = c.qt;
             T nb = L.idx2 * (xv[q + 1] + xv[q - 1]) + L.idy2 * (xv[q + WT] + xv[q - WT]);
             if (DIM == 3) nb = nb + L.idz2 * (op + om);
-            if constexpr (UP && STAR)
-                return (b_at(st, c) + nb) * t.x + (t.y != 0.f ? prolong(st, c, kodd) : T(0));
-            else if constexpr (UP) return (b_at(st, c) + nb) * t.x + t.y * prolong(st, c, kodd);
+            if constexpr (UP) return (b_at(st, c) + nb) * t.x + t.y * prolong(st, c, kodd);
             else return (b_at(st, c) + nb) * t.x;
         }
         const uint32_t code = code_at(st, c);
