@@ -5,6 +5,7 @@ follow (stream, kernel mode, memory)."""
 import numpy as np
 import pytest
 
+from test_gpu_failed_solve import memory_taken
 from test_gpu_parity import connected, fluid_interior
 
 pytestmark = pytest.mark.gpu
@@ -222,7 +223,6 @@ def test_repeat_follows_the_stream(handle):
 def test_repeat_without_room_for_a_second_engine(handle):
     """With the device's memory taken, a run-away solve is repeated in its own engine: the
     same result as with a second one, and the next mask is on covering aggregates again."""
-    import torch
     solid = np.zeros((1502, 2002), np.uint8)
     solid[:, 1000] = 1
     fl = fluid_interior(solid)
@@ -244,15 +244,9 @@ def test_repeat_without_room_for_a_second_engine(handle):
     handle.solve(c, q, opts, strict=True)
     one = handle.device_bytes()
     assert two > one and np.array_equal(q, good)
-    torch.cuda.init()
-    free, _ = torch.cuda.mem_get_info(0)
-    hog = torch.empty(free - (two - one) // 2, dtype=torch.uint8, device="cuda:0")
-    try:
-        p = np.zeros_like(b)
+    p = np.zeros_like(b)
+    with memory_taken((two - one) // 2):
         got = handle.solve(b, p, opts)
-    finally:
-        del hog
-        torch.cuda.empty_cache()
     assert handle.device_bytes() <= one
     assert got.status == ref.status == 1 and got.iterations == ref.iterations
     assert np.array_equal(p, want)

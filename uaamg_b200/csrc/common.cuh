@@ -196,6 +196,4 @@ inline dim3 cell_grid(int nx, int ny, int nz) {
                 DIM == 3 ? (nz + b.z - 1) / b.z : 1);
 }
 
-inline size_t grid_blocks(dim3 g) { return (size_t)g.x * g.y * g.z; }
-
 }  // namespace uaamg
