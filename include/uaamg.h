@@ -110,10 +110,12 @@ UAAMG_API uaamg_status uaamg_set_stream(uaamg_handle* h, void* stream);
  * inspected, use the reference's hierarchy.  FP32 and mixed solves precondition with
  * the same Galerkin sums over aggregates that cover every fluid cell (a coarse cell is
  * fluid when any child is, odd sizes round up) and transfers that reach the coarse face
- * neighbours, which needs far fewer iterations next to solids and on odd sizes; with
- * Dirichlet walls they use the reference's.  A solve whose residual grows on that
- * hierarchy (a right-hand side inconsistent on separate parts of the fluid) is repeated
- * on the reference's. */
+ * neighbours (with one smoothing sweep, uaamg_set_smoothing, and V-cycle kernels 0 or 2,
+ * uaamg_set_vcycle_kernels), which needs far fewer iterations next to solids and on odd
+ * sizes; with Dirichlet walls they use the reference's.  A preconditioned solve that runs
+ * away on that hierarchy (a right-hand side inconsistent on separate parts of the fluid)
+ * is repeated on the reference's, by a second engine that is made then and kept while the
+ * mask stays, or in the first one's place when the device has no room for it. */
 UAAMG_API uaamg_status uaamg_set_problem_2d(uaamg_handle* h, int nx, int ny, double dx, double dy,
                                   const uint8_t* solid);
 UAAMG_API uaamg_status uaamg_set_problem_3d(uaamg_handle* h, int nx, int ny, int nz, double dx,
@@ -154,7 +156,10 @@ UAAMG_API uaamg_status uaamg_set_dirichlet_walls(uaamg_handle* h, int on);
  * 3 = as 0 with four marches per level (forward sweep; residual + restriction;
  * prolongation + even colour; odd colour);
  * 4 = four marches per level on every level and a separate coarsest-level kernel.
- * All give identical results in FP64; 1 to 4 exist to cross-check 0. */
+ * All give identical results in FP64; 1 to 4 exist to cross-check 0.  FP32 and mixed
+ * solves have star transfers on every level in 0 and 2, in the small-level kernel only in
+ * 3, and constant transfers in 1 and 4.  1 runs one smoothing sweep whatever
+ * uaamg_set_smoothing says. */
 UAAMG_API uaamg_status uaamg_set_vcycle_kernels(uaamg_handle* h, int sweeps);
 
 /* Smoothing schedule of this handle's V-cycle: pre- and post-smoothing sweeps (1 to 4)

@@ -114,9 +114,9 @@ __device__ __forceinline__ void publish(unsigned long long* to, int epoch, int i
 // right-hand side is smooth, since the 2-norm weighs the rough error that the coarse
 // levels bring in: 130 times at 2048 x 1024 with scattered solids, 420 at 2000 x 6, 9400
 // at 60000 x 8, falling again from the second iteration on.  Its rz does not rise, but in
-// channels some 25 times as long as wide, and there falls again too; that of an inconsistent
-// one rises on from the third iteration, which is what counts when max_iter ends a solve
-// (last).
+// channels (from some six times as long as wide), where it falls again within four
+// iterations; that of an inconsistent one rises on from the third iteration, which is what
+// counts when max_iter ends a solve (last).
 // With a small inconsistent share of b the residual falls to it first and rises from there
 // (share 1e-4: to 1e-3 in 6 iterations, past 1 in 15).  Once it has been below half of r0,
 // 1000 times the best ends the solve, three times at max_iter; consistent solves rise 28

@@ -986,12 +986,13 @@ private:
         // coarse couplings towards them act as Dirichlet walls.  CG then needs many
         // iterations for the modes this pins (without solids 8-13).  The FP32 and mixed
         // solves (cover_) aggregate every fluid cell instead: sizes rounded up, a coarse
-        // cell fluid when any child is, the same Galerkin sums.  Mixed solves to 1e-6:
-        // 96^3 with 8 spheres 50 -> 14 iterations (5.5 -> 1.6 ms), 256^3 with 32 spheres
-        // 84 -> 15 (39.6 -> 8.2 ms), 384^2 with one disk 93 -> 12 (4.5 -> 0.9 ms),
-        // 129 x 97 x 65 204 -> 46 (19.6 -> 5.0 ms).  The FP64 form and every V-cycle applied by itself
-        // keep the reference's rule, and so do problems with Dirichlet walls (their wall
-        // channel is defined by it).
+        // cell fluid when any child is, the same Galerkin sums.  Iterations of mixed solves to
+        // 1e-6 with the reference's rule, with this one and constant transfers, and with star
+        // transfers (fused.cuh): 96^3 with 8 spheres 47 / 14 / 11, 256^3 with 32 spheres 82 /
+        // 15 / 12, 384^2 with one disk 78 / 11 / 9, 2048 x 1024 155 / 19 / 12, 129 x 97 x 65
+        // 197 / 45 / 15; an iteration takes about the same time.  The FP64 form and every
+        // V-cycle applied by itself keep the reference's rule, and so do problems with
+        // Dirichlet walls (their wall channel is defined by it).
         const bool cover = cover_ && !plain_ && !dirichlet_;
         star_ = cover;
         const int up = cover ? 1 : 0;
@@ -1750,9 +1751,9 @@ private:
     }
 
     // ---- PCG solve, in four stages so that many engines can interleave (batch and
-    // serving): begin (right-hand side, initial residual, first preconditioner
-    // application, graph capture), step (queue two iterations), poll (has the
-    // device stopped?), end (solution out, exit diagnostics).
+    // serving): begin (right-hand side, initial residual, graph capture), step (queue two
+    // iterations, each begun at its preconditioner application), poll (has the device
+    // stopped?), end (solution out, exit diagnostics).
 
     Stencil stencil() const {
         Stencil st;

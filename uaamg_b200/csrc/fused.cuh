@@ -45,7 +45,7 @@
 // plus w times, over its coupled faces, the difference between the residuals on the
 // far and on the near side of the face.  Constant transfers overshoot in directions
 // the smoother is weak in; with w = 1/5 the mixed solve of 129 x 97 x 65 with spacings
-// 1 : 1.5 : 0.67 takes 15 iterations instead of 46, of 256^3 10 instead of 15.  The
+// 1 : 1.5 : 0.67 takes 15 iterations instead of 45, of 256^3 12 instead of 15.  The
 // way down then needs the residual on the tile and a 1-cell ring and one plane either
 // side of the chunk, so its boxes have a 3-cell ring; the way up needs the parent
 // level's x in boxes one cell wider, two planes deep, and the parent's codes, whose
