@@ -311,3 +311,21 @@ def test_server_budget_holds_for_small_ids(shape):
             assert srv.info()["device_bytes"] <= one + one // 2
     finally:
         srv.stop()
+
+
+@pytest.mark.parametrize("shape,max_iter,reached", [((65, 33), 60, 1e-6), ((130, 70), 20, 1e-10), ((130, 70), 60, 1e-6),
+                                                    ((70, 66, 67), 60, 1e-10), ((70, 66, 67), 100, 1e-6)])
+def test_converged_chambers_with_a_tolerance_out_of_reach(handle, shape, max_iter, reached):
+    """Two chambers, each with a consistent right-hand side, and a tolerance of 0: the solve
+    gets far below 1e-6 and keeps it, whatever its rounding does until max_iter."""
+    padded = tuple(n + 2 for n in shape[::-1])
+    solid = np.zeros(padded, np.uint8)
+    solid[..., shape[0] // 2] = 1
+    fl = fluid_interior(solid)
+    b = np.where(fl, np.random.default_rng(4).standard_normal(padded), 0.0)
+    for part in (np.s_[..., :shape[0] // 2], np.s_[..., shape[0] // 2 + 1:]):
+        v, f = b[part], fl[part]
+        v[f] -= v[f].mean()
+    handle.set_problem(solid, 1.0, 1.0, 1.0)
+    st = handle.solve(b, np.zeros_like(b), handle.options("mixed", 0.0, max_iter, "rel"))
+    assert st.iterations == max_iter and st.rel_residual <= reached

@@ -119,14 +119,17 @@ __device__ __forceinline__ void publish(unsigned long long* to, int epoch, int i
 // counts when max_iter ends a solve (last).
 // With a small inconsistent share of b the residual falls to it first and rises from there
 // (share 1e-4: to 1e-3 in 6 iterations, past 1 in 15).  Once it has been below half of r0,
-// 1000 times the best ends the solve, three times at max_iter; consistent solves rise 28
-// times over their best at most there (1000 x 5 x 5; other shapes 3, few past 5).
+// 1000 times the best ends the solve, 30 times at max_iter; consistent solves rise 28 times
+// over their best at most there (1000 x 5 x 5; other shapes 3, few past 5).  Not below 1e-6
+// r0: there a tolerance out of reach lets the rounding of a consistent right-hand side run
+// away (two chambers, 1e-15 after 60 iterations and 1e-8 after 200), and the reference's
+// hierarchy may not get that far in max_iter iterations at all.
 __device__ __forceinline__ bool residual_grew(double rr, double best, double r0, double bnorm, double rz,
                                               double rz0, double rz_peak, int it, bool last) {
     const double f = fmax(r0, 1e-3 * bnorm);
     return rr > 1e12 * f * f ||
            (last && it > 1 && rr > 4.0 * f * f && rz > rz0 && 4.0 * rz > rz_peak) ||
-           (4.0 * best < r0 * r0 && rr > (last ? 9.0 : 1e6) * best);
+           (4.0 * best < r0 * r0 && rr > 1e-12 * r0 * r0 && rr > (last ? 9e2 : 1e6) * best);
 }
 
 // q = a / d and r = a % d for 0 <= a < 2^31, 0 < d, from a reciprocal 1/d computed
