@@ -156,7 +156,8 @@ UAAMG_API uaamg_status uaamg_set_dirichlet_walls(uaamg_handle* h, int on);
  * 3 = as 0 with four marches per level (forward sweep; residual + restriction;
  * prolongation + even colour; odd colour);
  * 4 = four marches per level on every level and a separate coarsest-level kernel.
- * All give identical results in FP64; 1 to 4 exist to cross-check 0.  FP32 and mixed
+ * All give identical V-cycles in FP64 (a solve's dot products differ in rounding); 1 to 4
+ * exist to cross-check 0.  FP32 and mixed
  * solves have star transfers on every level in 0 and 2, in the small-level kernel only in
  * 3, and constant transfers in 1 and 4.  1 runs one smoothing sweep whatever
  * uaamg_set_smoothing says. */

@@ -1691,10 +1691,16 @@ private:
         UAAMG_LAUNCH_SMEM((KTag{K_UPE, l, c * (2.0 * t + 1.0 + coef) + cc * t}),
                           (k_up_even<DIM, T, FINE, CSL>), grid, blk, (UpeCfg<DIM, T, FINE, CSL>::BYTES),
                           maps<DIM>(l, false, true), mlevel(l), x, done, err_);
+        MLevel<T> m = mlevel(l);
+        dim3 zgrid = grid;
+        if (DIM == 3 && sizeof(T) == 8) {  // the z sums' own partition (pick_chunks)
+            m.zc = zdot_zc_;
+            zgrid = march_grid<DIM>(L.g, zdot_zc_);
+        }
         if (zdot)
             UAAMG_LAUNCH_SMEM((KTag{K_UPO, l, c * (2.5 * t + 1.0 + coef)}),
-                              (k_up_odd<DIM, T, FINE, true, CSL>), grid, blk, (UpoCfg<DIM, T, FINE, CSL>::BYTES),
-                              maps<DIM>(l, true, false), mlevel(l), x, done, err_, partials_, cg_);
+                              (k_up_odd<DIM, T, FINE, true, CSL>), zgrid, blk, (UpoCfg<DIM, T, FINE, CSL>::BYTES),
+                              maps<DIM>(l, true, false), m, x, done, err_, partials_, cg_);
         else
             UAAMG_LAUNCH_SMEM((KTag{K_UPO, l, c * (2.5 * t + 1.0 + coef)}),
                               (k_up_odd<DIM, T, FINE, false, CSL>), grid, blk, (UpoCfg<DIM, T, FINE, CSL>::BYTES),
