@@ -832,14 +832,20 @@ private:
             else if (L.c32) pick_chunks_as<DIM, false, T, STAR>(L);
             else pick_chunks_as<DIM, false, CS, STAR>(L);
         }
+        // chunks halved from 16 planes until every SM has four blocks
+        const Geom& g = lv_[0].g;
+        const long long tiles = (long long)((g.nx + kMX - 1) / kMX) * ((g.ny + kMY - 1) / kMY);
+        int zc = 16;
+        while (zc > 2 && tiles * ((g.nz + zc - 1) / zc) < 4LL * num_sms_) zc /= 2;
+        // The finest level with Dirichlet walls runs as four marches, whose blocks need no
+        // long chunks to pay for their start: on the fused march's length instead, solves of
+        // 224^3 take 16.8 (FP64) and 6.2 ms (mixed), here 13.2 and 5.5; 128^3 4.34 and 1.72,
+        // here 3.62 and 1.60; below 96^3 the same.
+        if (dirichlet_) lv_[0].zc = zc;
         if constexpr (sizeof(T) == 8) {
             // The FP64 form's dot products are summed per block (search direction, z sums); their
-            // partition stays (chunks halved from 16 planes until every SM has four blocks):
-            // 256^3 on another one stops after 81 iterations instead of the reference's 82.
-            const Geom& g = lv_[0].g;
-            const long long tiles = (long long)((g.nx + kMX - 1) / kMX) * ((g.ny + kMY - 1) / kMY);
-            int zc = 16;
-            while (zc > 2 && tiles * ((g.nz + zc - 1) / zc) < 4LL * num_sms_) zc /= 2;
+            // partition stays: 256^3 on another one stops after 81 iterations instead of the
+            // reference's 82.
             zdot_zc_ = pm_zc_ = zc;
             return;
         }
