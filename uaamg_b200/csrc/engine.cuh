@@ -1026,6 +1026,8 @@ private:
         }
         if (pmv2d_env_ > 0) {
             pmv2d_per_sm_ = pmv2d_env_;
+        } else if (sizeof(T) == 8) {
+            pmv2d_per_sm_ = 4;  // the partition of the FP64 form's p.Ap (k_pmatvec_2d)
         } else {
             int per_sm = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pmatvec_2d<T>, 256, 0) ==

@@ -727,12 +727,14 @@ __global__ void __launch_bounds__(256) k_resid_x64(Geom g, const uint8_t* __rest
 // pair sharing its vertical neighbours.  Reads of ghost or solid cells are harmless
 // (the padded arrays hold them) and discarded by the neighbour rule.  p_old and
 // p_new are distinct buffers.
+// FP64: four blocks an SM are both the partition of p.Ap, which stays, and resident (64
+// registers, 56 bytes spilled; on three blocks of 80 registers a solve of 1024^2 rounds
+// otherwise, and takes 5.7 instead of 6.0 ms in 60 iterations).
 template <class T>
-__global__ void __launch_bounds__(256) k_pmatvec_2d(Geom g, const uint8_t* __restrict__ code,
-                                                     const T* __restrict__ z,
-                                                     const T* __restrict__ pold,
-                                                     T* __restrict__ pnew, T* __restrict__ ap,
-                                                     Stencil st, double* partials, CGState* cg) {
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 1)
+    k_pmatvec_2d(Geom g, const uint8_t* __restrict__ code, const T* __restrict__ z,
+                 const T* __restrict__ pold, T* __restrict__ pnew, T* __restrict__ ap, Stencil st,
+                 double* partials, CGState* cg) {
     const T idx2 = (T)st.idx2, idy2 = (T)st.idy2, diag = (T)st.diag;
     double acc[1] = {0.0};
     const int sx = g.sx;
