@@ -120,7 +120,7 @@ UAAMG_API uaamg_status uaamg_set_problem_2d(uaamg_handle* h, int nx, int ny, dou
                                   const uint8_t* solid);
 UAAMG_API uaamg_status uaamg_set_problem_3d(uaamg_handle* h, int nx, int ny, int nz, double dx,
                                   double dy, double dz, const uint8_t* solid);
-/* Same, mask already on the device. */
+/* Same, mask already on the device (read in the order of the handle's stream). */
 UAAMG_API uaamg_status uaamg_set_problem_device(uaamg_handle* h, int dim, int nx, int ny, int nz,
                                       double dx, double dy, double dz,
                                       const uint8_t* d_solid);

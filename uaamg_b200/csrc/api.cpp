@@ -85,9 +85,10 @@ using uaamg::api::fail;
 using uaamg::api::cuda_fail;
 using uaamg::api::map_engine;
 
+// (The handle's own stream only, the legacy default one included: cudaDeviceSynchronize
+// breaks the graph captures of other threads' handles.)
 void free_problem(uaamg_handle* h) {
-    if (h->stream) cudaStreamSynchronize(h->stream);
-    else cudaDeviceSynchronize();
+    cudaStreamSynchronize(h->stream);
     cudaFree(h->d_solid); h->d_solid = nullptr;
     cudaFree(h->d_rhs); h->d_rhs = nullptr;
     cudaFree(h->d_p); h->d_p = nullptr;
@@ -156,8 +157,7 @@ uaamg_status set_problem(uaamg_handle* h, int dim, int nx, int ny, int nz, doubl
     if (h->dim == dim && h->nx == nx && h->ny == ny && h->nz == nz) {
         // a new mask on the same grid: the buffers stay (allocating and freeing them took
         // 5 to 40 ms a call, against 1 to 2 ms for the set-up itself)
-        if (h->stream) cudaStreamSynchronize(h->stream);
-        else cudaDeviceSynchronize();
+        cudaStreamSynchronize(h->stream);
         h->lap_on = false;
         h->has_hist = false;
         for (bool& r : h->ready) r = false;
@@ -319,7 +319,7 @@ uaamg_status uaamg_set_variable_laplacian(uaamg_handle* h, const double* lap_dia
         }
     }
     // the solves in flight may still read the previous coefficients
-    cudaError_t e = h->stream ? cudaStreamSynchronize(h->stream) : cudaDeviceSynchronize();
+    cudaError_t e = cudaStreamSynchronize(h->stream);
     for (int a = 0; a < 3 && e == cudaSuccess; ++a)
         e = cudaMemcpyAsync(h->d_lap[a], src[a], bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);

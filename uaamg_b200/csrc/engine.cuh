@@ -1947,10 +1947,17 @@ private:
                     ce = cudaStreamEndCapture(cap_, &graph);
                 }
                 st_ = saved;
-                if (ce != cudaSuccess || !graph) { cuda_error = ce != cudaSuccess ? ce : cudaErrorUnknown; return E_CUDA; }
-                ce = cudaGraphInstantiate(&gexec_, graph, 0);
-                cudaGraphDestroy(graph);
-                if (ce != cudaSuccess) { gexec_ = nullptr; cuda_error = ce; return E_CUDA; }
+                if (ce == cudaSuccess && graph) {
+                    ce = cudaGraphInstantiate(&gexec_, graph, 0);
+                    if (ce != cudaSuccess) gexec_ = nullptr;
+                    cudaGraphDestroy(graph);
+                }
+                // A capture that another thread broke (a device synchronisation): this solve
+                // launches its kernels one by one.
+                if (!gexec_) {
+                    cudaGetLastError();
+                    use_graph_ = false;
+                }
                 glaunches_ = launches_ - before;
                 launches_ = before;
                 gkey_ = key;
