@@ -483,6 +483,8 @@ private:
         }
         if (e != E_OOM) {
             cuda_error = fb_->cuda_error;
+            delete fb_;  // (its set-up failed: nothing to keep)
+            fb_ = nullptr;
             return e;
         }
         const long before = launches_;
