@@ -329,3 +329,23 @@ def test_converged_chambers_with_a_tolerance_out_of_reach(handle, shape, max_ite
     handle.set_problem(solid, 1.0, 1.0, 1.0)
     st = handle.solve(b, np.zeros_like(b), handle.options("mixed", 0.0, max_iter, "rel"))
     assert st.iterations == max_iter and st.rel_residual <= reached
+
+
+@pytest.mark.parametrize("warm", [False, True])
+@pytest.mark.parametrize("precision", ["mixed", "fp32"])
+@pytest.mark.parametrize("wall,share,max_iter", [(10, 1e-4, 12), (10, 1e-6, 25), (80, 1e-4, 25), (80, 1e-6, 12)])
+def test_chambers_of_different_size(handle, wall, share, max_iter, precision, warm):
+    """A small chamber beside a large one, an absolute tolerance, from zero and from a warm
+    start: as test_inconsistent_share_ends_as_on_the_reference_hierarchy."""
+    solid = np.zeros((72, 92), np.uint8)
+    solid[:, wall] = 1
+    fl = fluid_interior(solid)
+    lab = np.where(fl, 1 + (np.arange(92) > wall)[None, :], 0)
+    b = _inconsistent(solid, lab, share)
+    p0 = np.where(fl, np.random.default_rng(6).standard_normal(solid.shape), 0.0) * warm
+    handle.set_problem(solid, 1.0, 1.0)
+    opts = lambda prec: handle.options(prec, 1e-6, max_iter, "abs", warm_start=warm)
+    ref = handle.solve(b, p0.copy(), opts("fp64"))
+    st = handle.solve(b, p0.copy(), opts(precision))
+    assert st.status == 1 and st.iterations == max_iter
+    assert st.rel_residual <= 6.0 * ref.rel_residual
